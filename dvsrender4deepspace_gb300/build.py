@@ -41,7 +41,8 @@ def _sources():
 
 
 def _headers():
-    return ([os.path.join(CSRC, f) for f in ("kernels.h", "dvs_internal.h", "device_optics.cuh", "device_circuit.cuh")]
+    return ([os.path.join(CSRC, f) for f in ("kernels.h", "dvs_internal.h", "device_optics.cuh", "device_circuit.cuh",
+                                            "device_math.cuh", "trace_item.cuh")]
             + [os.path.join(APPS, f) for f in sorted(os.listdir(APPS)) if f.endswith(".hpp")]
             + [os.path.join(ROOT, "include", f) for f in ("dvs_gb300.h", "dvs_gb300.hpp")])
 

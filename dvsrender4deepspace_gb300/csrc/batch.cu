@@ -35,12 +35,13 @@ __device__ __forceinline__ int job_of(const T *first, int n_jobs, T x) {
 // The job table travels as the launch's parameter block (__grid_constant__: no
 // copy), so a warp reads its job's view -- the same job for all its lanes --
 // through the constant cache, as the one-sensor kernel reads its view.
-template <int kRays, int kGeo>
-__global__ void __launch_bounds__(128, kRays == 2 ? DVS_TRACE_PAIR_MIN_BLOCKS : DVS_TRACE_MIN_BLOCKS)
+template <int kRays, int kGeo, bool kBeam>
+__global__ void __launch_bounds__(128, kRays == 2 ? DVS_TRACE_PAIR_MIN_BLOCKS
+                                       : kBeam    ? DVS_TRACE_BEAM_MIN_BLOCKS
+                                                  : DVS_TRACE_MIN_BLOCKS)
     trace_jobs_kernel(const __grid_constant__ TraceJobs P) {
-  __shared__ int s_code[kWarpsPerBlock][kStackSlots];
-  __shared__ float s_t[kWarpsPerBlock][kStackSlots];
-  __shared__ SubraySample s_subrays[kWarpsPerBlock][kSubrayTable];
+  __shared__ TraceShared s_warp[kWarpsPerBlock];
+  __shared__ Beam s_beam[kBeam ? kWarpsPerBlock : 1];
   __shared__ long long s_first[kMaxBatchJobs];
   __shared__ long long s_base;
   for (int j = threadIdx.x; j < P.n_jobs; j += blockDim.x) s_first[j] = P.jobs[j].first_item;
@@ -58,9 +59,8 @@ __global__ void __launch_bounds__(128, kRays == 2 ? DVS_TRACE_PAIR_MIN_BLOCKS : 
     if (item < P.total_items) {        // warp-uniform
       const int j = job_of<long long>(s_first, P.n_jobs, item);
       const TraceJob &J = P.jobs[j];
-      trace_cells_item<kRadiance, kRays, kGeo>(J.view, J.n_pix, nullptr, J.poses, J.c0, J.nc, J.cw_log2,
-                                               J.radiance, nullptr, J.counters, item - s_first[j], s_code[wib],
-                                               s_t[wib], s_subrays[wib]);
+      trace_cells_item<kRadiance, kRays, kGeo, kBeam>(J.view, J.n_pix, nullptr, J.poses, J.c0, J.nc, J.shape,
+                                               J.radiance, nullptr, J.counters, item - s_first[j], s_warp[wib], s_beam[kBeam ? wib : 0]);
     }
   }
 }
@@ -77,35 +77,74 @@ __global__ void __launch_bounds__(128) circuit_jobs_kernel(const CircuitJob *__r
                               J.ev_count, J.slab_t, J.slab_p, J.error, J.counters);
 }
 
-template <int kRays, int kGeo>
+template <int kRays, int kGeo, bool kBeam>
 cudaError_t trace_jobs_geo(const TraceJobs &jobs, cudaStream_t s) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_jobs_kernel<kRays, kGeo>, 128, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_jobs_kernel<kRays, kGeo, kBeam>, 128, 0);
   // resident blocks only (a persistent grid), fewer when there are fewer items than warps
   const long long resident = (long long)sms * (per_sm > 0 ? per_sm : 1);
   const long long needed = (jobs.total_items + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const long long grid = needed < resident ? needed : resident;
-  trace_jobs_kernel<kRays, kGeo><<<(int)grid, 128, 0, s>>>(jobs);
+  trace_jobs_kernel<kRays, kGeo, kBeam><<<(int)grid, 128, 0, s>>>(jobs);
   return cudaGetLastError();
 }
 
 template <int kRays>
 cudaError_t trace_jobs_rays(const TraceJobs &jobs, int geometry, cudaStream_t s) {
+  bool beam = false;  // one job with beams takes the kernel that has them
+  for (int j = 0; j < jobs.n_jobs; ++j) beam = beam || jobs.jobs[j].shape.beam;
+#define DVS_JOBS_GEO(G) (beam ? trace_jobs_geo<kRays, G, true>(jobs, s) : trace_jobs_geo<kRays, G, false>(jobs, s))
   switch (geometry) {
-    case kGeoHalfBounds: return trace_jobs_geo<kRays, kGeoHalfBounds>(jobs, s);
-    case kGeoWatertight: return trace_jobs_geo<kRays, kGeoWatertight>(jobs, s);
-    case kGeoHalfBounds | kGeoWatertight: return trace_jobs_geo<kRays, kGeoHalfBounds | kGeoWatertight>(jobs, s);
-    default: return trace_jobs_geo<kRays, kGeoReference>(jobs, s);
+    case kGeoHalfBounds: return DVS_JOBS_GEO(kGeoHalfBounds);
+    case kGeoWatertight: return DVS_JOBS_GEO(kGeoWatertight);
+    case kGeoHalfBounds | kGeoWatertight: return DVS_JOBS_GEO(kGeoHalfBounds | kGeoWatertight);
+    default: return DVS_JOBS_GEO(kGeoReference);
   }
+#undef DVS_JOBS_GEO
 }
 
 }  // namespace
 
-long long trace_job_items(int n_pix, int nc, int cw_log2) {
-  const int cw = 1 << cw_log2, ppw = 32 >> cw_log2;
-  return (long long)((n_pix + ppw - 1) / ppw) * ((nc + cw - 1) / cw);
+ItemShape trace_item_shape(int n_pix, int nc, int cw_log2, int sub_rays, int rays, bool scattered) {
+  constexpr int kItemPackets = 64;      // packets that share a beam
+  constexpr int kBeamPackets = 16;      // fewest that do
+  constexpr long long kMinItems = 8 * 2432;  // several rounds of the GPU's resident warps (152 SMs x 16)
+  const int cw = 1 << cw_log2, ppw = 32 >> cw_log2, n_groups = (nc + cw - 1) / cw;
+  const long long n_sets = (n_pix + ppw - 1) / ppw;
+  const int packets = (sub_rays + rays - 1) / rays;  // of one pixel set and cell group
+  ItemShape s{cw_log2, 1, 1, 0};
+  while (s.groups < n_groups && s.groups * packets < kItemPackets &&
+         n_sets * ((n_groups + 2 * s.groups - 1) / (2 * s.groups)) >= kMinItems)
+    s.groups = s.groups * 2 < n_groups ? s.groups * 2 : n_groups;
+  if (!scattered)
+    while (s.sets < 16 && s.sets * s.groups * packets < kItemPackets / 4 &&
+           (n_sets + 2 * s.sets - 1) / (2 * s.sets) * ((n_groups + s.groups - 1) / s.groups) >= kMinItems)
+      s.sets *= 2;
+  // fewer packets do not pay for the beam's own walks, and packets over more than four pixels (fewer than 8 cells) are
+  // themselves as wide as the beam
+  s.beam = cw_log2 >= 3 && s.sets * s.groups * packets >= kBeamPackets;
+  return s;
+}
+
+// Measured with beams: one ray per lane 93.6 ms against two 131 ms for an orbit batch (346x260, 16 sub-rays, 640
+// cells), 305 against 397 ms at 1280x720 (64 sub-rays, 64 cells): the beam leaves no node tests to share between a
+// lane's rays, and the second ray's code does not fit the instruction cache.  Without beams two per lane share them.
+int trace_rays(const SceneView &view, int n_pix, int nc, int cw_log2, bool scattered) {
+  const int ss2 = view.samples * view.samples;
+  if (view.rays == 0) {
+    if (trace_item_shape(n_pix, nc, cw_log2, ss2, 1, scattered).beam) return 1;
+    return ss2 % 2 == 0 ? 2 : 1;
+  }
+  // four rays per lane only in the reference format (the others keep two)
+  if (view.geometry == kGeoReference && view.rays >= 4 && ss2 % 4 == 0) return 4;
+  return view.rays >= 2 && ss2 % 2 == 0 ? 2 : 1;
+}
+
+long long trace_job_items(int n_pix, int nc, const ItemShape &s) {
+  const int cw = 1 << s.cw_log2, ppw = 32 >> s.cw_log2, n_groups = (nc + cw - 1) / cw, n_sets = (n_pix + ppw - 1) / ppw;
+  return (long long)((n_sets + s.sets - 1) / s.sets) * ((n_groups + s.groups - 1) / s.groups);
 }
 
 cudaError_t launch_trace_jobs(const TraceJobs &jobs, int rays, int geometry, cudaStream_t s) {

@@ -253,6 +253,7 @@ struct dvs_scene {
   int builder = 0;  // dvs_bvh_params.builder
   double build_seconds = 0;
   double sah_node_visits = 0, sah_triangle_tests = 0;
+  HapkeConst hc{};             // the material's constants (form_constants)
   float coherent_span = 1.0f;  // 0.5 % of the scene's largest extent
   // camera render buffers
   cudaStream_t stream = nullptr;
@@ -286,10 +287,22 @@ struct dvs_scene {
     v.cy = camera.cy;
     v.coherent_span = coherent_span;
     v.hapke = hapke;
-    v.rays = 2;
+    v.hc = hc;
+    v.rays = 0;  // automatic
     return v;
   }
   int pixels() const { return camera.width * camera.height; }
+  // The Hapke constants of this scene's material, on its stream.
+  cudaError_t form_constants() {
+    HapkeConst *d = nullptr;
+    cudaError_t e = cudaMallocAsync(&d, sizeof(HapkeConst), stream);
+    if (e != cudaSuccess) return e;
+    e = launch_hapke_const(hapke, d, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hc, d, sizeof(HapkeConst), cudaMemcpyDeviceToHost, stream);
+    cudaFreeAsync(d, stream);
+    const cudaError_t es = cudaStreamSynchronize(stream);
+    return e == cudaSuccess ? es : e;
+  }
 };
 
 struct dvs_sensor {
@@ -368,7 +381,8 @@ struct dvs_sensor {
   std::vector<int32_t> band_rank_of_pixel;  // band-local row-major pixel -> rank
   int pixels() const { return n_pix; }
   CellPose *probe_poses = nullptr;  // the five initial adaptive probe poses
-  int rays_per_lane = 2;  // traversal tuning: 1, 2 or 4 sub-rays per lane (dvs_sensor_set_tuning / autotune)
+  // traversal tuning: 1, 2 or 4 sub-rays per lane (dvs_sensor_set_tuning / autotune), 0 until one is set: automatic
+  int rays_per_lane = 0;
   // The view the hot path traces with: its radiance chunk is float when the
   // circuit is FP32 (photo.chunk_f32).  view64: the same with a double chunk,
   // for the initialization and the adaptive solver's knots and probes.
@@ -575,6 +589,7 @@ int dvs_scene_create(const float *vertices, const float *normals, const uint32_t
   if (e == cudaSuccess)
     e = cudaMemcpy(s->pixel_of_rank, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = s->form_constants();
   if (e != cudaSuccess) {
     dvs_scene_destroy(s);
     return fail(DVS_ERR_CUDA, std::string("[CUDA Error] in upload scene array : ") + cudaGetErrorString(e));
@@ -654,6 +669,8 @@ int dvs_scene_view_create(const dvs_scene *base, const dvs_camera *camera, int32
   if (e == cudaSuccess)
     e = cudaMemcpy(s->pixel_of_rank, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+  if (std::memcmp(&s->hapke, &base->hapke, sizeof(dvs_hapke)) == 0) s->hc = base->hc;
+  else if (e == cudaSuccess) e = s->form_constants();
   if (e != cudaSuccess) {
     dvs_scene_destroy(s);
     return fail(DVS_ERR_CUDA, std::string("[CUDA Error] in upload scene array : ") + cudaGetErrorString(e));
@@ -1690,7 +1707,8 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
   }
   SceneView view = s->view();
   float best = -1, def_ms = -1;
-  int best_log2 = default_log2, best_rays = s->rays_per_lane, tried = 0;
+  const int default_rays = trace_rays(view, n_sub, nc, default_log2, true);
+  int best_log2 = default_log2, best_rays = default_rays, tried = 0;
   cudaError_t err = cudaSuccess;
   for (int rays = 1; rays <= 4 && err == cudaSuccess; rays *= 2) {
     if (ss2 % rays) break;
@@ -1711,7 +1729,7 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
       }
       if (err != cudaSuccess) break;
       ++tried;
-      if (lg == default_log2 && rays == s->rays_per_lane) def_ms = ms;
+      if (lg == default_log2 && rays == default_rays) def_ms = ms;
       if (best < 0 || ms < best) {
         best = ms;
         best_log2 = lg;
@@ -1726,7 +1744,7 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
   if (def_ms > 0 && best > 0.97f * def_ms) {  // keep the current shape unless another is clearly faster
     best = def_ms;
     best_log2 = default_log2;
-    best_rays = s->rays_per_lane;
+    best_rays = default_rays;
   }
   s->opt.cells_per_warp = 1 << best_log2;
   s->rays_per_lane = best_rays;
@@ -1923,11 +1941,15 @@ int dvs_batch_process(dvs_batch *b, const dvs_optical_interval *const *intervals
     CUDA_TRY(cudaMalloc(&b->d_next, sizeof(unsigned long long) * rounds), "batch work counters");
     b->rounds_cap = rounds;
   }
-  // the job tables of every round; rays per lane shared by the batch (2 when
-  // every active member's sub-ray count is even)
+  // the job tables of every round; rays per lane shared by the batch: 2 when no active member has beams or an odd
+  // sub-ray count
   bool pairs = true;
-  for (size_t m = 0; m < n; ++m)
-    if (counts[m] && (b->members[m]->scene->samples * b->members[m]->scene->samples) % 2) pairs = false;
+  for (size_t m = 0; m < n; ++m) {
+    if (!counts[m]) continue;
+    SceneView v = b->members[m]->view();
+    v.rays = 0;
+    if (trace_rays(v, b->members[m]->pixels(), (int)std::min(chunks[m], n_cells[m]), cw[m], false) != 2) pairs = false;
+  }
   std::vector<int> n_trace(rounds, 0), n_circuit(rounds, 0), blocks(rounds, 0);
   std::vector<long long> items(rounds, 0);
   for (int r = 0; r < rounds; ++r) {
@@ -1949,8 +1971,9 @@ int dvs_batch_process(dvs_batch *b, const dvs_optical_interval *const *intervals
       t.n_pix = s->pixels();
       t.c0 = (int)c0;
       t.nc = nc;
-      t.cw_log2 = cw[m];
-      items[r] += trace_job_items(t.n_pix, nc, cw[m]);
+      const int sub_rays = s->scene->samples * s->scene->samples;
+      t.shape = trace_item_shape(t.n_pix, nc, cw[m], sub_rays, pairs ? 2 : 1, false);
+      items[r] += trace_job_items(t.n_pix, nc, t.shape);
       CircuitJob &c = cj[n_circuit[r]++];
       c.p = s->p;
       c.photo = s->photo;

@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "device_math.cuh"
 #include "kernels.h"
 
 namespace dvsgb {
@@ -33,6 +34,13 @@ __device__ __forceinline__ float3 normalize(float3 v) {
   if (len > 0.0f) return v / len;
   return f3(0.0f, 0.0f, 0.0f);
 }
+// normalize in the forms of device_math.cuh (a zero vector stays zero).
+__device__ __forceinline__ float3 unit(float3 v) {
+  const float len = sqrt_rn(dot(v, v));
+  if (!(len > 0.0f)) return f3(0.0f, 0.0f, 0.0f);
+  const float y = rcp_rn(len);
+  return f3(div_by(v.x, len, y), div_by(v.y, len, y), div_by(v.z, len, y));
+}
 __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 
 // ---- Hapke (include/dvs/hapke.hpp:14-157), FP32 --------------------------------
@@ -53,16 +61,15 @@ __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fm
 // (safe_tan, hapke.hpp:14-16), and psi == acos(-1) keeps the reference's
 // tan(pi_f / 2) < 0, whose exp overflows and makes the sample NaN (dropped by
 // the caller's fmaxf) -- here tan(psi/2) = -inf there.
-__device__ __forceinline__ float pow15(float y) { return y * sqrtf(y); }
-__device__ __forceinline__ float hg_double_lobe(float cosg, float b, float c) {
-  const float one_minus_bb = 1.0f - b * b;
-  const float term1 = ((1.0f + c) * 0.5f) * one_minus_bb / pow15(1.0f - 2.0f * b * cosg + b * b);
-  const float term2 = ((1.0f - c) * 0.5f) * one_minus_bb / pow15(1.0f + 2.0f * b * cosg + b * b);
+__device__ __forceinline__ float pow15(float y) { return y * sqrt_rn(y); }
+__device__ __forceinline__ float hg_double_lobe(float cosg, float b, const HapkeConst &h) {
+  const float term1 = div_rn(h.lobe_pos, pow15(1.0f - 2.0f * b * cosg + b * b));
+  const float term2 = div_rn(h.lobe_neg, pow15(1.0f + 2.0f * b * cosg + b * b));
   return term1 + term2;
 }
-__device__ __forceinline__ float b_s(float tg, float h) {
+__device__ __forceinline__ float b_s(float tg, float h, float inv_h) {
   if (h <= 0.0f) return tg <= 0.0f ? 1.0f : 0.0f;
-  return 1.0f / (1.0f + tg / h);
+  return rcp_rn(1.0f + div_by(tg, h, inv_h));
 }
 __device__ __forceinline__ float b_c(float tg, float h) {
   if (h <= 0.0f) return tg <= 0.0f ? 1.0f : 0.0f;
@@ -72,8 +79,8 @@ __device__ __forceinline__ float b_c(float tg, float h) {
 }
 __device__ __forceinline__ float hfunc(float x, float w, float r0) {
   if (x <= 1e-8f) return 1.0f;
-  const float term = r0 + (1.0f - 2.0f * r0 * x) * 0.5f * logf(1.0f + 1.0f / x);
-  return 1.0f / (1.0f - w * x * term);
+  const float term = r0 + (1.0f - 2.0f * r0 * x) * 0.5f * logf(1.0f + rcp_rn(x));
+  return rcp_rn(1.0f - w * x * term);
 }
 __device__ __forceinline__ float hfunc_r0(float w) {
   const float root = sqrtf(fmaxf(0.0f, 1.0f - w));
@@ -85,29 +92,30 @@ __device__ __forceinline__ float porosity_k(float phi) {
   return -logf(1.0f - p) / p;
 }
 
-// The parts of hapke.hpp that depend on the material only: porosity K,
-// tan(thetap), 1/tan(thetap), chi(thetap), the r0 of the H-function for the
-// scene's single-scattering albedo and the cap of tan(phase/2).  Each is the
-// value hapke.hpp recomputes inside every call (same operations, same
-// rounding), evaluated once per pixel sample loop instead of per shaded ray.
-struct HapkeConst {
-  float K, tan_t, cot_t, chi, r0_w, tg_max;
-  bool rough;
-};
+// The parts of hapke.hpp that depend on the material only, each the value
+// hapke.hpp recomputes inside every call (same operations, same rounding):
+// evaluated on the device once per scene (hapke_const_kernel) and read from the
+// view as constants.  Evaluated per pixel sample loop, two tanf, a powf and a
+// logf were a sixth of a one-ray loop.
 __device__ __forceinline__ HapkeConst hapke_const(const dvs_hapke &p) {
   HapkeConst h;
   h.K = porosity_k(p.phi);
+  h.inv_K = 1.0f / h.K;
   h.rough = !(p.thetap <= 1e-8f);
   h.tan_t = tanf(p.thetap);
   h.cot_t = 1.0f / h.tan_t;
   h.chi = 1.0f / sqrtf(1.0f + kPi * h.tan_t * h.tan_t);
   h.r0_w = hfunc_r0(p.w);
   h.tg_max = tanf(kPi / 2.0f - 1e-6f);
+  const float one_minus_bb = 1.0f - p.b * p.b;
+  h.lobe_pos = ((1.0f + p.c) * 0.5f) * one_minus_bb;
+  h.lobe_neg = ((1.0f - p.c) * 0.5f) * one_minus_bb;
+  h.inv_hS = 1.0f / p.hS;
   return h;
 }
 // The quotient q = cot(thetap) cos(y) / max(sin(y), 1e-6) shared by e1 and e2.
 __device__ __forceinline__ float e_quot(float cot_t, float cosy, float siny) {
-  return cot_t * cosy / fmaxf(siny, 1e-6f);
+  return div_rn(cot_t * cosy, fmaxf(siny, 1e-6f));
 }
 
 // Inlining policy of the large shading and traversal bodies (instruction-cache pressure).
@@ -117,19 +125,22 @@ __device__ __forceinline__ float e_quot(float cot_t, float cosy, float siny) {
 #define DVS_SHADE_INLINE
 #endif
 // hapke_reflectance (hapke.hpp:131-152) in the identity form above; r0 is
-// hfunc's r0 for this albedo.
+// hfunc's r0 for this albedo.  Quotients with a divisor in common share its
+// reciprocal, and constant divisors have theirs beforehand.  The divisors are
+// positive (2 - e1 >= 1, the shadowing denominators at least 1e-6) or end in a
+// NaN or infinite sample as with /, which the caller's fmaxf drops.
 DVS_SHADE_INLINE __device__ float hapke_reflectance(float cosi, float cose, float cosg, float albedo, float r0,
                                                     const dvs_hapke &p, const HapkeConst &h) {
   if (cosi <= 0 || cose <= 0) return 0;
   cosi = clampf(cosi, 0, 1);
   cose = clampf(cose, 0, 1);
   cosg = clampf(cosg, -1, 1);
-  const float sini = sqrtf(fmaxf(0, 1 - cosi * cosi)), sine = sqrtf(fmaxf(0, 1 - cose * cose));
-  const float tg = fminf(sqrtf((1.0f - cosg) / (1.0f + cosg)), h.tg_max);
-  const float cpsi = clampf((cosg - cosi * cose) / (sini * sine + 1e-6f), -1.0f, 1.0f);
+  const float sini = sqrt_rn(fmaxf(0, 1 - cosi * cosi)), sine = sqrt_rn(fmaxf(0, 1 - cose * cose));
+  const float tg = fminf(sqrt_rn(div_rn(1.0f - cosg, 1.0f + cosg)), h.tg_max);  // cos g = -1: NaN, and fminf takes tg_max
+  const float cpsi = clampf(div_rn(cosg - cosi * cose, sini * sine + 1e-6f), -1.0f, 1.0f);
   const float psi = acosf(cpsi);
-  const float p_g = hg_double_lobe(cosg, p.b, p.c);
-  const float BS = b_s(tg, p.hS);
+  const float p_g = hg_double_lobe(cosg, p.b, h);
+  const float BS = b_s(tg, p.hS, h.inv_hS);
   // b_c is finite, so with B_C0 == 0 the factor (1 + BC * B_C0) is exactly 1
   // whatever BC is: skip its evaluation.
   const float BC = p.B_C0 != 0.0f ? b_c(tg, p.hC) : 0.0f;
@@ -145,23 +156,31 @@ DVS_SHADE_INLINE __device__ float hapke_reflectance(float cosi, float cose, floa
     const float e2e = expf((-1.0f / kPi) * qe * qe), e2i = expf((-1.0f / kPi) * qi * qi);
     const float e1e = expf((-2.0f / kPi) * qe), e1i = expf((-2.0f / kPi) * qi);
     // eta(y) = chi * (cos y + sin y * tan(thetap) * e2(y) / (2 - e1(y)))
-    const float eta_e = ch * (cose + sine * tan_thetap * e2e / (2.0f - e1e));
-    const float eta_i = ch * (cosi + sini * tan_thetap * e2i / (2.0f - e1i));
-    const float tpsi = cpsi > -1.0f ? sqrtf((1.0f - cpsi) / (1.0f + cpsi)) : -kInf();  // tan(psi / 2)
+    const float eta_e = ch * (cose + div_rn(sine * tan_thetap * e2e, 2.0f - e1e));
+    const float eta_i = ch * (cosi + div_rn(sini * tan_thetap * e2i, 2.0f - e1i));
+    const float tpsi = cpsi > -1.0f ? sqrt_rn(div_rn(1.0f - cpsi, 1.0f + cpsi)) : -kInf();  // tan(psi / 2)
     const float fp = expf(-2.0f * tpsi);
-    if (cosi >= cose) {
-      mu0 = ch * (cosi + sini * tan_thetap * (cpsi * e2e + s2 * e2i) / (2.0f - e1e - (psi / kPi) * e1i));
-      mue = ch * (cose + sine * tan_thetap * (e2e - s2 * e2i) / (2.0f - e1e - (psi / kPi) * e1i));
-      S = mue / eta_e * cosi / eta_i * ch / (1.0f - fp + fp * ch * (cosi / eta_i));
-    } else {
-      mu0 = ch * (cosi + sini * tan_thetap * (e2i - s2 * e2e) / (2.0f - e1i - (psi / kPi) * e1e));
-      mue = ch * (cose + sine * tan_thetap * (cpsi * e2i + s2 * e2e) / (2.0f - e1i - (psi / kPi) * e1e));
-      S = mue / eta_e * cosi / eta_i * ch / (1.0f - fp + fp * ch * (cose / eta_e));
-    }
+    const float psi_pi = div_by(psi, kPi, 1.0f / kPi);
+    // the two branches of hapke.hpp with incidence and emission exchanged
+    const bool low = cosi >= cose;
+    const float e1a = low ? e1e : e1i, e1b = low ? e1i : e1e;
+    const float e2a = low ? e2e : e2i, e2b = low ? e2i : e2e;
+    const float cosa = low ? cosi : cose, sina = low ? sini : sine;  // the angle nearer the normal
+    const float cosb = low ? cose : cosi, sinb = low ? sine : sini;
+    const float den = 2.0f - e1a - psi_pi * e1b, yden = rcp_rn(den);
+    const float mua = ch * (cosa + div_by(sina * tan_thetap * (cpsi * e2a + s2 * e2b), den, yden));
+    const float mub = ch * (cosb + div_by(sinb * tan_thetap * (e2a - s2 * e2b), den, yden));
+    mu0 = low ? mua : mub;
+    mue = low ? mub : mua;
+    const float yi = rcp_rn(eta_i);
+    const float f = div_by(div_rn(mue, eta_e) * cosi, eta_i, yi) * ch;  // mue / eta_e * cosi / eta_i * ch
+    const float shadowed = low ? div_by(cosi, eta_i, yi) : div_rn(cose, eta_e);
+    S = div_rn(f, 1.0f - fp + fp * ch * shadowed);
   }
-  const float M = hfunc(mu0 / K, albedo, r0) * hfunc(mue / K, albedo, r0) - 1.0f;
-  const float LS = mu0 / (mu0 + mue + 1e-6f);
-  return (albedo / (4.0f * kPi)) * LS * K * (p_g * (1.0f + BS * p.B_S0) + M) * (1.0f + BC * p.B_C0) * S;
+  const float M = hfunc(div_by(mu0, K, h.inv_K), albedo, r0) * hfunc(div_by(mue, K, h.inv_K), albedo, r0) - 1.0f;
+  const float LS = div_rn(mu0, mu0 + mue + 1e-6f);
+  return div_by(albedo, 4.0f * kPi, 1.0f / (4.0f * kPi)) * LS * K * (p_g * (1.0f + BS * p.B_S0) + M) *
+         (1.0f + BC * p.B_C0) * S;
 }
 
 // ---- pose interpolation (include/dvs/device_optics.cuh:6-29) ---------------------
@@ -212,9 +231,9 @@ __device__ __forceinline__ float3 rotate_ray(const CellPose &q, float3 v) {
 // ---- traversal -------------------------------------------------------------------
 __device__ __forceinline__ float3 inverse_direction(float3 d) {  // device_ray.hpp:6-12
   float3 inv;
-  inv.x = 1.0f / (fabsf(d.x) > 1e-20f ? d.x : copysignf(1e-20f, d.x));
-  inv.y = 1.0f / (fabsf(d.y) > 1e-20f ? d.y : copysignf(1e-20f, d.y));
-  inv.z = 1.0f / (fabsf(d.z) > 1e-20f ? d.z : copysignf(1e-20f, d.z));
+  inv.x = rcp_rn(fabsf(d.x) > 1e-20f ? d.x : copysignf(1e-20f, d.x));
+  inv.y = rcp_rn(fabsf(d.y) > 1e-20f ? d.y : copysignf(1e-20f, d.y));
+  inv.z = rcp_rn(fabsf(d.z) > 1e-20f ? d.z : copysignf(1e-20f, d.z));
   return inv;
 }
 
@@ -230,7 +249,7 @@ __device__ __forceinline__ bool intersect_tri(float3 ray, float3 o, float3 v0, f
   const float3 pvec = cross(ray, e2);
   const float det = dot(e1, pvec);
   if (fabsf(det) < kRayEps) return false;
-  const float inv_det = 1.0f / det;
+  const float inv_det = rcp_rn(det);
   const float3 tvec = o - v0;
   u = dot(tvec, pvec) * inv_det;
   if (u < 0.0f || u > 1.0f) return false;
@@ -274,9 +293,9 @@ __device__ __forceinline__ WtRay wt_setup(float3 d) {
   WtRay w;
   w.kz = ax > ay ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
   const float3 p = wt_perm(d, w.kz);
-  w.sx = p.x / p.z;
-  w.sy = p.y / p.z;
-  w.sz = 1.0f / p.z;
+  w.sz = rcp_rn(p.z);  // the dominant axis: at least 0.57 of the length
+  w.sx = div_by(p.x, p.z, w.sz);
+  w.sy = div_by(p.y, p.z, w.sz);
   return w;
 }
 // o, v0, v1, v2 in the ray's cyclic order (wt_perm).
@@ -303,7 +322,7 @@ __device__ __forceinline__ bool intersect_wt(const WtRay &w, float3 o, float3 v0
   const float det = U + V + W;
   if (det == 0.0f) return false;
   const float T = U * (w.sz * az) + V * (w.sz * bz) + W * (w.sz * cz);
-  const float rcp = 1.0f / det;
+  const float rcp = rcp_rn(det);  // beyond the float range: NaN, a miss
   t = T * rcp;
   if (!(t > kRayEps)) return false;
   u = V * rcp;
@@ -686,9 +705,17 @@ DVS_SHADE_INLINE __device__ bool trace_shadow_packet(const SceneView &S, float3 
 }
 
 
+// The float after a finite x in the direction of the sign of `to` (nextafterf toward +-infinity); x when `to` is zero.
+__device__ __forceinline__ float next_toward(float x, float to) {
+  const int b = __float_as_int(x);
+  const int step = (b >= 0) == (to > 0) ? 1 : -1;
+  const float y = x == 0.0f ? copysignf(__int_as_float(1), to) : __int_as_float(b + step);
+  return to != 0 ? y : x;
+}
+
 // shadow_origin (device_optics.cuh:37-51) from the leaf-order triangle record.
 __device__ float3 shadow_origin(float3 a, float3 e1, float3 e2, float u, float v, float3 light) {
-  float3 point = a + u * e1 + v * e2, normal = normalize(cross(e1, e2));
+  float3 point = a + u * e1 + v * e2, normal = unit(cross(e1, e2));
   if (dot(normal, light) < 0) normal = -normal;
   constexpr float epsilon = 5.960464477539063e-8f, gamma = 8 * epsilon / (1 - 8 * epsilon);
   float3 error = f3(gamma * (fabsf(a.x) + fabsf(u * e1.x) + fabsf(v * e2.x)),
@@ -697,10 +724,7 @@ __device__ float3 shadow_origin(float3 a, float3 e1, float3 e2, float u, float v
   float distance = fabsf(normal.x) * error.x + fabsf(normal.y) * error.y + fabsf(normal.z) * error.z + 1e-6f;
   float3 offset = normal * distance;
   point = point + offset;
-  if (offset.x != 0) point.x = nextafterf(point.x, copysignf(kInf(), offset.x));
-  if (offset.y != 0) point.y = nextafterf(point.y, copysignf(kInf(), offset.y));
-  if (offset.z != 0) point.z = nextafterf(point.z, copysignf(kInf(), offset.z));
-  return point;
+  return f3(next_toward(point.x, offset.x), next_toward(point.y, offset.y), next_toward(point.z, offset.z));
 }
 
 // shadow_origin from a record (a, b, c = its three float4s): the edges are
@@ -756,13 +780,13 @@ __device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool a
   const float3 origin = f3(pose.px, pose.py, pose.pz);
   const int ss = S.samples;
   const int px_i = pixel % S.width, py_i = pixel / S.width;
-  const HapkeConst hc = hapke_const(S.hapke);
-  const float3 lnorm = normalize(light);  // as in sample_pixel_group
+  const HapkeConst &hc = S.hc;
+  const float3 lnorm = unit(light);  // as in sample_pixel_group
   for (int sy = 0; sy < ss; ++sy)
     for (int sx = 0; sx < ss; ++sx) {
       const float px = subrays ? subrays[sy * ss + sx].px : subray_x(S, px_i, sx);
       const float py = subrays ? subrays[sy * ss + sx].py : subray_y(S, py_i, sy);
-      const float3 ray = normalize(rotate_ray(pose, f3(px, -py, -1)));
+      const float3 ray = unit(rotate_ray(pose, f3(px, -py, -1)));
       const HitRecord hit = trace_nearest_packet<kGeo>(S, origin, ray, active && out.valid, stack_code, stack_t);
       if (active && out.valid) ++out.primary;
       if (hit.hit < 0) out.valid = false;
@@ -780,7 +804,7 @@ __device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool a
           const float4 *q = reinterpret_cast<const float4 *>(sr);
           const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
           const float w = 1 - hit.u - hit.v;
-          normal = normalize(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit.u + f3(s2.x, s2.y, s2.z) * hit.v);
+          normal = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit.u + f3(s2.x, s2.y, s2.z) * hit.v);
           lit = !(dot(normal, light) <= 0 || dot(normal, -ray) <= 0);
           if (lit) {
             const float4 *r = tri_record<kGeo>(S, hit.tri, 2);
@@ -800,7 +824,7 @@ __device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool a
           if (lit && !occ) {
             const double cos4 = subrays ? subrays[sy * ss + sx].cos4 : cos4_of(px, py);
             // hapke_directional_reflectance (hapke.hpp:153-157)
-            const float3 n = normalize(normal), l = lnorm, v = normalize(-ray);
+            const float3 n = unit(normal), l = lnorm, v = unit(-ray);
             const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo, r0, S.hapke, hc);
             out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
           }
@@ -1109,12 +1133,383 @@ __device__ void trace_shadow_packet_r(const SceneView &S, const float3 (&o)[R], 
   __syncwarp();
 }
 
+// ---- beams: one walk of the tree for all the packets of a warp's item -------------------
+// A warp's item is many packets through nearly the same rays: every sub-ray of
+// a pixel (or of a few neighbouring pixels) at many circuit cells.  Walking the
+// tree from the root for each packet repeats the same node tests: on the
+// 1280x720 workload they were more than half of the trace's instructions, all
+// of them in one dependent chain of load, test and vote per level.  So the
+// warp walks the tree once for the bundle of all its rays (the beam) and keeps
+// the leaves the bundle may reach, decoded and sorted by entry distance, in
+// shared memory; each packet then tests only these.  A second list holds the
+// leaves between the beam's hit points and the light.
+//
+// The lists never change a result: a leaf's triangles are tested after the
+// ray's own slab test as before, and a leaf that is not in the list is one
+// that the ray's slab test fails (the beam's interval bounds are extremes of the same
+// rounded operations).  What the beam assumes of a ray -- its direction, or
+// its shadow origin, inside the beam's ranges -- is checked for every ray, and
+// a packet with a ray outside takes the general walk.  An item whose beam has no
+// one-signed direction, or reaches more leaves than a list holds, has no lists
+// and walks the tree for every packet, two sub-rays per lane.
+constexpr int kBeamLeaves = 32;  // one per lane
+struct Beam {                    // shared memory, one per warp
+  float4 leaf[kBeamLeaves][2];   // {lo, hi.x}, {hi.y, hi.z, first triangle, count}, nearest entry first
+  float4 shadow[kBeamLeaves][2];
+  float3 olo, ohi, dlo, dhi;     // ranges of the rays' origins and directions
+  float3 llo, lhi;               // range of the light directions' inverses
+  float3 slo, shi;               // range of the shadow origins
+};
+// What a warp holds of its item's lists: their lengths, and where shadow_in_list starts.
+struct BeamLists {
+  int leaves, shadow, first;
+};
+constexpr int kNoList = -1;  // a list's length when there is none
+
+__device__ __forceinline__ float3 min3(float3 a, float3 b) { return f3(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)); }
+__device__ __forceinline__ float3 max3(float3 a, float3 b) { return f3(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)); }
+__device__ __forceinline__ bool within(float3 v, float3 lo, float3 hi) {
+  return v.x >= lo.x && v.x <= hi.x && v.y >= lo.y && v.y <= hi.y && v.z >= lo.z && v.z <= hi.z;
+}
+__device__ __forceinline__ float wlow(float x) { return funord(__reduce_min_sync(kFull, ford(x))); }
+__device__ __forceinline__ float whigh(float x) { return funord(__reduce_max_sync(kFull, ford(x))); }
+__device__ __forceinline__ float3 wlow3(float3 v) { return f3(wlow(v.x), wlow(v.y), wlow(v.z)); }
+__device__ __forceinline__ float3 whigh3(float3 v) { return f3(whigh(v.x), whigh(v.y), whigh(v.z)); }
+
+// The interval bundle of given ranges; coherent means each axis' inverse direction keeps one sign.
+__device__ __forceinline__ Packet range_packet(float3 olo, float3 ohi, float3 ilo, float3 ihi) {
+  Packet P;
+  P.olo = olo; P.ohi = ohi; P.ilo = ilo; P.ihi = ihi;
+  P.nx = ihi.x < 0.0f;
+  P.ny = ihi.y < 0.0f;
+  P.nz = ihi.z < 0.0f;
+  P.coherent = (P.nx || ilo.x > 0.0f) && (P.ny || ilo.y > 0.0f) && (P.nz || ilo.z > 0.0f);
+  P.o_near = f3(P.nx ? olo.x : ohi.x, P.ny ? olo.y : ohi.y, P.nz ? olo.z : ohi.z);
+  P.o_far = f3(P.nx ? ohi.x : olo.x, P.ny ? ohi.y : olo.y, P.nz ? ohi.z : olo.z);
+  return P;
+}
+// The primary beam's bundle: 1/d of directions of one sign decreases with d, so the ends of the inverse's range are
+// the inverses of the ends, rounded outward by more than rcp_rn's last bit.  A range that holds zero on an axis (or comes so near it that
+// inverse_direction could clamp) has no such bundle.
+__device__ __forceinline__ float rcp_low(float d) { const float y = 1.0f / d; return y - 2.4e-7f * fabsf(y); }
+__device__ __forceinline__ float rcp_high(float d) { const float y = 1.0f / d; return y + 2.4e-7f * fabsf(y); }
+__device__ __forceinline__ bool one_sign(float lo, float hi) { return lo > 1e-18f || hi < -1e-18f; }
+__device__ __forceinline__ Packet primary_packet(const Beam &B) {
+  const float3 dlo = B.dlo, dhi = B.dhi;
+  Packet P = range_packet(B.olo, B.ohi, f3(rcp_low(dhi.x), rcp_low(dhi.y), rcp_low(dhi.z)),
+                          f3(rcp_high(dlo.x), rcp_high(dlo.y), rcp_high(dlo.z)));
+  P.coherent = one_sign(dlo.x, dhi.x) && one_sign(dlo.y, dhi.y) && one_sign(dlo.z, dhi.z);
+  return P;
+}
+__device__ __forceinline__ ChildRec list_leaf(const float4 (*list)[2], int i) {
+  const float4 a = list[i][0], b = list[i][1];
+  return ChildRec{f3(a.x, a.y, a.z), f3(a.w, b.x, b.y), __float_as_int(b.z), __float_as_int(b.w)};
+}
+
+// The leaves a bundle may reach, in no order: up to four nodes at a time, one
+// child per lane.  Returns their number, kNoList when they are more than the list holds.
+template <int kGeo>
+__device__ __forceinline__ int collect_leaves(const SceneView &S, const Packet &P, int *stack, float4 (*list)[2]) {
+  const int lane = threadIdx.x & 31, group = lane >> 3, slot = lane & 7;
+  const unsigned below = (1u << lane) - 1u;
+  int sp = 1, n = 0;
+  if (lane == 0) stack[0] = 0;
+  __syncwarp();
+  while (sp > 0) {
+    const int take = min(sp, 4);
+    sp -= take;
+    const int node = group < take ? stack[sp + group] : -1;
+    ChildRec c{};
+    bool hit = false;
+    if (node >= 0) {
+      float key;
+      c = load_child<kGeo>(S, node, slot);
+      hit = c.count >= 0 && packet_slab(c, P, kRayEps, 1e30f, key);
+    }
+    const unsigned leaves = __ballot_sync(kFull, hit && c.count > 0);
+    const unsigned inner = __ballot_sync(kFull, hit && c.count == 0);
+    const int nl = __popc(leaves), ni = __popc(inner);
+    if (n + nl > kBeamLeaves || sp + ni > kStackSlots) {
+      __syncwarp();
+      return kNoList;
+    }
+    if (hit) {
+      if (c.count > 0) {
+        float4 *q = list[n + __popc(leaves & below)];
+        q[0] = make_float4(c.lo.x, c.lo.y, c.lo.z, c.hi.x);
+        q[1] = make_float4(c.hi.y, c.hi.z, __int_as_float(c.child), __int_as_float(c.count));
+      } else {
+        stack[sp + __popc(inner & below)] = c.child;  // the nodes read above are below or in other lanes' registers
+      }
+    }
+    n += nl;
+    sp += ni;
+    __syncwarp();
+  }
+  return n;
+}
+
+// The primary list: the beam's leaves by entry distance (ties in walk order).
+template <int kGeo>
+__device__ __forceinline__ int build_primary_list(const SceneView &S, Beam &B, int *stack) {
+  const Packet P = primary_packet(B);
+  if (!P.coherent) return kNoList;
+  const int n = collect_leaves<kGeo>(S, P, stack, B.leaf);
+  if (n > 1) {
+    const int lane = threadIdx.x & 31;
+    float4 a, b;
+    float key = kInf();
+    if (lane < n) {
+      a = B.leaf[lane][0];
+      b = B.leaf[lane][1];
+      packet_slab(list_leaf(B.leaf, lane), P, kRayEps, 1e30f, key);
+    }
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const float kj = __shfl_sync(kFull, key, j);
+      rank += kj < key || (kj == key && j < lane) ? 1 : 0;
+    }
+    __syncwarp();
+    if (lane < n) {
+      B.leaf[rank][0] = a;
+      B.leaf[rank][1] = b;
+    }
+    __syncwarp();
+  }
+  return n;
+}
+
+// The shadow list.  The shadow origins lie on the list's triangles inside the
+// beam: per leaf the beam's entry and exit distance bound the hit points, cut to
+// the leaf's box; the margin covers the float hit point and shadow_origin's offset
+// (packets check their origins against the range).
+template <int kGeo>
+__device__ __forceinline__ int build_shadow_list(const SceneView &S, Beam &B, int n_leaf, int *stack) {
+  const int lane = threadIdx.x & 31;
+  const Packet P = primary_packet(B);
+  float3 lo = f3(kInf(), kInf(), kInf()), hi = -lo;
+  if (lane < n_leaf) {
+    const ChildRec c = list_leaf(B.leaf, lane);
+    float near, t0, t1;
+    packet_slab(c, P, kRayEps, 1e30f, near);
+    float L, U, far = 1e30f;
+    axis_bounds_fixed(c.lo.x, c.hi.x, P.nx, P.o_near.x, P.o_far.x, P.ilo.x, P.ihi.x, L, U);
+    far = fminf(far, U);
+    axis_bounds_fixed(c.lo.y, c.hi.y, P.ny, P.o_near.y, P.o_far.y, P.ilo.y, P.ihi.y, L, U);
+    far = fminf(far, U);
+    axis_bounds_fixed(c.lo.z, c.hi.z, P.nz, P.o_near.z, P.o_far.z, P.ilo.z, P.ihi.z, L, U);
+    far = fminf(far, U);
+    t0 = near;
+    t1 = fmaxf(far, near);
+    const float3 dlo = B.dlo, dhi = B.dhi;
+    lo = max3(c.lo, B.olo + min3(t0 * dlo, t1 * dlo));
+    hi = min3(c.hi, B.ohi + max3(t0 * dhi, t1 * dhi));
+    const float m = 3e-6f * fmaxf(fmaxf(fmaxf(fabsf(c.lo.x), fabsf(c.hi.x)), fmaxf(fabsf(c.lo.y), fabsf(c.hi.y))),
+                                  fmaxf(fabsf(c.lo.z), fabsf(c.hi.z))) + 1e-5f;
+    lo = lo - f3(m, m, m);
+    hi = hi + f3(m, m, m);
+  }
+  lo = wlow3(lo);
+  hi = whigh3(hi);
+  if (lane == 0) {
+    B.slo = lo;
+    B.shi = hi;
+  }
+  __syncwarp();
+  const Packet L = range_packet(lo, hi, B.llo, B.lhi);
+  if (!L.coherent) return kNoList;
+  return collect_leaves<kGeo>(S, L, stack, B.shadow);
+}
+
+// A longer list is first cut to the leaves the packet's own interval bundle may reach, one leaf per lane: the bundle's
+// extremes and the test cost about as much as five leaves tested by every ray.
+constexpr int kListFilter = 5;
+__device__ __forceinline__ unsigned list_mask(const float4 (*list)[2], int n, const Packet &P) {
+  const int lane = threadIdx.x & 31;
+  bool hit = false;
+  if (lane < n) {
+    float key;
+    hit = packet_slab(list_leaf(list, lane), P, kRayEps, 1e30f, key);
+  }
+  return __ballot_sync(kFull, hit);
+}
+__device__ __forceinline__ unsigned whole_list(int n) { return n >= 32 ? kFull : (1u << n) - 1u; }
+// The extremes of a packet's R vectors per lane, live ones only.
+template <int R>
+__device__ __forceinline__ void packet_range(const float3 (&v)[R], const bool (&live)[R], float3 &lo, float3 &hi) {
+  lo = f3(kInf(), kInf(), kInf());
+  hi = -lo;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (live[r]) {
+      lo = min3(lo, v[r]);
+      hi = max3(hi, v[r]);
+    }
+  lo = wlow3(lo);
+  hi = whigh3(hi);
+}
+
+// The general walks, out of line: they serve the packets no list holds for.
+template <int R>
+struct PacketRays {
+  float3 o[R], d[R];
+  bool live[R];
+};
+template <int R>
+struct PacketHits {
+  HitRecord h[R];
+};
+template <int R, int kGeo>
+__device__ __noinline__ PacketHits<R> nearest_general(const SceneView &S, PacketRays<R> in, int *stack_code,
+                                                      float *stack_t) {
+  PacketHits<R> out;
+  trace_nearest_packet_r<R, kGeo>(S, in.o, in.d, in.live, stack_code, stack_t, out.h);
+  return out;
+}
+template <int R>
+struct ShadowRays {
+  float3 o[R], light;
+  int self[R];
+  bool live[R];
+};
+template <int R, int kGeo>
+__device__ __noinline__ unsigned shadow_general(const SceneView &S, ShadowRays<R> in, int *stack_code,
+                                                float *stack_t) {
+  bool occ[R];
+  trace_shadow_packet_r<R, kGeo>(S, in.o, in.light, shadow_dir<kGeo>(in.light), in.live, in.self, stack_code, stack_t,
+                                 occ);
+  unsigned m = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) m |= occ[r] ? 1u << r : 0u;
+  return m;
+}
+
+// Nearest hits of a packet from the beam's list (trace_nearest_packet_r's leaves, nearest first).
+template <int R, int kGeo>
+__device__ __forceinline__ void nearest_in_list(const SceneView &S, const Beam &B, int n, float3 o,
+                                                const float3 (&d)[R], const bool (&live)[R], HitRecord (&h)[R]) {
+  float3 idir[R], op[R];
+  float closest[R];
+  WtRay wr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    idir[r] = inverse_direction(d[r]);
+    wr[r] = wt_ray<kGeo>(d[r]);
+    op[r] = wt_origin<kGeo>(wr[r], o);
+    closest[r] = live[r] ? 1e30f : -1.0f;
+    h[r] = HitRecord{0, -1, 0.f, 0.f, 0.f};
+  }
+  unsigned left = whole_list(n);
+  if (n > kListFilter) {
+    float3 ilo, ihi;
+    packet_range<R>(idir, live, ilo, ihi);
+    left = list_mask(B.leaf, n, range_packet(B.olo, B.ohi, ilo, ihi));  // one-signed, as the beam
+  }
+  for (; left; left &= left - 1u) {
+    const ChildRec c = list_leaf(B.leaf, __ffs(left) - 1);
+    bool need[R], any = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float tn;
+      need[r] = live[r] && slab(c.lo, c.hi, o, idir[r], kRayEps, closest[r], tn);
+      any = any || need[r];
+    }
+    if (!__any_sync(kFull, any)) continue;
+    for (int k = 0; k < c.count; ++k) {
+      const float4 *q4 = tri_record<kGeo>(S, c.child + k, wr[0].kz);
+      float4 a = __ldg(q4), b = __ldg(q4 + 1), q = __ldg(q4 + 2);
+      int loaded = wr[0].kz;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if constexpr ((kGeo & kGeoWatertight) != 0) {
+          if (wr[r].kz != loaded) {
+            const float4 *p4 = tri_record<kGeo>(S, c.child + k, wr[r].kz);
+            a = __ldg(p4);
+            b = __ldg(p4 + 1);
+            q = __ldg(p4 + 2);
+            loaded = wr[r].kz;
+          }
+        }
+        float t, u, v;
+        if (need[r] && tri_hit<kGeo>(wr[r], d[r], o, op[r], a, b, q, t, u, v) && t < closest[r]) {
+          closest[r] = t;
+          h[r].hit = 1; h[r].tri = c.child + k; h[r].t = t; h[r].u = u; h[r].v = v;
+        }
+      }
+    }
+  }
+}
+
+// Occlusion of a packet's shadow rays from the shadow list; `first`: where to
+// start, the leaf that last occluded a ray of this item (any hit ends a ray,
+// so the order decides nothing but the time).
+template <int R, int kGeo>
+__device__ __forceinline__ unsigned shadow_in_list(const SceneView &S, const Beam &B, int n, const float3 (&o)[R],
+                                                   float3 light, const ShadowDir &sd, const bool (&live)[R],
+                                                   const int (&self)[R], int &first) {
+  const float t_max = 1e30f;
+  unsigned occluded = 0;
+  float3 op[R];
+  bool alive[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    op[r] = wt_origin<kGeo>(sd.wr, o[r]);
+    alive[r] = live[r];
+  }
+  unsigned left = whole_list(n);
+  if (n > kListFilter) {
+    float3 olo, ohi;
+    packet_range<R>(o, live, olo, ohi);
+    left = list_mask(B.shadow, n, range_packet(olo, ohi, B.llo, B.lhi));
+  }
+  left = __funnelshift_r(left, left, first);  // bit j: leaf (first + j) mod 32
+  const int start = first;
+  for (; left; left &= left - 1u) {
+    const int i = (start + __ffs(left) - 1) & 31;
+    const ChildRec c = list_leaf(B.shadow, i);
+    bool need[R], any = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float tn;
+      need[r] = alive[r] && slab(c.lo, c.hi, o[r], sd.idir, kRayEps, t_max, tn);
+      any = any || need[r];
+    }
+    if (__any_sync(kFull, any)) {
+      const unsigned before = occluded;
+      for (int k = 0; k < c.count; ++k) {
+        const int id = c.child + k;
+        const float4 *q4 = tri_record<kGeo>(S, id, sd.wr.kz);
+        const float4 a = __ldg(q4), b = __ldg(q4 + 1), q = __ldg(q4 + 2);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float t, u, v;
+          if (need[r] && alive[r] && id != self[r] &&
+              tri_hit<kGeo>(sd.wr, light, o[r], op[r], a, b, q, t, u, v) && t > kRayEps && t < t_max) {
+            occluded |= 1u << r;
+            alive[r] = false;
+          }
+        }
+      }
+      if (__any_sync(kFull, occluded != before)) {
+        first = i;
+        bool some = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) some = some || alive[r];
+        if (!__any_sync(kFull, some)) break;
+      }
+    }
+  }
+  return occluded;
+}
+
 // sample_pixel_packet with R neighbouring sub-rays per lane (ss^2 a multiple
 // of R).  The per-ray work, the order of the FP64 radiance and depth sums and
 // the ray counts are those of the one-ray loop.
-template <int kMode, int R, int kGeo = kGeoReference>
-__device__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool active, const CellPose &pose,
-                                          int *stack_code, float *stack_t, const SubraySample *subrays) {
+// kBeam: the item has lists, and the packet's leaves come from them where its rays are inside the beam.
+template <int kMode, int R, int kGeo, bool kBeam>
+__device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool active,
+                                                          const CellPose &pose, int *stack_code, float *stack_t,
+                                                          const SubraySample *subrays, Beam &B, BeamLists &lists) {
   PixelSample out{0.0, -1.0f, true, 0u, 0u};
   double depth = 0;
   int valid_depth = 0;
@@ -1122,15 +1517,15 @@ __device__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool ac
   const float3 origin = f3(pose.px, pose.py, pose.pz);
   const int ss = S.samples, n_sub = ss * ss;
   const int px_i = pixel % S.width, py_i = pixel / S.width;
-  const HapkeConst hc = hapke_const(S.hapke);
+  const HapkeConst &hc = S.hc;
   // hapke_directional_reflectance normalizes the light for every shaded ray
   // (hapke.hpp:153-157); it is the same vector for all of this lane's rays
-  const float3 lnorm = normalize(light);
+  const float3 lnorm = unit(light);
   const ShadowDir sdir = shadow_dir<kGeo>(light);
   for (int j = 0; j < n_sub; j += R) {
     float px[R], py[R];
-    float3 ray[R], org[R];
-    bool live[R];
+    float3 ray[R];
+    bool live[R], inside = true;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (subrays) {
@@ -1141,12 +1536,30 @@ __device__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool ac
         px[r] = subray_x(S, px_i, sx);
         py[r] = subray_y(S, py_i, sy);
       }
-      ray[r] = normalize(rotate_ray(pose, f3(px[r], -py[r], -1)));
-      org[r] = origin;
+      ray[r] = unit(rotate_ray(pose, f3(px[r], -py[r], -1)));
       live[r] = active && out.valid;
+      if constexpr (kBeam) inside = inside && (!live[r] || within(ray[r], B.dlo, B.dhi));
     }
     HitRecord hit[R];
-    trace_nearest_packet_r<R, kGeo>(S, org, ray, live, stack_code, stack_t, hit);
+    if constexpr (!kBeam) {
+      float3 org[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) org[r] = origin;
+      trace_nearest_packet_r<R, kGeo>(S, org, ray, live, stack_code, stack_t, hit);
+    } else if (__all_sync(kFull, inside)) {
+      nearest_in_list<R, kGeo>(S, B, lists.leaves, origin, ray, live, hit);
+    } else {
+      PacketRays<R> in;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        in.o[r] = origin;
+        in.d[r] = ray[r];
+        in.live[r] = live[r];
+      }
+      const PacketHits<R> got = nearest_general<R, kGeo>(S, in, stack_code, stack_t);
+#pragma unroll
+      for (int r = 0; r < R; ++r) hit[r] = got.h[r];
+    }
     bool lit[R];
     float3 normal[R], sorigin[R];
     float albedo[R], r0[R];
@@ -1171,7 +1584,7 @@ __device__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool ac
           const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[r].tri);
           const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
           const float w = 1 - hit[r].u - hit[r].v;
-          normal[r] = normalize(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u +
+          normal[r] = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u +
                                 f3(s2.x, s2.y, s2.z) * hit[r].v);
           lit[r] = !(dot(normal[r], light) <= 0 || dot(normal[r], -ray[r]) <= 0);
           if (lit[r]) {
@@ -1191,14 +1604,36 @@ __device__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool ac
 #pragma unroll
       for (int r = 0; r < R; ++r) any_lit = any_lit || lit[r];
       if (__any_sync(kFull, any_lit)) {
-        bool occ[R];
-        trace_shadow_packet_r<R, kGeo>(S, sorigin, light, sdir, lit, self, stack_code, stack_t, occ);
+        unsigned occluded = 0;
+        bool near = true;
+        if constexpr (kBeam) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) near = near && (!lit[r] || within(sorigin[r], B.slo, B.shi));
+        }
+        if constexpr (!kBeam) {
+          bool occ[R];
+          trace_shadow_packet_r<R, kGeo>(S, sorigin, light, sdir, lit, self, stack_code, stack_t, occ);
+#pragma unroll
+          for (int r = 0; r < R; ++r) occluded |= occ[r] ? 1u << r : 0u;
+        } else if (__all_sync(kFull, near)) {
+          occluded = shadow_in_list<R, kGeo>(S, B, lists.shadow, sorigin, light, sdir, lit, self, lists.first);
+        } else {
+          ShadowRays<R> in;
+          in.light = light;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            in.o[r] = sorigin[r];
+            in.self[r] = self[r];
+            in.live[r] = lit[r];
+          }
+          occluded = shadow_general<R, kGeo>(S, in, stack_code, stack_t);
+        }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           if (lit[r]) ++out.shadow;
-          if (lit[r] && !occ[r]) {
+          if (lit[r] && !((occluded >> r) & 1u)) {
             const double cos4 = subrays ? subrays[j + r].cos4 : cos4_of(px[r], py[r]);
-            const float3 n = normalize(normal[r]), l = lnorm, v = normalize(-ray[r]);
+            const float3 n = unit(normal[r]), l = lnorm, v = unit(-ray[r]);
             const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], S.hapke, hc);
             out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
           }
@@ -1230,8 +1665,8 @@ __device__ PixelSample sample_pixel_subrays(const SceneView &S, int pixel, const
   const float3 origin = f3(pose.px, pose.py, pose.pz);
   const int ss = S.samples, n_sub = ss * ss;
   const int px_i = pixel % S.width, py_i = pixel / S.width;
-  const HapkeConst hc = hapke_const(S.hapke);
-  const float3 lnorm = normalize(light);  // as in sample_pixel_group
+  const HapkeConst &hc = S.hc;
+  const float3 lnorm = unit(light);  // as in sample_pixel_group
   const ShadowDir sdir = shadow_dir<kGeo>(light);
   bool valid = true;
   for (int g = 0; g < n_sub; g += 32 * R) {
@@ -1245,7 +1680,7 @@ __device__ PixelSample sample_pixel_subrays(const SceneView &S, int pixel, const
       const int jj = j < n_sub ? j : 0;
       px[r] = subray_x(S, px_i, jj % ss);
       py[r] = subray_y(S, py_i, jj / ss);
-      ray[r] = normalize(rotate_ray(pose, f3(px[r], -py[r], -1)));
+      ray[r] = unit(rotate_ray(pose, f3(px[r], -py[r], -1)));
       org[r] = origin;
     }
     HitRecord hit[R];
@@ -1268,7 +1703,7 @@ __device__ PixelSample sample_pixel_subrays(const SceneView &S, int pixel, const
         const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[r].tri);
         const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
         const float w = 1 - hit[r].u - hit[r].v;
-        normal[r] = normalize(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u +
+        normal[r] = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u +
                               f3(s2.x, s2.y, s2.z) * hit[r].v);
         lit[r] = !(dot(normal[r], light) <= 0 || dot(normal[r], -ray[r]) <= 0);
         if (lit[r]) {
@@ -1290,7 +1725,7 @@ __device__ PixelSample sample_pixel_subrays(const SceneView &S, int pixel, const
       for (int r = 0; r < R; ++r)
         if (lit[r] && !occ[r]) {
           const double cos4 = cos4_of(px[r], py[r]);
-          const float3 n = normalize(normal[r]), l = lnorm, v = normalize(-ray[r]);
+          const float3 n = unit(normal[r]), l = lnorm, v = unit(-ray[r]);
           const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], S.hapke, hc);
           term[r] = fmaxf(0, n_h * pose.intensity) * cos4;
         }

@@ -31,6 +31,8 @@ namespace dvsgb {
 namespace {
 
 // ---- kernels ------------------------------------------------------------------------
+__global__ void hapke_const_kernel(dvs_hapke p, HapkeConst *out) { *out = hapke_const(p); }
+
 __global__ void pose_from_state_kernel(const dvs_optical_state *state, CellPose *out) {
   // A pose used as given (initialize_pixels, event_sensor.cu:22): the
   // quaternion is not renormalized; only the light is normalized.
@@ -65,19 +67,20 @@ __global__ void cell_poses_kernel(const dvs_optical_interval *ivs, const Cell *c
 }
 
 
-template <int kMode, int kRays, int kGeo>
+template <int kMode, int kRays, int kGeo, bool kBeam>
 __global__ void __launch_bounds__(128, kRays == 4   ? DVS_TRACE_QUAD_MIN_BLOCKS
                                        : kRays == 2 ? DVS_TRACE_PAIR_MIN_BLOCKS
+                                       : kBeam      ? DVS_TRACE_BEAM_MIN_BLOCKS
                                                     : DVS_TRACE_MIN_BLOCKS)
-    trace_cells_kernel(SceneView S, int n_pix, const int32_t *rank_list, const CellPose *poses, int c0, int nc,
-                       int cw_log2, double *radiance, float *depth_out, unsigned long long *counters) {
-  __shared__ int s_code[kWarpsPerBlock][kStackSlots];
-  __shared__ float s_t[kWarpsPerBlock][kStackSlots];
-  __shared__ SubraySample s_subrays[kWarpsPerBlock][kSubrayTable];
+    trace_cells_kernel(const __grid_constant__ SceneView S, int n_pix, const int32_t *rank_list, const CellPose *poses,
+                       int c0, int nc, ItemShape shape, double *radiance, float *depth_out,
+                       unsigned long long *counters) {
+  __shared__ TraceShared s_warp[kWarpsPerBlock];
+  __shared__ Beam s_beam[kBeam ? kWarpsPerBlock : 1];
   const int wib = threadIdx.x >> 5;
-  const long long warp = (long long)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  trace_cells_item<kMode, kRays, kGeo>(S, n_pix, rank_list, poses, c0, nc, cw_log2, radiance, depth_out, counters,
-                                       warp, s_code[wib], s_t[wib], s_subrays[wib]);
+  const long long item = (long long)blockIdx.x * kWarpsPerBlock + wib;
+  trace_cells_item<kMode, kRays, kGeo, kBeam>(S, n_pix, rank_list, poses, c0, nc, shape, radiance, depth_out, counters, item,
+                                       s_warp[wib], s_beam[kBeam ? wib : 0]);
 }
 
 // Few poses per pixel: one warp per (pixel, pose), lanes carrying the
@@ -264,6 +267,11 @@ cudaError_t launch_poisson_draws(int generator, double lambda, unsigned seed, in
 }
 
 // ---- launchers ----------------------------------------------------------------------
+cudaError_t launch_hapke_const(const dvs_hapke &hapke, HapkeConst *out, cudaStream_t s) {
+  hapke_const_kernel<<<1, 1, 0, s>>>(hapke, out);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_pose_from_state(const dvs_optical_state *state, CellPose *out, cudaStream_t s) {
   pose_from_state_kernel<<<1, 32, 0, s>>>(state, out);
   return cudaGetLastError();
@@ -303,17 +311,19 @@ void trace_list_geo(const SceneView &scene, int n_pix, const int32_t *rank_list,
                                                                 nullptr, counters);
     return;
   }
-  const int cw = 1 << cw_log2, ppw = 32 >> cw_log2;
-  const long long warps = (long long)((n_pix + ppw - 1) / ppw) * ((nc + cw - 1) / cw);
   const int ss2 = scene.samples * scene.samples;
-  // four rays per lane only in the reference format (the others keep two)
-  const int rays = (kGeo == kGeoReference && scene.rays >= 4 && ss2 % 4 == 0) ? 4
-                   : (scene.rays >= 2 && ss2 % 2 == 0)                       ? 2
-                                                                              : 1;
-  const int grid = blocks(warps * 32, 128);
+  const int rays = trace_rays(scene, n_pix, nc, cw_log2, rank_list != nullptr);
+  const ItemShape shape = trace_item_shape(n_pix, nc, cw_log2, ss2, rays, rank_list != nullptr);
+  const int grid = blocks(trace_job_items(n_pix, nc, shape) * 32, 128);
 #define DVS_TRACE_LAUNCH(MODE, RAYS, DEPTH)                                                                         \
-  trace_cells_kernel<MODE, RAYS, kGeo><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, cw_log2,       \
-                                                            radiance, DEPTH, counters)
+  do {                                                                                                              \
+    if (shape.beam)                                                                                                 \
+      trace_cells_kernel<MODE, RAYS, kGeo, true><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc,       \
+                                                                      shape, radiance, DEPTH, counters);            \
+    else                                                                                                            \
+      trace_cells_kernel<MODE, RAYS, kGeo, false><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc,      \
+                                                                       shape, radiance, DEPTH, counters);           \
+  } while (0)
   if (depth) {
     if constexpr (kGeo == kGeoReference)
       if (rays == 4) { DVS_TRACE_LAUNCH(kRadianceDepth, 4, depth); return; }
@@ -423,18 +433,24 @@ cudaError_t launch_event_depth(const SceneView &scene, const dvs_optical_interva
 }
 
 namespace {
+template <int kMode, int kRays, int kGeo>
+cudaError_t preload_cells() {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, true>);
+  return e == cudaSuccess ? cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, false>) : e;
+}
 template <int kGeo>
 cudaError_t preload_camera_geo() {
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, trace_subray_kernel<kRadianceDepth, kGeo>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_subray_kernel<kRadiance, kGeo>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadianceDepth, 1, kGeo>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadianceDepth, 2, kGeo>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadiance, 1, kGeo>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadiance, 2, kGeo>);
+  if (e == cudaSuccess) e = preload_cells<kRadianceDepth, 1, kGeo>();
+  if (e == cudaSuccess) e = preload_cells<kRadianceDepth, 2, kGeo>();
+  if (e == cudaSuccess) e = preload_cells<kRadiance, 1, kGeo>();
+  if (e == cudaSuccess) e = preload_cells<kRadiance, 2, kGeo>();
   if constexpr (kGeo == kGeoReference) {
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadianceDepth, 4, kGeo>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kRadiance, 4, kGeo>);
+    if (e == cudaSuccess) e = preload_cells<kRadianceDepth, 4, kGeo>();
+    if (e == cudaSuccess) e = preload_cells<kRadiance, 4, kGeo>();
   }
   return e;
 }

@@ -8,6 +8,16 @@
 
 namespace dvsgb {
 
+// Material constants of the Hapke model, formed on the device once per scene (launch_hapke_const).
+struct HapkeConst {
+  float K, inv_K;            // porosity factor and its reciprocal
+  float tan_t, cot_t, chi;   // mean slope thetap: tan, cot and chi(thetap)
+  float r0_w;                // the H-function's r0 at the scene's single-scattering albedo
+  float tg_max;              // cap of tan(phase / 2)
+  float lobe_pos, lobe_neg;  // numerators of the two Henyey-Greenstein lobes
+  float inv_hS;              // 1 / hS
+  int32_t rough;             // thetap > 1e-8
+};
 struct SceneView {
   const BvhNode *nodes;       // reference geometry (FP32 child bounds)
   const BvhQNode *qnodes;     // FP16 child bounds (geometry bit 0), same indices
@@ -19,7 +29,8 @@ struct SceneView {
   float fx, fy, cx, cy;
   float coherent_span;  // largest origin spread a warp packet traverses as one interval bundle
   dvs_hapke hapke;
-  int32_t rays;         // sub-rays a lane may carry: 1, 2 or 4 (used when samples^2 is a multiple)
+  HapkeConst hc;
+  int32_t rays;         // sub-rays a lane may carry: 1, 2 or 4 (used when samples^2 is a multiple), 0 = automatic
   int32_t radiance_f32; // 1: the radiance chunk is written as float (read by an FP32 circuit), 0: as double
 };
 
@@ -124,6 +135,7 @@ struct OpticalKnot {
 enum : int { kRefTraced = 0, kRefFallback = 1, kRefMaxKnots = 2, kRefExactSegments = 3, kRefSlots = 4 };
 
 // ---- launchers (return cudaGetLastError()) ----------------------------------
+cudaError_t launch_hapke_const(const dvs_hapke &hapke, HapkeConst *out, cudaStream_t s);
 cudaError_t launch_pose_from_state(const dvs_optical_state *state, CellPose *out, cudaStream_t s);
 cudaError_t launch_poses_from_states(const dvs_optical_state *states, int n, CellPose *out, cudaStream_t s);
 // Motion-blur exposure: image[pixel] = sum_j float(radiance[j][rank]) * weights[j], in pose order.
@@ -138,16 +150,23 @@ cudaError_t launch_cell_poses(const dvs_optical_interval *ivs, const Cell *cells
 // into its radiance chunk.  first_item: the first work item (warp packet) of
 // this sensor in the batch's item space; items are job-major.
 constexpr int kMaxBatchJobs = 128;
+// A warp's item in a trace launch: `sets` pixel sets of 32 >> cw_log2
+// Morton-adjacent pixels x `groups` groups of 1 << cw_log2 cells; beam: the
+// item holds enough packets to walk the tree once for all of them.
+struct ItemShape {
+  int32_t cw_log2, sets, groups, beam;
+};
 struct TraceJob {
   SceneView view;
   const CellPose *poses;
   double *radiance;
   unsigned long long *counters;
   long long first_item;
-  int32_t n_pix, c0, nc, cw_log2;
+  int32_t n_pix, c0, nc, pad;
+  ItemShape shape;
 };
 // A trace launch's whole job table, passed as the kernel's parameter block
-// (22.5 KB at 128 jobs, within the 32 KB parameter limit).
+// (24.6 KB at 128 jobs, within the 32 KB parameter limit).
 struct TraceJobs {
   TraceJob jobs[kMaxBatchJobs];
   long long total_items;
@@ -169,8 +188,12 @@ struct CircuitJob {
   unsigned long long *counters;
   int32_t n, c0, nc, max_events, first_block, pad;
 };
-// Work items of one sensor's trace share (warp packets of cw_log2 cells).
-long long trace_job_items(int n_pix, int nc, int cw_log2);
+// The sub-rays per lane a trace of this view runs with: the view's, or automatically one where its items hold beams
+// and two (when the sub-ray count is even) where they do not.
+int trace_rays(const SceneView &view, int n_pix, int nc, int cw_log2, bool scattered);
+// The item shape of a trace of n_pix pixels (neighbours in rank order, or scattered ones) x nc cells, and its items.
+ItemShape trace_item_shape(int n_pix, int nc, int cw_log2, int sub_rays, int rays, bool scattered);
+long long trace_job_items(int n_pix, int nc, const ItemShape &shape);
 // Persistent trace of every job's items: a grid of resident blocks whose warps
 // pull items from jobs.next_item (zeroed by the caller on the same stream).
 // rays: 1 or 2 sub-rays per lane for every job; geometry: the jobs' shared

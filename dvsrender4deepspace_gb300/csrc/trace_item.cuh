@@ -17,6 +17,16 @@ constexpr int kWarpsPerBlock = 4;  // all ray kernels launch 128 threads
 #endif
 constexpr int kSubrayTable = 256;  // sub-rays per pixel with a shared sub-ray table (ss <= 16)
 
+// A wider bundle of directions (the sum of its extents per axis) takes no beam.
+constexpr float kBeamSpread = 0.1f;
+// A warp's shared memory in the trace kernels: the traversal stack and the
+// sub-ray table (and, in kernels with beams, a Beam beside it).
+struct TraceShared {
+  int code[kStackSlots];
+  float t[kStackSlots];
+  SubraySample subrays[kSubrayTable];
+};
+
 // Element o of a radiance chunk: double, or float when the chunk feeds an
 // FP32 circuit (which uses the value as a float: the same bits, half the bytes).
 __device__ __forceinline__ void store_radiance(const SceneView &S, double *chunk, size_t o, double value) {
@@ -29,64 +39,152 @@ __device__ __forceinline__ void store_radiance(const SceneView &S, double *chunk
 #ifndef DVS_TRACE_PAIR_MIN_BLOCKS
 #define DVS_TRACE_PAIR_MIN_BLOCKS 4
 #endif
+#ifndef DVS_TRACE_BEAM_MIN_BLOCKS
+#define DVS_TRACE_BEAM_MIN_BLOCKS 4
+#endif
 #ifndef DVS_TRACE_QUAD_MIN_BLOCKS
 #define DVS_TRACE_QUAD_MIN_BLOCKS 3
 #endif
 
-// One warp's share of a trace launch: warp item `warp` of the (pixel group,
-// cell group) grid of one sensor -- 32/CW Morton-adjacent pixels x CW
-// consecutive cells.  Called by trace_cells_kernel (one item per warp) and by
-// the batch's persistent kernel (items pulled from a work counter).
-template <int kMode, int kRays, int kGeo>
-__device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, const int32_t *rank_list,
-                                                 const CellPose *poses, int c0, int nc, int cw_log2,
-                                                 double *radiance, float *depth_out, unsigned long long *counters,
-                                                 long long warp, int *stack_code, float *stack_t,
-                                                 SubraySample *subrays) {
-  // n_pix pixels: all Morton ranks, or the ranks listed in rank_list
-  const int lane = threadIdx.x & 31;
-  const int cw = 1 << cw_log2, ppw = 32 >> cw_log2;
-  const int n_groups = (nc + cw - 1) >> cw_log2;
-  const long long pgroup = warp / n_groups;
-  const int g = (int)(warp % n_groups);
-  if (pgroup * ppw >= n_pix) return;  // warp-uniform
-  const int rank = (int)(pgroup * ppw) + (lane >> cw_log2);
-  const int cell = g * cw + (lane & (cw - 1));
-  const bool active = rank < n_pix && cell < nc;
-  const int pixel = rank < n_pix ? __ldg(S.pixel_of_rank + (rank_list ? rank_list[rank] : rank)) : 0;
-  const CellPose pose = poses[c0 + (active ? cell : 0)];
-  const int ss2 = S.samples * S.samples;
-  // the warp's ppw pixels: their sub-rays' coordinates and FP64 cos^4 once per
-  // warp (entry p * ss2 + j: sub-ray j of the pixel in lanes p * cw ...)
-  const int table = ppw * ss2;
-  const bool shared_subrays = kMode != kDepthOnly && table <= kSubrayTable;
-  if (shared_subrays) {
-    for (int q0 = 0; q0 < table; q0 += 32) {  // warp-uniform: every lane takes part in the shuffle
-      const int q = q0 + lane, p = min(q / ss2, ppw - 1);
-      const int pix = __shfl_sync(kFull, pixel, p << cw_log2);
-      if (q < table) {
-        const int j = q - p * ss2;
-        const float x = subray_x(S, pix % S.width, j % S.samples), y = subray_y(S, pix / S.width, j / S.samples);
-        subrays[q] = SubraySample{cos4_of(x, y), x, y};
+// The ranges of every ray of an item -- its pixel sets [s0, s1) at its cell
+// groups [g0, g1) -- into the beam, and its leaf list.  Directions: the
+// corner sub-rays of each pixel at each cell.  Between the corners a
+// normalized direction bends by at most about its extent squared; the margin
+// covers that, and each packet checks its rays against the range.
+template <int kGeo>
+__device__ __forceinline__ BeamLists begin_beam(const SceneView &S, int n_pix, const int32_t *rank_list,
+                                                const CellPose *poses, int c0, int nc, int cw_log2, int s0, int s1,
+                                                int g0, int g1, Beam &B, int *stack) {
+  const int lane = threadIdx.x & 31, cw = 1 << cw_log2, ppw = 32 >> cw_log2, last = S.samples - 1;
+  const float inf = kInf();
+  float3 olo = f3(inf, inf, inf), ohi = -olo, dlo = olo, dhi = -olo, llo = olo, lhi = -olo;
+  for (int s = s0; s < s1; ++s) {
+    const int rank = s * ppw + (lane >> cw_log2);
+    const int pixel = rank < n_pix ? __ldg(S.pixel_of_rank + (rank_list ? rank_list[rank] : rank)) : 0;
+    const int px_i = pixel % S.width, py_i = pixel / S.width;
+    const float x0 = subray_x(S, px_i, 0), x1 = subray_x(S, px_i, last);
+    const float y0 = subray_y(S, py_i, 0), y1 = subray_y(S, py_i, last);
+    for (int g = g0; g < g1; ++g) {
+      const int cell = g * cw + (lane & (cw - 1));
+      if (rank >= n_pix || cell >= nc) continue;
+      const CellPose pose = poses[c0 + cell];
+      const float3 o = f3(pose.px, pose.py, pose.pz), l = inverse_direction(f3(pose.lx, pose.ly, pose.lz));
+      olo = min3(olo, o);
+      ohi = max3(ohi, o);
+      llo = min3(llo, l);
+      lhi = max3(lhi, l);
+      for (int k = 0; k < (last ? 4 : 1); ++k) {
+        const float3 d = unit(rotate_ray(pose, f3(k & 1 ? x1 : x0, -(k & 2 ? y1 : y0), -1)));
+        dlo = min3(dlo, d);
+        dhi = max3(dhi, d);
       }
     }
-    __syncwarp();
   }
-  const SubraySample *mine = shared_subrays ? subrays + (lane >> cw_log2) * ss2 : nullptr;
-  const PixelSample s =
-      kRays > 1 ? sample_pixel_group<kMode, kRays, kGeo>(S, pixel, active, pose, stack_code, stack_t, mine)
-                : sample_pixel_packet<kMode, kGeo>(S, pixel, active, pose, stack_code, stack_t, mine);
-  if (active) {
-    const size_t o = (size_t)cell * n_pix + rank;
-    store_radiance(S, radiance, o, s.valid ? s.radiance : __longlong_as_double(0x7ff8000000000000ll));
-    if (depth_out) depth_out[o] = s.depth;
+  olo = wlow3(olo);
+  ohi = whigh3(ohi);
+  dlo = wlow3(dlo);
+  dhi = whigh3(dhi);
+  llo = wlow3(llo);
+  lhi = whigh3(lhi);
+  const float ext = (dhi.x - dlo.x) + (dhi.y - dlo.y) + (dhi.z - dlo.z);
+  BeamLists lists{kNoList, kNoList, 0};
+  if (!(ext <= kBeamSpread)) return lists;  // a wide bundle reaches too many leaves (or a ray has no direction)
+  const float m = ext * ext + 4e-7f;
+  if (lane == 0) {
+    B.olo = olo;
+    B.ohi = ohi;
+    B.dlo = dlo - f3(m, m, m);
+    B.dhi = dhi + f3(m, m, m);
+    B.llo = llo;
+    B.lhi = lhi;
   }
-  const unsigned prim = warp_sum(s.primary), shad = warp_sum(s.shadow);
+  __syncwarp();
+  lists.leaves = build_primary_list<kGeo>(S, B, stack);
+  if (lists.leaves >= 0) lists.shadow = build_shadow_list<kGeo>(S, B, lists.leaves, stack);
+  return lists;
+}
+
+// The packets of an item without lists, out of line (few items of a launch with beams): two sub-rays per lane where
+// their count is even, as a launch without beams.
+template <int kMode, int kGeo>
+__device__ __noinline__ PixelSample sample_without_beam(const SceneView &S, int pixel, bool active,
+                                                        const CellPose &pose, TraceShared &sh,
+                                                        const SubraySample *subrays) {
+  BeamLists none{kNoList, kNoList, 0};
+  Beam &unused = *reinterpret_cast<Beam *>(&sh);  // not touched without lists
+  if (S.samples % 2 == 0)
+    return sample_pixel_group<kMode, 2, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
+  return sample_pixel_group<kMode, 1, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
+}
+
+// One warp's item of a trace launch: shape.sets pixel sets (32/CW
+// Morton-adjacent pixels each) x shape.groups cell groups (CW consecutive
+// cells each) of one sensor, a packet of 32 x kRays rays at a time.  Called by
+// trace_cells_kernel (one item per warp) and by the batch's persistent kernel
+// (items pulled from a work counter).
+template <int kMode, int kRays, int kGeo, bool kBeam>
+__device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, const int32_t *rank_list,
+                                                 const CellPose *poses, int c0, int nc, ItemShape shape,
+                                                 double *radiance, float *depth_out, unsigned long long *counters,
+                                                 long long item, TraceShared &sh, Beam &beam) {
+  // n_pix pixels: all Morton ranks, or the ranks listed in rank_list
+  const int lane = threadIdx.x & 31, cw_log2 = shape.cw_log2;
+  const int cw = 1 << cw_log2, ppw = 32 >> cw_log2;
+  const int n_groups = (nc + cw - 1) >> cw_log2, n_sets = (n_pix + ppw - 1) / ppw;
+  const int per_set = (n_groups + shape.groups - 1) / shape.groups;
+  const long long first_set = item / per_set * shape.sets;
+  if (first_set >= n_sets) return;  // warp-uniform
+  const int s0 = (int)first_set, s1 = min(n_sets, s0 + shape.sets);
+  const int g0 = (int)(item % per_set) * shape.groups, g1 = min(n_groups, g0 + shape.groups);
+  const int ss2 = S.samples * S.samples;
+  BeamLists lists{kNoList, kNoList, 0};
+  if (kBeam && shape.beam)
+    lists = begin_beam<kGeo>(S, n_pix, rank_list, poses, c0, nc, cw_log2, s0, s1, g0, g1, beam, sh.code);
+  unsigned primary = 0, shadow = 0;
+  for (int set = s0; set < s1; ++set) {
+    const int rank = set * ppw + (lane >> cw_log2);
+    const int pixel = rank < n_pix ? __ldg(S.pixel_of_rank + (rank_list ? rank_list[rank] : rank)) : 0;
+    // the set's ppw pixels: their sub-rays' coordinates and FP64 cos^4 once per
+    // set (entry p * ss2 + j: sub-ray j of the pixel in lanes p * cw ...)
+    const int table = ppw * ss2;
+    const bool shared_subrays = kMode != kDepthOnly && table <= kSubrayTable;
+    if (shared_subrays) {
+      for (int q0 = 0; q0 < table; q0 += 32) {  // warp-uniform: every lane takes part in the shuffle
+        const int q = q0 + lane, p = min(q / ss2, ppw - 1);
+        const int pix = __shfl_sync(kFull, pixel, p << cw_log2);
+        if (q < table) {
+          const int j = q - p * ss2;
+          const float x = subray_x(S, pix % S.width, j % S.samples), y = subray_y(S, pix / S.width, j / S.samples);
+          sh.subrays[q] = SubraySample{cos4_of(x, y), x, y};
+        }
+      }
+      __syncwarp();
+    }
+    const SubraySample *mine = shared_subrays ? sh.subrays + (lane >> cw_log2) * ss2 : nullptr;
+    for (int g = g0; g < g1; ++g) {
+      const int cell = g * cw + (lane & (cw - 1));
+      const bool active = rank < n_pix && cell < nc;
+      const CellPose pose = poses[c0 + (active ? cell : 0)];
+      PixelSample s;
+      if (kBeam && lists.shadow < 0)
+        s = sample_without_beam<kMode, kGeo>(S, pixel, active, pose, sh, mine);
+      else
+        s = sample_pixel_group<kMode, kRays, kGeo, kBeam>(S, pixel, active, pose, sh.code, sh.t, mine, beam, lists);
+      if (active) {
+        const size_t o = (size_t)cell * n_pix + rank;
+        store_radiance(S, radiance, o, s.valid ? s.radiance : __longlong_as_double(0x7ff8000000000000ll));
+        if (depth_out) depth_out[o] = s.depth;
+      }
+      primary += s.primary;
+      shadow += s.shadow;
+    }
+    __syncwarp();  // the table is rewritten for the next set, the lists for the warp's next item
+  }
+  const unsigned prim = warp_sum(primary), shad = warp_sum(shadow);
   if (lane == 0 && counters) {
     atomicAdd(counters + kCntPrimary, (unsigned long long)prim);
     atomicAdd(counters + kCntShadow, (unsigned long long)shad);
   }
-  if (shared_subrays) __syncwarp();  // the table is rewritten by the warp's next item
 }
 
 // One pixel of a circuit launch (generate_pixels' circuit half,
