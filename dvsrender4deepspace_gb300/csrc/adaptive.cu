@@ -10,12 +10,10 @@
 // tracing of the cells inside them.  The circuit then integrates every
 // native cell from the interpolated (or exactly traced) radiance.
 //
-// GB300 mapping: the reference gives each pixel a warp whose lanes split the
-// sub-rays.  Here a lane owns a pixel and runs its own refinement stack; the
-// 32 Morton-adjacent pixels of a warp probe in lock-step, so every probe is
-// one coherent warp packet through the BVH (lanes with nothing to probe ride
-// along inactive).  The probe value is the pixel's serial sub-ray mean, the
-// same double the reference's warp_radiance returns.
+// GB300 mapping: a warp per pixel, as the reference, but with the pixel's
+// pending segments one per lane (refine_kernel).  The probe value is the
+// pixel's serial sub-ray mean, the same double the reference's warp_radiance
+// returns.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -28,10 +26,6 @@ namespace {
 
 constexpr int kRefineStack = 16;  // optical_sampler.cu:43
 
-struct RefineEntry {
-  double a, b, left, middle, right;
-};
-
 // native_pose (optical_sampler.cu:26-30): the interval holding t.
 __device__ __forceinline__ CellPose native_pose(const dvs_optical_interval *ivs, int count, double t) {
   int lo = 0, hi = count - 1;
@@ -40,17 +34,6 @@ __device__ __forceinline__ CellPose native_pose(const dvs_optical_interval *ivs,
     if (t > ivs[m].t1) lo = m + 1; else hi = m;
   }
   return pose_at(ivs[lo], t);
-}
-
-// One lock-step probe: lanes with `want` trace their pixel at their time.
-template <int kGeo>
-__device__ __forceinline__ double probe(const SceneView &S, int pixel, bool want, const dvs_optical_interval *ivs,
-                                        int n_ivs, double t, int *sc, float *stt, bool &bad, unsigned &rays) {
-  const CellPose pose = native_pose(ivs, n_ivs, want ? t : ivs[0].t0);
-  const PixelSample s = sample_pixel_packet<kRadiance, kGeo>(S, pixel, want, pose, sc, stt, nullptr);
-  if (want && (!s.valid || !isfinite(s.radiance))) bad = true;
-  rays += s.primary + s.shadow;
-  return s.radiance;
 }
 
 __device__ __forceinline__ double segment_fraction(const OpticalKnot *values, int a) { return fabs(values[a].fraction); }
@@ -62,103 +45,219 @@ __global__ void probe_poses_kernel(const dvs_optical_interval *ivs, int n_ivs, d
   if (j < 5) out[j] = native_pose(ivs, n_ivs, start + (end - start) * j * .25);
 }
 
-// refine_pixels (optical_sampler.cu:39-84), one pixel per lane.  The five
+// refine_pixels (optical_sampler.cu:39-84), one warp per pixel.  The five
 // initial probes come traced by the native trace kernel (initial[j * n +
 // rank]: every pixel is probed at the same five times, so they are five
 // circuit cells of a temporal warp packet); the bisection probes, which only
 // some pixels need, are traced here.
+//
+// The lanes hold the pixel's pending segments in time order: the reference's
+// depth-first stack, opened ahead.  A segment's verdict depends on the segment
+// and on how many wait behind it in that stack (`behind`, which a split hands
+// on: +1 to the left half), not on when it is reached, so every iteration
+// judges all pending segments at once (the FP64 receptor steps, one segment
+// per lane), emits the finished ones at the front in order, and splits up to
+// kAhead pending segments: two probes each, their poses one per lane, their
+// sub-rays 32 to a packet through the pixel's beam.  Knots, fallbacks and
+// counters are the depth-first walk's: an overflow of the knot capacity takes
+// back the count of the splits that walk would not have reached.
+//
+// Bound by the latency of the probes' packets and the FP64 pipe of the
+// verdicts.  One pixel per lane instead (32 pixels in lock-step, each lane
+// its sub-rays one after the other) took 312 ms for 120 x 90 pixels and
+// 200 horizons of 10 us at 16 sub-rays, every probe a packet of 32 times.
+constexpr int kAhead = 16;        // pending segments beyond which only the first is split: with its at most
+                                  // kRefineStack - 1 further left halves the list stays within 32 lanes
+constexpr int kProbeRays = 16;    // sub-rays of a probe traced and summed at a time
+struct RefineShared {
+  int code[kStackSlots];
+  float t[kStackSlots];
+  Beam beam;
+  CellPose pose[32];
+  double term[32][kProbeRays + 1];  // [probe][sub-ray], rows apart in the banks
+  double seg[5][32];
+  int behind[32], verdict[32];
+};
+enum : int { kUndecided = 0, kSmooth = 1, kExact = 2, kSplit = 3 };
+
 template <int kGeo>
-__global__ void __launch_bounds__(128) refine_kernel(SceneView S, int n, const dvs_optical_interval *ivs, int n_ivs,
-                                                     double start, double end, PhotoParams photo, double tolerance,
-                                                     CircuitState st, double charge, int capacity,
-                                                     const double *initial_radiance, OpticalKnot *knots,
-                                                     int32_t *counts, unsigned long long *ref_stats,
-                                                     int32_t *error, unsigned long long *counters) {
-  __shared__ int s_code[4][kStackSlots];
-  __shared__ float s_t[4][kStackSlots];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = blockIdx.x * blockDim.x + threadIdx.x;
-  if (__all_sync(kFull, rank >= n)) return;  // warp-uniform
-  const bool mine = rank < n;
-  const int pixel = mine ? S.pixel_of_rank[rank] : 0;
-  int *sc = s_code[wib];
-  float *stt = s_t[wib];
+__global__ void __launch_bounds__(128, 4)
+    refine_kernel(const __grid_constant__ SceneView S, int n, const dvs_optical_interval *ivs, int n_ivs, double start,
+                  double end, PhotoParams photo, double tolerance, CircuitState st, double charge, int capacity,
+                  const double *initial_radiance, OpticalKnot *knots, int32_t *counts, unsigned long long *ref_stats,
+                  int32_t *error, unsigned long long *counters) {
+  extern __shared__ __align__(16) unsigned char refine_shared[];
+  RefineShared &sh = reinterpret_cast<RefineShared *>(refine_shared)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int rank = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (rank >= n) return;  // warp-uniform
+  const int pixel = S.pixel_of_rank[rank];
+  const int px_i = pixel % S.width, py_i = pixel / S.width, ss2 = S.samples * S.samples;
   bool bad = false;
   unsigned rays = 0;
   double initial[5];
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
-    initial[j] = mine ? initial_radiance[(size_t)j * n + rank] : 0.0;
-    if (mine && !isfinite(initial[j])) bad = true;
+    initial[j] = initial_radiance[(size_t)j * n + rank];
+    if (!isfinite(initial[j])) bad = true;
   }
-  RefineEntry stack[kRefineStack];
-  int top = 0, written = 0;
-  bool fallback = false;
-  unsigned long long queries = 5;
-  OpticalKnot *out = knots + (size_t)(mine ? rank : 0) * capacity;
-  double v0 = 0, budget = 0;
-  if (mine) {
-    stack[0] = {.5, 1, initial[2], initial[3], initial[4]};
-    stack[1] = {0, .5, initial[0], initial[1], initial[2]};
-    top = 2;
-    out[0] = {0, initial[0]};
-    written = 1;
-    v0 = st.receptor_log[rank];
-    budget = 1e-3 * fmin(st.threshold_pos[rank], st.threshold_neg[rank]);  // kOpticalVoltageThresholdFraction
+  OpticalKnot *out = knots + (size_t)rank * capacity;
+  const double v0 = st.receptor_log[rank];
+  const double budget = 1e-3 * fmin(st.threshold_pos[rank], st.threshold_neg[rank]);  // kOpticalVoltageThresholdFraction
+  if (lane == 0) out[0] = {0, initial[0]};
+  // lane i: pending segment i
+  double a = 0, b = .5, left = initial[0], middle = initial[1], right = initial[2];
+  int behind = 1, verdict = kUndecided;
+  if (lane == 1) {
+    a = .5;
+    b = 1;
+    left = initial[2];
+    middle = initial[3];
+    right = initial[4];
+    behind = 0;
   }
-  int exact_segments = 0;
-  while (__any_sync(kFull, mine && top > 0 && !fallback)) {
-    const bool work = mine && top > 0 && !fallback;
-    bool need = false;
-    double ta = 0, tb = 0, mid = 0;
-    RefineEntry e{0, 0, 0, 0, 0};
-    if (work) {
-      e = stack[--top];
-      const double actual = e.middle * photo.electrons_per_radiance + photo.dark_electrons;
-      const double estimate = (e.left + e.right) * .5 * photo.electrons_per_radiance + photo.dark_electrons;
+  int pending = 2, written = 1, splits = 0, exact_segments = 0, not_reached = 0;
+  bool fallback = false, no_beam = true;
+  BeamLists lists{kNoList, kNoList, 0};
+  while (pending > 0) {
+    if (lane < pending && verdict == kUndecided) {
+      const double actual = middle * photo.electrons_per_radiance + photo.dark_electrons;
+      const double estimate = (left + right) * .5 * photo.electrons_per_radiance + photo.dark_electrons;
       const double residual = fabs(log(fmax(1e-30, actual) / fmax(1e-30, estimate)));
-      const double leaf_duration = (e.b - e.a) * (end - start);
+      const double leaf_duration = (b - a) * (end - start);
       const double voltage_error = fabs(receptor_log_at(v0, actual, leaf_duration, charge) -
                                         receptor_log_at(v0, estimate, leaf_duration, charge));
-      if (voltage_error <= budget && (residual <= tolerance || fmax(actual, estimate) * leaf_duration < 1.0)) {
-        if (written + 2 > capacity) {
-          fallback = true;
+      if (voltage_error <= budget && (residual <= tolerance || fmax(actual, estimate) * leaf_duration < 1.0))
+        verdict = kSmooth;
+      else if ((b - a) * (end - start) <= photo.integration_step || behind + 2 > kRefineStack)
+        verdict = kExact;  // unresolved at the electrical sampling scale: exact tracing
+      else
+        verdict = kSplit;
+    }
+    __syncwarp();
+    const unsigned to_split = __ballot_sync(kFull, lane < pending && verdict == kSplit);
+    const int done = to_split ? __ffs(to_split) - 1 : pending;  // finished segments at the front
+    if (done > 0) {
+      const unsigned two = __ballot_sync(kFull, lane < done && verdict == kSmooth);
+      const unsigned one = __ballot_sync(kFull, lane < done && verdict == kExact);
+      const int at = written + 2 * __popc(two & below) + __popc(one & below);
+      const bool over = lane < done && (verdict == kSmooth ? at + 2 > capacity : at >= capacity);
+      const unsigned overs = __ballot_sync(kFull, over);
+      const int emit = overs ? __ffs(overs) - 1 : done;
+      const unsigned emitted = emit >= 32 ? kFull : (1u << emit) - 1u;
+      if (lane < emit) {
+        if (verdict == kSmooth) {
+          out[at] = {(a + b) * .5, middle};
+          out[at + 1] = {b, right};
         } else {
-          out[written] = {(e.a + e.b) * .5, e.middle};
-          out[written + 1] = {e.b, e.right};
-          written += 2;
+          out[at] = {-b, right};
         }
-      } else if ((e.b - e.a) * (end - start) <= photo.integration_step || top + 2 > kRefineStack) {
-        // unresolved at the electrical sampling scale: exact tracing
-        if (written >= capacity) {
-          fallback = true;
-        } else {
-          out[written] = {-e.b, e.right};
-          ++written;
-          ++exact_segments;
-        }
-      } else {
-        need = true;
-        mid = (e.a + e.b) * .5;
-        ta = start + (end - start) * (e.a + mid) * .5;
-        tb = start + (end - start) * (mid + e.b) * .5;
+      }
+      written += 2 * __popc(two & emitted) + __popc(one & emitted);
+      exact_segments += __popc(one & emitted);
+      if (overs) {
+        fallback = true;
+        not_reached = pending - 1 - emit - __shfl_sync(kFull, behind, emit);
+        break;
+      }
+      pending -= done;
+      const int from = (lane + done) & 31;
+      a = __shfl_sync(kFull, a, from);
+      b = __shfl_sync(kFull, b, from);
+      left = __shfl_sync(kFull, left, from);
+      middle = __shfl_sync(kFull, middle, from);
+      right = __shfl_sync(kFull, right, from);
+      behind = __shfl_sync(kFull, behind, from);
+      verdict = __shfl_sync(kFull, verdict, from);
+    }
+    if (pending == 0) break;
+    // the first pending segment splits; others while the list stays within kAhead
+    const unsigned wants = to_split >> done;
+    const int count = max(1, min(__popc(wants), kAhead - pending));
+    const bool mine = ((wants >> lane) & 1u) && __popc(wants & below) < count;
+    const unsigned chosen = __ballot_sync(kFull, mine);
+    const int slot = __popc(chosen & below);
+    if (no_beam) {  // the first split: the pixel's beam over the window, from the corners at the initial probe times
+      no_beam = false;
+      const int last = S.samples - 1, j = min(lane >> 2, 4);
+      const CellPose pose = native_pose(ivs, n_ivs, start + (end - start) * j * .25);
+      const float3 o = f3(pose.px, pose.py, pose.pz), l = inverse_direction(f3(pose.lx, pose.ly, pose.lz));
+      const float3 d = unit(rotate_ray(pose, f3(subray_x(S, px_i, lane & 1 ? last : 0),
+                                                -subray_y(S, py_i, lane & 2 ? last : 0), -1)));
+      lists = close_beam<kGeo>(S, o, o, d, d, l, l, 0.05f, sh.beam, sh.code);
+    }
+    if (mine) {
+      sh.seg[0][slot] = a;
+      sh.seg[1][slot] = b;
+    }
+    __syncwarp();
+    const int probes = 2 * count;
+    if (lane < probes) {
+      const double pa = sh.seg[0][lane >> 1], pb = sh.seg[1][lane >> 1], mid = (pa + pb) * .5;
+      const double t = lane & 1 ? start + (end - start) * (mid + pb) * .5 : start + (end - start) * (pa + mid) * .5;
+      sh.pose[lane] = native_pose(ivs, n_ivs, t);
+    }
+    __syncwarp();
+    double sum = 0;
+    for (int r0 = 0; r0 < ss2; r0 += kProbeRays) {
+      const int m = min(kProbeRays, ss2 - r0), total = probes * m;
+      for (int q0 = 0; q0 < total; q0 += 32) {
+        const int q = min(q0 + lane, total - 1), k = q / m, r = r0 + q - k * m;
+        const bool live = q0 + lane < total;
+        const CellPose pose = sh.pose[k];
+        const RaySample s = sample_ray<kRadiance, kGeo, true>(S, subray_x(S, px_i, r % S.samples),
+                                                              subray_y(S, py_i, r / S.samples), pose, live, sh.code,
+                                                              sh.t, sh.beam, lists);
+        if (live) sh.term[k][q - k * m] = s.term;
+        if (s.overflow) bad = true;
+        rays += (live ? 1u : 0u) + (s.lit ? 1u : 0u);
+      }
+      __syncwarp();
+      if (lane < probes)
+        for (int i = 0; i < m; ++i) sum += sh.term[lane][i];  // in sub-ray order, as the pixel sample's sum
+      __syncwarp();
+    }
+    sum /= ss2;
+    if (lane < probes && !isfinite(sum)) bad = true;
+    // the list with each chosen segment replaced by its halves
+    const double left_mid = __shfl_sync(kFull, sum, (2 * slot) & 31), right_mid = __shfl_sync(kFull, sum, (2 * slot + 1) & 31);
+    const int to = lane + slot;
+    if (lane < pending) {
+      const double mid = (a + b) * .5;
+      sh.seg[0][to] = a;
+      sh.seg[1][to] = mine ? mid : b;
+      sh.seg[2][to] = left;
+      sh.seg[3][to] = mine ? left_mid : middle;
+      sh.seg[4][to] = mine ? middle : right;
+      sh.behind[to] = mine ? behind + 1 : behind;
+      sh.verdict[to] = mine ? kUndecided : verdict;
+      if (mine) {
+        sh.seg[0][to + 1] = mid;
+        sh.seg[1][to + 1] = b;
+        sh.seg[2][to + 1] = middle;
+        sh.seg[3][to + 1] = right_mid;
+        sh.seg[4][to + 1] = right;
+        sh.behind[to + 1] = behind;
+        sh.verdict[to + 1] = kUndecided;
       }
     }
-    if (__any_sync(kFull, need)) {
-      const double left_mid = probe<kGeo>(S, pixel, need, ivs, n_ivs, ta, sc, stt, bad, rays);
-      const double right_mid = probe<kGeo>(S, pixel, need, ivs, n_ivs, tb, sc, stt, bad, rays);
-      if (need) {
-        queries += 2;
-        stack[top] = {mid, e.b, e.middle, right_mid, e.right};
-        stack[top + 1] = {e.a, mid, e.left, left_mid, e.middle};
-        top += 2;
-      }
-    }
+    __syncwarp();
+    pending += count;
+    splits += count;
+    a = sh.seg[0][lane];
+    b = sh.seg[1][lane];
+    left = sh.seg[2][lane];
+    middle = sh.seg[3][lane];
+    right = sh.seg[4][lane];
+    behind = sh.behind[lane];
+    verdict = sh.verdict[lane];
+    __syncwarp();
   }
   if (bad) atomicOr(error, kErrOptical);
-  if (mine) {
+  if (lane == 0) {
     counts[rank] = fallback ? -1 : written;
-    atomicAdd(ref_stats + kRefTraced, queries);
+    atomicAdd(ref_stats + kRefTraced, 5ull + 2ull * (unsigned)(splits - not_reached));
     if (fallback) atomicAdd(ref_stats + kRefFallback, 1ull);
     else atomicMax(ref_stats + kRefMaxKnots, (unsigned long long)written);
     if (exact_segments) atomicAdd(ref_stats + kRefExactSegments, (unsigned long long)exact_segments);
@@ -345,10 +444,15 @@ cudaError_t launch_refine(const SceneView &scene, int n, const dvs_optical_inter
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_trace_cells(scene, n, probe_poses, 0, 5, 3, probe_radiance, nullptr, counters, s);
   if (e != cudaSuccess) return e;
-#define DVS_REFINE(G)                                                                                         \
-  refine_kernel<G><<<blocks_of(n, 128), 128, 0, s>>>(scene, n, ivs, n_ivs, start, end, photo, tolerance, st, charge, \
-                                                     capacity, probe_radiance, knots, counts, ref_stats, error,     \
-                                                     counters)
+#define DVS_REFINE(G)                                                                                              \
+  do {                                                                                                             \
+    e = cudaFuncSetAttribute(refine_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);          \
+    if (e != cudaSuccess) return e;                                                                                \
+    refine_kernel<G><<<blocks_of(n, 4), 128, shared, s>>>(scene, n, ivs, n_ivs, start, end, photo, tolerance, st,  \
+                                                          charge, capacity, probe_radiance, knots, counts,         \
+                                                          ref_stats, error, counters);                             \
+  } while (0)
+  const size_t shared = 4 * sizeof(RefineShared);
   switch (scene.geometry) {
     case kGeoHalfBounds: DVS_REFINE(kGeoHalfBounds); break;
     case kGeoWatertight: DVS_REFINE(kGeoWatertight); break;

@@ -1349,6 +1349,46 @@ __device__ __forceinline__ void packet_range(const float3 (&v)[R], const bool (&
   hi = whigh3(hi);
 }
 
+// A wider bundle of directions (the sum of its extents per axis) takes no beam.
+constexpr float kBeamSpread = 0.1f;
+// A beam and its lists from each lane's ranges of origins, directions and
+// inverse light directions; reach: what the rays' origins and light directions may leave the
+// ranges by, as a share of their extent.
+template <int kGeo>
+__device__ __forceinline__ BeamLists close_beam(const SceneView &S, float3 olo, float3 ohi, float3 dlo, float3 dhi,
+                                                float3 llo, float3 lhi, float reach, Beam &B, int *stack) {
+  olo = wlow3(olo);
+  ohi = whigh3(ohi);
+  dlo = wlow3(dlo);
+  dhi = whigh3(dhi);
+  llo = wlow3(llo);
+  lhi = whigh3(lhi);
+  const float ext = (dhi.x - dlo.x) + (dhi.y - dlo.y) + (dhi.z - dlo.z);
+  BeamLists lists{kNoList, kNoList, 0};
+  if (!(ext <= kBeamSpread)) return lists;  // a wide bundle reaches too many leaves (or a ray has no direction)
+  const float m = ext * ext + 4e-7f;
+  if (reach > 0.0f) {
+    const float3 a = max3(-olo, ohi), o = reach * (ohi - olo) + 5e-7f * max3(a, -a);
+    const float3 b = max3(-llo, lhi), l = reach * (lhi - llo) + 5e-7f * max3(b, -b);
+    olo = olo - o;
+    ohi = ohi + o;
+    llo = llo - l;
+    lhi = lhi + l;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    B.olo = olo;
+    B.ohi = ohi;
+    B.dlo = dlo - f3(m, m, m);
+    B.dhi = dhi + f3(m, m, m);
+    B.llo = llo;
+    B.lhi = lhi;
+  }
+  __syncwarp();
+  lists.leaves = build_primary_list<kGeo>(S, B, stack);
+  if (lists.leaves >= 0) lists.shadow = build_shadow_list<kGeo>(S, B, lists.leaves, stack);
+  return lists;
+}
+
 // The general walks, out of line: they serve the packets no list holds for.
 template <int R>
 struct PacketRays {
@@ -1643,6 +1683,73 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
   }
   out.radiance /= ss * ss;
   out.depth = valid_depth ? float(depth / valid_depth) : -1.0f;
+  return out;
+}
+
+// One sub-ray per lane, each lane with its own pose and image-plane
+// coordinates: the body of sample_pixel_group's loop for packets whose lanes
+// are sub-rays, poses or pixels.  term: the ray's addend of the pixel's
+// FP64 radiance sum (0 when unlit).  kChecked: the beam's origin and light
+// ranges were formed from other poses than these, so each ray's are checked too.
+struct RaySample {
+  double term;
+  float t;  // hit distance
+  bool hit, lit, overflow;
+};
+template <int kMode, int kGeo, bool kChecked>
+__device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, float py, const CellPose &pose, bool live,
+                                                int *stack_code, float *stack_t, Beam &B, BeamLists &lists) {
+  RaySample out{0.0, 0.0f, false, false, false};
+  const float3 light = f3(pose.lx, pose.ly, pose.lz);
+  const float3 origin = f3(pose.px, pose.py, pose.pz);
+  const float3 ray[1] = {unit(rotate_ray(pose, f3(px, -py, -1)))};
+  const bool lives[1] = {live};
+  const ShadowDir sdir = shadow_dir<kGeo>(light);
+  HitRecord hit[1];
+  bool inside = within(ray[0], B.dlo, B.dhi);
+  if (kChecked) inside = inside && within(origin, B.olo, B.ohi) && within(sdir.idir, B.llo, B.lhi);
+  const bool listed = lists.shadow >= 0 && __all_sync(kFull, inside || !live);
+  if (listed) {
+    nearest_in_list<1, kGeo>(S, B, lists.leaves, origin, ray, lives, hit);
+  } else {
+    const PacketHits<1> got = nearest_general<1, kGeo>(S, PacketRays<1>{{origin}, {ray[0]}, {live}}, stack_code, stack_t);
+    hit[0] = got.h[0];
+  }
+  out.overflow = live && hit[0].hit < 0;
+  out.hit = live && hit[0].hit == 1;
+  out.t = hit[0].t;
+  if (kMode == kDepthOnly) return out;
+  float3 normal = f3(0, 0, 0), sorigin[1] = {f3(0, 0, 0)};
+  float albedo = S.hapke.w, r0 = S.hc.r0_w;
+  if (out.hit) {
+    const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[0].tri);
+    const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
+    const float w = 1 - hit[0].u - hit[0].v;
+    normal = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[0].u + f3(s2.x, s2.y, s2.z) * hit[0].v);
+    out.lit = !(dot(normal, light) <= 0 || dot(normal, -ray[0]) <= 0);
+    if (out.lit) {
+      const float4 *r = tri_record<kGeo>(S, hit[0].tri, 2);
+      const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
+      sorigin[0] = shadow_origin_rec<kGeo>(a, b, c, hit[0].u, hit[0].v, light);
+      if (S.has_albedo) {
+        albedo = s0.w * w + s1.w * hit[0].u + s2.w * hit[0].v;
+        r0 = hfunc_r0(albedo);
+      }
+    }
+  }
+  if (!__any_sync(kFull, out.lit)) return out;
+  const bool lit[1] = {out.lit};
+  const int self[1] = {hit[0].tri};
+  unsigned occluded;
+  if (listed && __all_sync(kFull, !out.lit || within(sorigin[0], B.slo, B.shi)))
+    occluded = shadow_in_list<1, kGeo>(S, B, lists.shadow, sorigin, light, sdir, lit, self, lists.first);
+  else
+    occluded = shadow_general<1, kGeo>(S, ShadowRays<1>{{sorigin[0]}, light, {self[0]}, {out.lit}}, stack_code, stack_t);
+  if (out.lit && !occluded) {
+    const float3 n = unit(normal), l = unit(light), v = unit(-ray[0]);
+    const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo, r0, S.hapke, S.hc);
+    out.term = fmaxf(0, n_h * pose.intensity) * cos4_of(px, py);
+  }
   return out;
 }
 

@@ -17,8 +17,6 @@ constexpr int kWarpsPerBlock = 4;  // all ray kernels launch 128 threads
 #endif
 constexpr int kSubrayTable = 256;  // sub-rays per pixel with a shared sub-ray table (ss <= 16)
 
-// A wider bundle of directions (the sum of its extents per axis) takes no beam.
-constexpr float kBeamSpread = 0.1f;
 // A warp's shared memory in the trace kernels: the traversal stack and the
 // sub-ray table (and, in kernels with beams, a Beam beside it).
 struct TraceShared {
@@ -80,28 +78,7 @@ __device__ __forceinline__ BeamLists begin_beam(const SceneView &S, int n_pix, c
       }
     }
   }
-  olo = wlow3(olo);
-  ohi = whigh3(ohi);
-  dlo = wlow3(dlo);
-  dhi = whigh3(dhi);
-  llo = wlow3(llo);
-  lhi = whigh3(lhi);
-  const float ext = (dhi.x - dlo.x) + (dhi.y - dlo.y) + (dhi.z - dlo.z);
-  BeamLists lists{kNoList, kNoList, 0};
-  if (!(ext <= kBeamSpread)) return lists;  // a wide bundle reaches too many leaves (or a ray has no direction)
-  const float m = ext * ext + 4e-7f;
-  if (lane == 0) {
-    B.olo = olo;
-    B.ohi = ohi;
-    B.dlo = dlo - f3(m, m, m);
-    B.dhi = dhi + f3(m, m, m);
-    B.llo = llo;
-    B.lhi = lhi;
-  }
-  __syncwarp();
-  lists.leaves = build_primary_list<kGeo>(S, B, stack);
-  if (lists.leaves >= 0) lists.shadow = build_shadow_list<kGeo>(S, B, lists.leaves, stack);
-  return lists;
+  return close_beam<kGeo>(S, olo, ohi, dlo, dhi, llo, lhi, 0.0f, B, stack);
 }
 
 // The packets of an item without lists, out of line (few items of a launch with beams): two sub-rays per lane where
