@@ -343,31 +343,38 @@ __global__ void __launch_bounds__(128) integrate_knots_kernel(int n, const Cell 
   const int n_exact = exact_counts ? exact_counts[rank] : 0;
   const int32_t *my_exact = exact_cells + (size_t)rank * capacity;
   const double *my_exact_rad = exact_radiance + (size_t)rank * capacity;
-  PixelRegs s{st.receptor_log[rank], st.reference_log[rank], st.refractory_until[rank], st.threshold_pos[rank],
-              st.threshold_neg[rank], st.reset_pending[rank] != 0};
+  CircuitRun run = circuit_begin(st, rank, p);
   curandStateXORWOW_t rng = st.rng[rank];
   double *my_t = slab_t + (size_t)rank * max_events;
   int8_t *my_p = slab_p + (size_t)rank * max_events;
   int a = 0, exact_index = 0, count = 0, failed = 0;
+  // the segment [a, a + 1] of the knots: its left end and light, and the light's slope over the window fraction
+  double left = segment_fraction(values, 0), right = segment_fraction(values, 1);
+  double from = values[0].radiance, slope = (values[1].radiance - from) / (right - left);
+  const double inv_window = 1.0 / (end - start);
   for (int c = 0; c < n_cells; ++c) {
-    const double t0 = cells[c].t0, t1 = cells[c].t1;
-    const double fraction = ((t0 + t1) * .5 - start) / (end - start);
-    while (a + 2 < size && fraction > segment_fraction(values, a + 1)) ++a;
-    const double weight =
-        (fraction - segment_fraction(values, a)) / (segment_fraction(values, a + 1) - segment_fraction(values, a));
-    double light = values[a].radiance + (values[a + 1].radiance - values[a].radiance) * weight;
+    const Cell cell = cells[c];
+    const double t0 = cell.t0, t1 = cell.t1;
+    const double fraction = ((t0 + t1) * .5 - start) * inv_window;
+    if (a + 2 < size && fraction > right) {
+      do {
+        ++a;
+        right = segment_fraction(values, a + 1);
+      } while (a + 2 < size && fraction > right);
+      left = segment_fraction(values, a);
+      from = values[a].radiance;
+      slope = (values[a + 1].radiance - from) / (right - left);
+    }
+    double light = from + slope * (fraction - left);
     if (exact_index < n_exact && my_exact[exact_index] == c) light = my_exact_rad[exact_index++];
     double rate = fmax(0.0, light) * photo.electrons_per_radiance + photo.dark_electrons;
-    if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) / (t1 - t0);
-    const int emitted = advance_pixel(s, p, rate, t0, t1, my_t + count, my_p + count, max_events - count, rng);
+    if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
+    const int emitted = circuit_cell(run, p, rate, t0, t1, my_t + count, my_p + count, max_events - count, rng);
     if (emitted == -1) { failed = kErrCapacity; break; }
     if (emitted == -2) { failed = kErrStalled; break; }
     count += emitted;
   }
-  st.receptor_log[rank] = s.receptor_log;
-  st.reference_log[rank] = s.reference_log;
-  st.refractory_until[rank] = s.refractory_until;
-  st.reset_pending[rank] = s.reset_pending ? 1 : 0;
+  circuit_end(run, st, rank);
   st.rng[rank] = rng;
   if (failed) {
     atomicOr(error, failed);

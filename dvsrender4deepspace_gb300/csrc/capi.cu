@@ -861,6 +861,7 @@ int dvs_sensor_create(dvs_scene *scene, const dvs_physic *physic, const dvs_sens
   ALLOC(s->st.refractory_until, sizeof(double) * n, "pixel states");
   ALLOC(s->st.threshold_pos, sizeof(double) * n, "pixel states");
   ALLOC(s->st.threshold_neg, sizeof(double) * n, "pixel states");
+  ALLOC(s->st.receptor, sizeof(double) * n, "pixel states");
   ALLOC(s->st.reset_pending, sizeof(int8_t) * n, "pixel states");
   ALLOC(s->st.rng, sizeof(curandStateXORWOW_t) * n, "pixel RNG");
   s->st.pixel = s->order;
@@ -901,6 +902,7 @@ int dvs_sensor_destroy(dvs_sensor *s) {
   cudaFree(s->st.refractory_until);
   cudaFree(s->st.threshold_pos);
   cudaFree(s->st.threshold_neg);
+  cudaFree(s->st.receptor);
   cudaFree(s->st.reset_pending);
   cudaFree(s->st.rng);
   cudaFree(s->ev_count);
@@ -1038,6 +1040,7 @@ static int stage_batch(dvs_sensor *s, const dvs_optical_interval *ivs, size_t co
       cell.t1 = step + 1 == steps ? iv.t1 : iv.t0 + (step + 1) * dt;
       cell.interval = (int32_t)i;
       cell.dt = (float)(cell.t1 - cell.t0);
+      cell.inv_len = 1.0 / (cell.t1 - cell.t0);
     }
   }
   std::memcpy(s->h_ivs, ivs, sizeof(dvs_optical_interval) * count);
@@ -1537,7 +1540,7 @@ int dvs_sensor_drain(dvs_sensor *s, dvs_event *out, size_t capacity, size_t *n_o
 int dvs_sensor_device_bytes(const dvs_sensor *s, uint64_t *bytes) {
   if (!s || !bytes) return fail(DVS_ERR_INVALID, "null argument");
   const uint64_t n = (uint64_t)s->pixels(), ev = (uint64_t)s->max_events;
-  uint64_t b = n * (5 * sizeof(double) + sizeof(int8_t) + sizeof(curandStateXORWOW_t) + sizeof(int32_t));
+  uint64_t b = n * (6 * sizeof(double) + sizeof(int8_t) + sizeof(curandStateXORWOW_t) + sizeof(int32_t));
   b += n * ev * (sizeof(double) + sizeof(int8_t) + sizeof(DevEvent));
   b += s->radiance_cap * sizeof(double) + s->ivs_cap * sizeof(dvs_optical_interval) + s->cells_cap * sizeof(Cell) +
        s->poses_cap * sizeof(CellPose);
@@ -1599,19 +1602,19 @@ static int autotune_chunk(dvs_sensor *s, size_t n_cells, dvs_tuning *out) {
   out->chunk_cells = ncs;
   out->chunk_best_ms = out->chunk_default_ms = -1;
   if (cands.size() < 2) return DVS_OK;
-  // shadow state: the five FP64 fields, the reset flags and (when drawn) the XORWOW states
+  // shadow state: the six FP64 fields, the reset flags and (when drawn) the XORWOW states
   const bool rng = !s->photo.philox && (s->photo.shot_noise || s->p.reset_noise_std > 0);
   const size_t fbytes = sizeof(double) * (size_t)n, rbytes = rng ? sizeof(curandStateXORWOW_t) * (size_t)n : 0;
   char *shadow = nullptr;
-  CUDA_TRY(cudaMalloc(&shadow, 5 * fbytes + (size_t)n + rbytes), "autotune shadow state");
+  CUDA_TRY(cudaMalloc(&shadow, 6 * fbytes + rbytes + (size_t)n), "autotune shadow state");
   CircuitState st = s->st;
-  double **fields[5] = {&st.receptor_log, &st.reference_log, &st.refractory_until, &st.threshold_pos,
-                        &st.threshold_neg};
-  double *src[5] = {s->st.receptor_log, s->st.reference_log, s->st.refractory_until, s->st.threshold_pos,
-                    s->st.threshold_neg};
-  for (int f = 0; f < 5; ++f) *fields[f] = reinterpret_cast<double *>(shadow + f * fbytes);
-  st.reset_pending = reinterpret_cast<int8_t *>(shadow + 5 * fbytes);
-  if (rng) st.rng = reinterpret_cast<curandStateXORWOW_t *>(shadow + 5 * fbytes + (size_t)n);
+  double **fields[6] = {&st.receptor_log, &st.reference_log, &st.refractory_until, &st.threshold_pos,
+                        &st.threshold_neg, &st.receptor};
+  double *src[6] = {s->st.receptor_log, s->st.reference_log, s->st.refractory_until, s->st.threshold_pos,
+                    s->st.threshold_neg, s->st.receptor};
+  for (int f = 0; f < 6; ++f) *fields[f] = reinterpret_cast<double *>(shadow + f * fbytes);
+  if (rng) st.rng = reinterpret_cast<curandStateXORWOW_t *>(shadow + 6 * fbytes);
+  st.reset_pending = reinterpret_cast<int8_t *>(shadow + 6 * fbytes + rbytes);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t err = cudaEventCreate(&e0);
   if (err == cudaSuccess) err = cudaEventCreate(&e1);
@@ -1621,7 +1624,7 @@ static int autotune_chunk(dvs_sensor *s, size_t n_cells, dvs_tuning *out) {
   int best_c = (int)def_chunk;
   for (int c : cands) {
     if (err != cudaSuccess) break;
-    for (int f = 0; f < 5 && err == cudaSuccess; ++f)
+    for (int f = 0; f < 6 && err == cudaSuccess; ++f)
       err = cudaMemcpyAsync(*fields[f], src[f], fbytes, cudaMemcpyDeviceToDevice, s->stream);
     if (err == cudaSuccess)
       err = cudaMemcpyAsync(st.reset_pending, s->st.reset_pending, (size_t)n, cudaMemcpyDeviceToDevice, s->stream);

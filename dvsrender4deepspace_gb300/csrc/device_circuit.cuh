@@ -104,6 +104,136 @@ __device__ int advance_pixel(PixelRegs &s, const PixelParams &p, double rate, do
   return count;
 }
 
+// ---- the FP64 circuit over a run of cells ----------------------------------------------
+// Nearly every cell of nearly every pixel sees no event, and GB300's FP64 pipe
+// is narrow, so what such a cell costs in FP64 instructions is the kernel's
+// time.  advance_pixel's own path takes exp(u), exp(-k), expm1(-k), log and
+// four divisions for u' = -log(e^-k / e^u + (1 - e^-k) / rate), k = rate dt / charge.
+// Carrying the receptor itself, x = e^u, the same step is
+//   x' = x rate / (e^-k rate + (1 - e^-k) x)
+// -- one exponential and one division -- and the comparator's u' - ref < theta is
+// x' < e^(ref + theta), with bounds that change only with the reference.  The
+// receptor's log is formed where an event, a reset or the end of the run needs
+// it; such a cell goes through advance_pixel unchanged.  A refractory cell
+// only moves x: its reference follows the receptor and is written down after.
+//
+// In real arithmetic the two steps are the same.  In FP64 this one rounds less:
+// u near 10 has a last bit of 2e-15, so one log and exp a cell move x by
+// that relative amount, the step above by a few 1e-16.  x is kept between runs
+// (CircuitState::receptor), so how cells are batched changes no bit.  A
+// leaking reference moves the bounds in every cell and takes advance_pixel.
+
+// 1 - e^-k for 0 <= k < 0.35 by the Taylor series of (1 - e^-k) / k, whose first term left out is k^14 / 15! < 3e-19.
+__device__ __forceinline__ double one_minus_exp_small(double k) {
+  double s = 1.0 / 87178291200.0;  // 1 / 14!
+  s = fma(-k, s, 1.0 / 6227020800.0);
+  s = fma(-k, s, 1.0 / 479001600.0);
+  s = fma(-k, s, 1.0 / 39916800.0);
+  s = fma(-k, s, 1.0 / 3628800.0);
+  s = fma(-k, s, 1.0 / 362880.0);
+  s = fma(-k, s, 1.0 / 40320.0);
+  s = fma(-k, s, 1.0 / 5040.0);
+  s = fma(-k, s, 1.0 / 720.0);
+  s = fma(-k, s, 1.0 / 120.0);
+  s = fma(-k, s, 1.0 / 24.0);
+  s = fma(-k, s, 1.0 / 6.0);
+  s = fma(-k, s, 0.5);
+  s = fma(-k, s, 1.0);
+  return k * s;
+}
+// The receptor after dt at a constant rate.
+__device__ __forceinline__ double receptor_step(double x, double rate, double dt, double inv_charge) {
+  const double g = dt * inv_charge, k = rate * g;
+  if (!(k > 0)) return x / fma(x, g, 1.0);  // no photons: the receptor discharges
+  double a, b;
+  if (k < 0.35) {
+    b = one_minus_exp_small(k);
+    a = 1.0 - b;
+  } else {
+    a = exp(-k);
+    b = 1.0 - a;
+  }
+  return x * rate / fma(b, x, a * rate);
+}
+
+struct CircuitRun {
+  PixelRegs s;
+  double x, high, low;  // receptor and the comparator's bounds on it
+  double inv_charge;
+  bool direct;    // a leaking reference: advance_pixel for every cell
+  bool follows;   // the reference is the receptor's log, not yet written down
+};
+__device__ __forceinline__ void circuit_bounds(CircuitRun &c) {
+  c.high = exp(c.s.reference_log + c.s.threshold_pos);
+  c.low = exp(c.s.reference_log - c.s.threshold_neg);
+}
+__device__ __forceinline__ CircuitRun circuit_begin(const CircuitState &st, int k, const PixelParams &p) {
+  CircuitRun c;
+  c.s = PixelRegs{st.receptor_log[k], st.reference_log[k], st.refractory_until[k], st.threshold_pos[k],
+                  st.threshold_neg[k], st.reset_pending[k] != 0};
+  c.direct = p.reference_leak > 0;
+  c.follows = false;
+  c.inv_charge = 1.0 / p.charge_scale;
+  if (!c.direct) {
+    c.x = st.receptor[k];
+    if (!(log(c.x) == c.s.receptor_log)) c.x = exp(c.s.receptor_log);  // written by another circuit
+    circuit_bounds(c);
+  }
+  return c;
+}
+// advance_pixel for one cell of a run.  By value both ways: a reference would
+// hold the run and the generator in local memory for the cells that need no call.
+struct EventCell {
+  CircuitRun c;
+  curandStateXORWOW_t rng;
+  int emitted;
+};
+__device__ __noinline__ EventCell circuit_event_cell(EventCell e, PixelParams p, double rate, double t0, double t1,
+                                                     double *out_t, int8_t *out_p, int capacity) {
+  CircuitRun &c = e.c;
+  if (!c.direct) {
+    c.s.receptor_log = log(c.x);
+    if (c.follows) c.s.reference_log = c.s.receptor_log;
+    c.follows = false;
+  }
+  e.emitted = advance_pixel(c.s, p, rate, t0, t1, out_t, out_p, capacity, e.rng);
+  if (!c.direct) {
+    c.x = exp(c.s.receptor_log);
+    circuit_bounds(c);
+  }
+  return e;
+}
+__device__ __forceinline__ int circuit_cell(CircuitRun &c, const PixelParams &p, double rate, double t0, double t1,
+                                            double *out_t, int8_t *out_p, int capacity, curandStateXORWOW_t &rng) {
+  if (!c.direct && t0 < t1) {
+    const bool refractory = t1 < c.s.refractory_until;
+    const bool settled = t0 >= c.s.refractory_until && !c.s.reset_pending && c.x < c.high && c.x > c.low;
+    if (refractory || settled) {
+      const double y = receptor_step(c.x, rate, t1 - t0, c.inv_charge);
+      if (refractory || (y < c.high && y > c.low)) {
+        c.x = y;
+        c.follows = refractory;
+        return 0;
+      }
+    }
+  }
+  const EventCell e = circuit_event_cell(EventCell{c, rng, 0}, p, rate, t0, t1, out_t, out_p, capacity);
+  c = e.c;
+  rng = e.rng;
+  return e.emitted;
+}
+__device__ __forceinline__ void circuit_end(CircuitRun &c, const CircuitState &st, int k) {
+  if (!c.direct) {
+    c.s.receptor_log = log(c.x);
+    if (c.follows) c.s.reference_log = c.s.receptor_log;
+    st.receptor[k] = c.x;
+  }
+  st.receptor_log[k] = c.s.receptor_log;
+  st.reference_log[k] = c.s.reference_log;
+  st.refractory_until[k] = c.s.refractory_until;
+  st.reset_pending[k] = c.s.reset_pending ? 1 : 0;
+}
+
 // ---- FP32 circuit (precision mode) ------------------------------------------------
 // The same pixel model with the receptor and contrast arithmetic in FP32 and
 // everything that fixes when an event happens in FP64: absolute times,

@@ -129,6 +129,7 @@ __global__ void init_pixels_kernel(int n, const int32_t *pixel_of_rank, const do
   }
   const double u = log(fmax(1e-30, rad * photo.electrons_per_radiance + photo.dark_electrons));
   st.receptor_log[k] = u;
+  st.receptor[k] = exp(u);
   st.reference_log[k] = u;
   st.refractory_until[k] = -1;
   st.threshold_pos[k] = fmax(minimum, p.threshold_pos + stddev * curand_normal_double(&rng));

@@ -43,8 +43,9 @@ struct alignas(16) CellPose {
 };
 
 // One circuit integration cell (event_sensor.cu:37-40): [t0, t1) of interval.
-struct alignas(8) Cell {
+struct alignas(16) Cell {
   double t0, t1;
+  double inv_len;  // 1 / (t1 - t0), formed once on the host: a photon count's rate without a division per pixel
   int32_t interval;
   float dt;  // (float)(t1 - t0), rounded once on the host: the FP32 circuit's cell length
 };
@@ -64,6 +65,7 @@ struct PhotoParams {
 // Pixel-circuit state, structure of arrays indexed by Morton rank.
 struct CircuitState {
   double *receptor_log, *reference_log, *refractory_until, *threshold_pos, *threshold_neg;
+  double *receptor;  // exp(receptor_log) as the FP64 circuit carries it; valid where its log is receptor_log
   int8_t *reset_pending;
   curandStateXORWOW_t *rng;
   const int32_t *pixel;  // rank -> row-major pixel of the full image (the noise streams' key)

@@ -184,24 +184,20 @@ __device__ __forceinline__ void circuit_rank(int r, int n, const int32_t *rank_l
   int8_t *my_p = slab_p + (size_t)k * max_events;
   int failed = 0;
   if (!kF32) {
-    PixelRegs s{st.receptor_log[k], st.reference_log[k], st.refractory_until[k], st.threshold_pos[k],
-                st.threshold_neg[k], st.reset_pending[k] != 0};
+    CircuitRun run = circuit_begin(st, k, p);
     for (int c = 0; c < nc; ++c) {
       const Cell cell = cells[c0 + c];
       const double rad = radiance[(size_t)c * n + r];
       if (!isfinite(rad)) { failed = kErrOptical; break; }
       double rate = rad * photo.electrons_per_radiance + photo.dark_electrons;
       const double t0 = cell.t0, t1 = cell.t1;
-      if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) / (t1 - t0);
-      const int emitted = advance_pixel(s, p, rate, t0, t1, my_t + cnt, my_p + cnt, max_events - cnt, rng);
+      if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
+      const int emitted = circuit_cell(run, p, rate, t0, t1, my_t + cnt, my_p + cnt, max_events - cnt, rng);
       if (emitted == -1) { failed = kErrCapacity; break; }
       if (emitted == -2) { failed = kErrStalled; break; }
       cnt += emitted;
     }
-    st.receptor_log[k] = s.receptor_log;
-    st.reference_log[k] = s.reference_log;
-    st.refractory_until[k] = s.refractory_until;
-    st.reset_pending[k] = s.reset_pending ? 1 : 0;
+    circuit_end(run, st, k);
   } else {
     // precision mode: the state is held in FP32 registers for the chunk
     PixelRegsF s{(float)st.receptor_log[k], (float)st.reference_log[k], st.refractory_until[k],
