@@ -128,10 +128,16 @@ struct DeviceReadout {
   ReadoutSort sort{};
   ReadoutFifo fifo{};
   size_t max_batch = 0;
-  int grid = 1;  // sort/scan blocks, sized from the previous batch
+  // Sort/scan blocks, one per 4096 events of the previous batch.  Before the
+  // first: unknown_grid, one per 4096 events at an event every 16 pixels, since one
+  // block alone sorts a first burst of 30,000 events in 2.5 ms and 22 blocks in 0.3.
+  int grid = 0, unknown_grid = 1;
   void *arena = nullptr;
-  int32_t *h_status = nullptr;  // [out_count, status]
-  unsigned long long *h_counters = nullptr;  // [dropped, peak]
+  struct HostStatus {
+    unsigned long long dropped, peak;
+    int32_t out_count, status;
+  };
+  HostStatus *host = nullptr;
 
   cudaError_t create(double bandwidth, double latency, size_t capacity, size_t batch, cudaStream_t st) {
     max_batch = std::max<size_t>(batch, 1);
@@ -149,9 +155,11 @@ struct DeviceReadout {
                  o_hist = take(4 * 256 * (size_t)max_grid), o_dtot = take(4 * 256), o_vary = take(8 * 3),
                  o_ring = take(sizeof(DevEvent) * ring), o_bmax = take(8 * (size_t)max_grid),
                  o_comp = take(8 * max_batch), o_del = take(8 * max_batch),
-                 o_out = take(sizeof(DevEvent) * (ring + max_batch)), o_u64 = take(8 * 5), o_avail = take(8),
-                 o_i32 = take(4 * 3), o_plan = take(8 * 3);
-    cudaError_t e = cudaMalloc(&arena, off);
+                 o_out = take(sizeof(DevEvent) * (ring + max_batch)), o_u64 = take(8 * 6), o_avail = take(8),
+                 o_i32 = take(4), o_plan = take(8 * 3);
+    unknown_grid = blocks_for(batch / 16);
+    cudaError_t e = prepare_readout();
+    if (e == cudaSuccess) e = cudaMalloc(&arena, off);
     if (e != cudaSuccess) return e;
     bytes = off;
     char *b = static_cast<char *>(arena);
@@ -164,16 +172,16 @@ struct DeviceReadout {
     sort.hist = reinterpret_cast<unsigned *>(b + o_hist);
     sort.digit_total = reinterpret_cast<unsigned *>(b + o_dtot);
     sort.varying = reinterpret_cast<unsigned long long *>(b + o_vary);
-    int32_t *i32 = reinterpret_cast<int32_t *>(b + o_i32);
-    fifo.overflow = i32;
-    fifo.status = i32 + 1;
-    fifo.out_count = i32 + 2;
+    fifo.overflow = reinterpret_cast<int32_t *>(b + o_i32);
     unsigned long long *u64 = reinterpret_cast<unsigned long long *>(b + o_u64);
     fifo.head = u64;
     fifo.tail = u64 + 1;
-    fifo.peak = u64 + 2;
-    fifo.peak_batch = u64 + 3;
-    fifo.dropped = u64 + 4;
+    fifo.peak_batch = u64 + 2;
+    // the words the host reads after a submit, copied together (HostStatus)
+    fifo.dropped = u64 + 3;
+    fifo.peak = u64 + 4;
+    fifo.out_count = reinterpret_cast<int32_t *>(u64 + 5);
+    fifo.status = fifo.out_count + 1;
     fifo.available = reinterpret_cast<double *>(b + o_avail);
     fifo.ring = reinterpret_cast<DevEvent *>(b + o_ring);
     fifo.ring_size = ring;
@@ -186,14 +194,13 @@ struct DeviceReadout {
     fifo.plan = reinterpret_cast<long long *>(b + o_plan);
     fifo.out = reinterpret_cast<DevEvent *>(b + o_out);
     e = cudaMemsetAsync(b + o_u64, 0, o_plan + 8 * 3 - o_u64, st);  // positions, counters, availability, words
-    if (e == cudaSuccess) e = cudaMallocHost(&h_status, sizeof(int32_t) * 2);
-    if (e == cudaSuccess) e = cudaMallocHost(&h_counters, sizeof(unsigned long long) * 2);
+    if (e == cudaSuccess) e = cudaMallocHost(&host, sizeof(HostStatus));
+    if (e == cudaSuccess) *host = HostStatus{};
     return e;
   }
   ~DeviceReadout() {
     cudaFree(arena);
-    if (h_status) cudaFreeHost(h_status);
-    if (h_counters) cudaFreeHost(h_counters);
+    if (host) cudaFreeHost(host);
   }
   static size_t next_pow2(size_t v) {
     size_t p = 1;
@@ -206,28 +213,26 @@ struct DeviceReadout {
                      cudaStream_t st) {
     ReadoutFifo f = fifo;
     f.gate = gate;
-    cudaError_t e = launch_readout_submit(events, count, sort, f, now, grid, st);
+    used_grid = grid > 0 ? grid : unknown_grid;
+    cudaError_t e = launch_readout_submit(events, count, sort, f, now, used_grid, st);
     return e == cudaSuccess ? copy_status(st) : e;
   }
   cudaError_t drain(cudaStream_t st) {
-    cudaError_t e = launch_readout_drain(fifo, grid, st);
+    cudaError_t e = launch_readout_drain(fifo, grid > 0 ? grid : unknown_grid, st);
     return e == cudaSuccess ? copy_status(st) : e;
   }
   cudaError_t copy_status(cudaStream_t st) {
-    cudaError_t e = cudaMemcpyAsync(h_status, fifo.out_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_status + 1, fifo.status, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_counters, fifo.dropped, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h_counters + 1, fifo.peak, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    return e;
+    return cudaMemcpyAsync(host, fifo.dropped, sizeof(HostStatus), cudaMemcpyDeviceToHost, st);
   }
+  static int blocks_for(size_t events) { return (int)std::min<size_t>(608, std::max<size_t>(1, (events + 4095) / 4096)); }
   // After the stream reached the copies: the next batches' sort grid.
   void observed(size_t events) {
-    grid = (int)std::min<size_t>(608, std::max<size_t>(1, (events + 4095) / 4096));
+    grid = blocks_for(events);
   }
   size_t bytes = 0;  // device memory held
-  // kernels of one submit: keys, packing, 12 radix passes of 3, the scan's 3, commit, release, advance
-  int launches() const { return readout_submit_launches(fifo.step > 0); }
+  int used_grid = 1;  // of the last submit
+  // kernels of the last submit: one, or keys, packing, 12 radix passes of 3, the scan's 3, commit, release, advance
+  int launches() const { return readout_submit_launches(fifo.step > 0, used_grid); }
 };
 
 // ---- handles --------------------------------------------------------------------
@@ -870,8 +875,8 @@ int dvs_sensor_create(dvs_scene *scene, const dvs_physic *physic, const dvs_sens
   ALLOC(s->slab_p, sizeof(int8_t) * (size_t)n * s->max_events, "event slabs");
   ALLOC(s->events, sizeof(DevEvent) * (size_t)n * s->max_events, "events");
   ALLOC(s->counters, sizeof(unsigned long long) * kCntSlots, "counters");
-  ALLOC(s->error_word, sizeof(int32_t), "error flag");
-  ALLOC(s->event_total, sizeof(int32_t), "event count");
+  ALLOC(s->event_total, 2 * sizeof(int32_t), "event count and error flag");
+  s->error_word = s->event_total + 1;  // beside the count: cleared and copied together
   ALLOC(s->d_state, sizeof(dvs_optical_state), "pose");
 #undef ALLOC
   if ((e = cudaMallocHost(&s->h_status, sizeof(int32_t) * 4)) != cudaSuccess) return bail(e, "status staging");
@@ -910,7 +915,6 @@ int dvs_sensor_destroy(dvs_sensor *s) {
   cudaFree(s->slab_p);
   cudaFree(s->events);
   cudaFree(s->counters);
-  cudaFree(s->error_word);
   cudaFree(s->event_total);
   cudaFree(s->radiance);
   cudaFree(s->ivs);
@@ -1090,8 +1094,7 @@ static void chunk_shape(const dvs_sensor *s, size_t n_cells, size_t rows, size_t
 static int clear_batch_outputs(dvs_sensor *s, cudaStream_t stream) {
   const int n = s->pixels();
   CUDA_TRY(cudaMemsetAsync(s->ev_count, 0, sizeof(int32_t) * n, stream), "clear events");
-  CUDA_TRY(cudaMemsetAsync(s->event_total, 0, sizeof(int32_t), stream), "clear events");
-  CUDA_TRY(cudaMemsetAsync(s->error_word, 0, sizeof(int32_t), stream), "clear status");
+  CUDA_TRY(cudaMemsetAsync(s->event_total, 0, 2 * sizeof(int32_t), stream), "clear events and status");
   return DVS_OK;
 }
 
@@ -1160,8 +1163,8 @@ static void collect_timers(dvs_sensor *s) {
 // the stream synchronized), appended to the ready list; counters updated.
 static int fetch_released(dvs_sensor *s) {
   DeviceReadout &d = *s->dro;
-  if (d.h_status[1]) return fail(DVS_ERR_CAPACITY, "readout queue capacity exceeds the device ring buffer");
-  const int32_t released = d.h_status[0];
+  if (d.host->status) return fail(DVS_ERR_CAPACITY, "readout queue capacity exceeds the device ring buffer");
+  const int32_t released = d.host->out_count;
   if (released > 0) {
     CUDA_TRY(grow_pinned(s->h_events, s->h_events_cap, (size_t)released), "event staging");
     CUDA_TRY(cudaMemcpyAsync(s->h_events, d.fifo.out, sizeof(DevEvent) * released, cudaMemcpyDeviceToHost,
@@ -1173,16 +1176,15 @@ static int fetch_released(dvs_sensor *s) {
     const DevEvent &e = s->h_events[i];
     s->ready.push_back(HostEvent{e.t, e.x, e.y, e.polarity, e.depth});
   }
-  s->stats.dropped = d.h_counters[0];
-  s->stats.peak_queue = d.h_counters[1];
+  s->stats.dropped = d.host->dropped;
+  s->stats.peak_queue = d.host->peak;
   return DVS_OK;
 }
 
 // collect_events (event_sensor.cu:296-305): status, events, readout.
 static int collect(dvs_sensor *s, double end, size_t *n_ready) {
-  CUDA_TRY(cudaMemcpyAsync(s->h_status, s->event_total, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream), "copy count");
-  CUDA_TRY(cudaMemcpyAsync(s->h_status + 1, s->error_word, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream),
-           "copy status");
+  CUDA_TRY(cudaMemcpyAsync(s->h_status, s->event_total, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream),
+           "copy count and status");
   CUDA_TRY(cudaStreamSynchronize(s->stream), "copy status");
   collect_timers(s);
   const int32_t count = s->h_status[0], word = s->h_status[1];
@@ -2045,8 +2047,12 @@ int dvs_batch_process(dvs_batch *b, const dvs_optical_interval *const *intervals
       if (e == cudaSuccess)
         e = launch_event_depth(s->view(), s->ivs, (int)counts[m], s->events, s->event_total, s->error_word,
                                s->counters, st);
-      if (e == cudaSuccess && s->dro)
+      if (e == cudaSuccess && s->dro) {
+        // the captured shape is replayed while the members' shapes stay, so a member without a batch behind it takes
+        // the form for few events; it serves any number
+        if (s->dro->grid == 0) s->dro->grid = 1;
         e = s->dro->submit(s->events, s->event_total, s->error_word, &s->ivs[counts[m] - 1].t1, st);
+      }
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(b->ev_end, st, cudaEventRecordExternal);
     cudaGraph_t graph = nullptr;
@@ -2196,8 +2202,8 @@ struct dvs_device_readout {
 namespace {
 int device_readout_fetch(dvs_device_readout *r) {
   CUDA_TRY(cudaStreamSynchronize(r->stream), "device readout");
-  if (r->dro.h_status[1]) return fail(DVS_ERR_CAPACITY, "readout queue capacity exceeds the device ring buffer");
-  const int32_t released = r->dro.h_status[0];
+  if (r->dro.host->status) return fail(DVS_ERR_CAPACITY, "readout queue capacity exceeds the device ring buffer");
+  const int32_t released = r->dro.host->out_count;
   if (released > 0) {
     CUDA_TRY(cudaMemcpyAsync(r->h_out, r->dro.fifo.out, sizeof(DevEvent) * released, cudaMemcpyDeviceToHost,
                              r->stream),
@@ -2286,6 +2292,7 @@ int dvs_device_readout_submit(dvs_device_readout *r, const dvs_event *events, si
     d.polarity = events[i].polarity;
     r->h_in[i] = d;
   }
+  r->dro.observed(n);  // the host knows this batch's size
   *r->h_count = (int32_t)n;
   *r->h_now = now;
   if (n) CUDA_TRY(cudaMemcpyAsync(r->d_in, r->h_in, sizeof(DevEvent) * n, cudaMemcpyHostToDevice, r->stream),
@@ -2297,7 +2304,6 @@ int dvs_device_readout_submit(dvs_device_readout *r, const dvs_event *events, si
   int rc = device_readout_fetch(r);
   if (rc) return rc;
   CUDA_TRY(cudaEventElapsedTime(&r->last_ms, r->e0, r->e1), "device readout timer");
-  r->dro.observed(n);
   *n_ready = r->ready.size() - r->head;
   return DVS_OK;
 }
@@ -2333,8 +2339,8 @@ int dvs_device_readout_read(dvs_device_readout *r, dvs_event *out, size_t capaci
 
 int dvs_device_readout_counters(const dvs_device_readout *r, uint64_t *dropped, uint64_t *peak_queue) {
   if (!r) return fail(DVS_ERR_INVALID, "null argument");
-  if (dropped) *dropped = r->dro.h_counters[0];
-  if (peak_queue) *peak_queue = r->dro.h_counters[1];
+  if (dropped) *dropped = r->dro.host->dropped;
+  if (peak_queue) *peak_queue = r->dro.host->peak;
   return DVS_OK;
 }
 

@@ -114,12 +114,14 @@ struct ReadoutFifo {
 // Orders a batch of *count events by (t, y, x) and passes it through the
 // FIFO at time *now (device memory, so a captured graph reads each step's);
 // the released events land in f.out (*f.out_count of them).  grid: blocks
-// of the sort and scan kernels (the sort's hist holds 256 x grid).
+// of the sort and scan kernels (the sort's hist holds 256 x grid); 1: the whole
+// submit in one kernel of one block.  prepare_readout: once per device before it.
+cudaError_t prepare_readout();
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st);
 cudaError_t launch_readout_drain(ReadoutFifo f, int grid, cudaStream_t st);
 // Kernels one launch_readout_submit enqueues (delayed: a bandwidth > 0 FIFO).
-int readout_submit_launches(bool delayed);
+int readout_submit_launches(bool delayed, int grid);
 
 // Error word bits (host maps them to DVS_ERR_* with capacity first, as
 // event_sensor.cu:300-301 tests code 1 before any other code).

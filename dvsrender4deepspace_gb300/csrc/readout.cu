@@ -44,6 +44,13 @@ constexpr int kPasses = 12;          // 4 bytes of the (y, x) key, then 8 of the
 constexpr int kScanThreads = 1024;   // one thread per sort block in the per-digit scan
 constexpr unsigned kFull = 0xffffffffu;
 
+// The blocks that run a phase together: the grid of its own kernel, or the one
+// block of ro_block_kernel, which runs all phases one after the other.
+struct Team {
+  int block, blocks;
+};
+__device__ __forceinline__ Team grid_team() { return Team{(int)blockIdx.x, (int)gridDim.x}; }
+
 // Order-preserving bits of a double (the sort key of t) and back.
 __device__ __forceinline__ unsigned long long time_key(double t) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(t);
@@ -117,10 +124,10 @@ __device__ __forceinline__ int sorted_buffer(const KeyLayout &L) { return __popc
 __device__ __forceinline__ unsigned digit_of(int pass, unsigned long long kt, unsigned kyx) {
   return pass < 4 ? (kyx >> (8 * pass)) & 0xffu : (unsigned)(kt >> (8 * (pass - 4))) & 0xffu;
 }
-// [begin, end) of block b's tile when n items are split over gridDim.x blocks.
-__device__ __forceinline__ void tile_of(int n, int b, int &begin, int &end) {
-  const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-  begin = min(n, b * per);
+// [begin, end) of the block's tile when n items are split over the team.
+__device__ __forceinline__ void tile_of(int n, Team team, int &begin, int &end) {
+  const int per = (n + team.blocks - 1) / team.blocks;
+  begin = min(n, team.block * per);
   end = min(n, begin + per);
 }
 __device__ __forceinline__ unsigned long long ring_index(const ReadoutFifo &f, unsigned long long c) {
@@ -152,7 +159,7 @@ __device__ __forceinline__ long long first_after(const double *a, long long k, d
 // Keys of the batch in arrival order, the OR of every key against the first
 // event's (varying[0..1], zeroed before the launch) and the first event's time
 // key (varying[2]).  256 threads.
-__global__ void __launch_bounds__(256) ro_keys_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s) {
+__device__ __forceinline__ void ro_keys(Team team, const DevEvent *events, const int32_t *count, ReadoutSort s) {
   __shared__ unsigned long long red[256 / 32][2];
   const int n = *count;
   if (n <= 0) return;  // grid-uniform
@@ -161,7 +168,7 @@ __global__ void __launch_bounds__(256) ro_keys_kernel(const DevEvent *events, co
   const unsigned kyx0 = yx_key(first);
   unsigned long long dt = 0;
   unsigned dyx = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = team.block * blockDim.x + threadIdx.x; i < n; i += team.blocks * blockDim.x) {
     const DevEvent e = events[i];
     const unsigned long long kt = time_key(e.t);
     const unsigned kyx = yx_key(e);
@@ -179,7 +186,7 @@ __global__ void __launch_bounds__(256) ro_keys_kernel(const DevEvent *events, co
     red[warp][1] = yx;
   }
   __syncthreads();
-  if (blockIdx.x == 0 && threadIdx.x == 0) s.varying[2] = kt0;
+  if (team.block == 0 && threadIdx.x == 0) s.varying[2] = kt0;
   if (threadIdx.x == 0) {
     unsigned long long a = 0, b = 0;
     for (int w = 0; w < 256 / 32; ++w) {
@@ -192,11 +199,11 @@ __global__ void __launch_bounds__(256) ro_keys_kernel(const DevEvent *events, co
 }
 
 // Packed layout: the packed key replaces the time key, in place.
-__global__ void __launch_bounds__(256) ro_pack_kernel(const int32_t *count, ReadoutSort s) {
+__device__ __forceinline__ void ro_pack(Team team, const int32_t *count, ReadoutSort s) {
   const KeyLayout L = key_layout(s);
   if (!L.packed) return;  // grid-uniform
   const int n = *count;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  for (int i = team.block * blockDim.x + threadIdx.x; i < n; i += team.blocks * blockDim.x)
     s.kt[0][i] = pack_key(L, s.kt[0][i], s.kyx[0][i]);
 }
 
@@ -236,7 +243,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan_256(unsigned v, unsigne
 
 // Per block: the histogram of the pass's digit over its tile, digit-major
 // (hist[d * grid + b]).
-__global__ void __launch_bounds__(kSortThreads) ro_hist_kernel(int pass, const int32_t *count, ReadoutSort s) {
+__device__ __forceinline__ void ro_hist(Team team, int pass, const int32_t *count, ReadoutSort s) {
   constexpr int kPer = 4;  // keys per thread and round: their loads are in flight together
   __shared__ unsigned h[kDigits];
   const KeyLayout L = key_layout(s);
@@ -248,7 +255,7 @@ __global__ void __launch_bounds__(kSortThreads) ro_hist_kernel(int pass, const i
   h[threadIdx.x] = 0;
   __syncthreads();
   int begin, end;
-  tile_of(n, blockIdx.x, begin, end);
+  tile_of(n, team, begin, end);
   for (int r0 = begin; r0 < end; r0 += kPer * kSortThreads) {  // block-uniform rounds: every lane reaches the match
     unsigned d[kPer];
 #pragma unroll
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(kSortThreads) ro_hist_kernel(int pass, const i
     for (int j = 0; j < kPer; ++j) count_digit(h, d[j], d[j] != kFull, aggregate);
   }
   __syncthreads();
-  s.hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
+  s.hist[threadIdx.x * team.blocks + team.block] = h[threadIdx.x];
 }
 
 // Block d (one per digit, grid <= 1024 sort blocks, one thread each): the
@@ -305,7 +312,7 @@ __global__ void __launch_bounds__(kScanThreads) ro_scan_kernel(int pass, int gri
 // then written out in that order, so a digit's keys of one tile land in one
 // run of consecutive addresses instead of one scattered store each.
 constexpr int kTileKeys = 4 * kSortThreads;
-__global__ void __launch_bounds__(kSortThreads) ro_scatter_kernel(int pass, const int32_t *count, ReadoutSort s) {
+__device__ __forceinline__ void ro_scatter(Team team, int pass, const int32_t *count, ReadoutSort s) {
   constexpr int kWarps = kSortThreads / 32, kPer = kTileKeys / kSortThreads;
   __shared__ unsigned base[kDigits], tcount[kDigits], toff[kDigits], run[kDigits];
   __shared__ unsigned warp_total[kWarps];
@@ -321,9 +328,9 @@ __global__ void __launch_bounds__(kSortThreads) ro_scatter_kernel(int pass, cons
   unsigned long long *kt_out = kt_of(s, 1 - cur);
   unsigned *kyx_out = kyx_of(s, 1 - cur), *idx_out = idx_of(s, 1 - cur);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  base[t] = block_exclusive_scan_256(s.digit_total[t], warp_total) + s.hist[t * gridDim.x + blockIdx.x];
+  base[t] = block_exclusive_scan_256(s.digit_total[t], warp_total) + s.hist[t * team.blocks + team.block];
   int begin, end;
-  tile_of(n, blockIdx.x, begin, end);
+  tile_of(n, team, begin, end);
   for (int c0 = begin; c0 < end; c0 += kTileKeys) {  // block-uniform tiles
     const int tn = min(kTileKeys, end - c0);
     unsigned long long k_t[kPer];
@@ -425,13 +432,13 @@ __device__ __forceinline__ unsigned long long slack_key(const KeyLayout &L, unsi
 }
 
 // Per block: the maximum of u_k over its tile.
-__global__ void __launch_bounds__(256) ro_fifo_max_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+__device__ __forceinline__ void ro_fifo_max(Team team, const int32_t *count, ReadoutSort s, ReadoutFifo f) {
   __shared__ unsigned long long red[256 / 32];
   const KeyLayout L = key_layout(s);
   const int n = *count, cur = sorted_buffer(L);
   const unsigned long long *kt = kt_of(s, cur);
   int begin, end;
-  tile_of(n, blockIdx.x, begin, end);
+  tile_of(n, team, begin, end);
   unsigned long long m = 0;
   for (int k = begin + threadIdx.x; k < end; k += blockDim.x) m = u64_max(m, slack_key(L, kt[k], k, f.step));
   m = warp_max_key(m);
@@ -440,13 +447,13 @@ __global__ void __launch_bounds__(256) ro_fifo_max_kernel(const int32_t *count, 
   if (threadIdx.x == 0) {
     unsigned long long b = red[0];
     for (int w = 1; w < 256 / 32; ++w) b = u64_max(b, red[w]);
-    f.block_max[blockIdx.x] = b;
+    f.block_max[team.block] = b;
   }
 }
 
 // Per block: the prefix maximum from the carried availability and the earlier
 // blocks' maxima, then the completion and delivery time of every arrival.
-__global__ void __launch_bounds__(256) ro_fifo_scan_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+__device__ __forceinline__ void ro_fifo_scan(Team team, const int32_t *count, ReadoutSort s, ReadoutFifo f) {
   constexpr int kWarps = 256 / 32;
   __shared__ unsigned long long wmax[kWarps];
   __shared__ unsigned long long carry_in;
@@ -455,9 +462,9 @@ __global__ void __launch_bounds__(256) ro_fifo_scan_kernel(const int32_t *count,
   const unsigned long long *kt = kt_of(s, cur);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int begin, end;
-  tile_of(n, blockIdx.x, begin, end);
+  tile_of(n, team, begin, end);
   unsigned long long c = threadIdx.x == 0 ? time_key(*f.available) : 0ull;
-  for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) c = u64_max(c, f.block_max[b]);
+  for (int b = threadIdx.x; b < (int)team.block; b += blockDim.x) c = u64_max(c, f.block_max[b]);
   c = warp_max_key(c);
   if (lane == 0) wmax[warp] = c;
   __syncthreads();
@@ -493,7 +500,7 @@ __global__ void __launch_bounds__(256) ro_fifo_scan_kernel(const int32_t *count,
 
 // Occupancy at every arrival: the overflow flag and the batch's peak, reduced
 // per warp and per block first (one atomic per block, not per event).
-__global__ void __launch_bounds__(256) ro_fifo_occupancy_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+__device__ __forceinline__ void ro_fifo_occupancy(Team team, const int32_t *count, ReadoutSort s, ReadoutFifo f) {
   __shared__ unsigned red_peak[256 / 32];
   __shared__ int red_over[256 / 32];
   const KeyLayout L = key_layout(s);
@@ -503,7 +510,7 @@ __global__ void __launch_bounds__(256) ro_fifo_occupancy_kernel(const int32_t *c
   // occupancy + 1 <= ring entries (< 2^25) + batch events (< 2^31): fits 32 bits
   unsigned peak = 0;
   int over = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+  for (int k = team.block * blockDim.x + threadIdx.x; k < n; k += team.blocks * blockDim.x) {
     const double t = key_time(time_key_of(L, kt[k]));
     const long long lo = first_after(f.delivery, k, t);  // earlier arrivals still queued at t: [lo, k)
     const long long occ = carried_after(f, head, tail, t) + (k - lo);
@@ -533,9 +540,9 @@ __global__ void __launch_bounds__(256) ro_fifo_occupancy_kernel(const int32_t *c
 // the release plan (carried released, batch released, batch accepted), the
 // availability and the peak.  Overflow: the serial FIFO with its drops
 // (event_readout.cpp:13-30), writing the output and the ring directly.
-__global__ void ro_fifo_commit_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
-                                      const double *now_at) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ __forceinline__ void ro_fifo_commit(const DevEvent *events, const int32_t *count, const ReadoutSort &s,
+                                               const ReadoutFifo &f, const double *now_at) {
+  if (threadIdx.x != 0) return;
   const double now = *now_at;
   if (f.gate && *f.gate) {  // the batch failed: the FIFO neither takes nor releases anything
     f.plan[0] = -1;
@@ -607,13 +614,13 @@ __global__ void ro_fifo_commit_kernel(const DevEvent *events, const int32_t *cou
 
 // The plan's copies: released carried entries and batch events to the output
 // (queue order), the batch's later deliveries to the ring.
-__global__ void ro_fifo_release_kernel(const DevEvent *events, ReadoutSort s, ReadoutFifo f) {
+__device__ __forceinline__ void ro_fifo_release(Team team, const DevEvent *events, ReadoutSort s, ReadoutFifo f) {
   const long long carried_out = f.plan[0], batch_out = f.plan[1], accepted = f.plan[2];
   if (carried_out < 0) return;
   const int cur = sorted_buffer(key_layout(s));
   const unsigned long long head = *f.head, tail = *f.tail;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < carried_out + accepted; i += stride) {
+  const long long stride = (long long)team.blocks * blockDim.x;
+  for (long long i = team.block * (long long)blockDim.x + threadIdx.x; i < carried_out + accepted; i += stride) {
     if (i < carried_out) {
       f.out[i] = f.ring[ring_index(f, head + i)];
     } else {
@@ -626,10 +633,144 @@ __global__ void ro_fifo_release_kernel(const DevEvent *events, ReadoutSort s, Re
   }
 }
 
-__global__ void ro_fifo_advance_kernel(ReadoutFifo f) {
-  if (f.plan[0] < 0) return;
+__device__ __forceinline__ void ro_fifo_advance(const ReadoutFifo &f) {
+  if (threadIdx.x != 0 || f.plan[0] < 0) return;
   *f.head += (unsigned long long)f.plan[0];
   *f.tail += (unsigned long long)(f.plan[2] - f.plan[1]);
+}
+
+// ---- the phases as kernels ------------------------------------------------------------
+__global__ void __launch_bounds__(256) ro_keys_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s) {
+  ro_keys(grid_team(), events, count, s);
+}
+__global__ void __launch_bounds__(256) ro_pack_kernel(const int32_t *count, ReadoutSort s) {
+  ro_pack(grid_team(), count, s);
+}
+__global__ void __launch_bounds__(kSortThreads) ro_hist_kernel(int pass, const int32_t *count, ReadoutSort s) {
+  ro_hist(grid_team(), pass, count, s);
+}
+__global__ void __launch_bounds__(kSortThreads) ro_scatter_kernel(int pass, const int32_t *count, ReadoutSort s) {
+  ro_scatter(grid_team(), pass, count, s);
+}
+__global__ void __launch_bounds__(256) ro_fifo_max_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+  ro_fifo_max(grid_team(), count, s, f);
+}
+__global__ void __launch_bounds__(256) ro_fifo_scan_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+  ro_fifo_scan(grid_team(), count, s, f);
+}
+__global__ void __launch_bounds__(256) ro_fifo_occupancy_kernel(const int32_t *count, ReadoutSort s, ReadoutFifo f) {
+  ro_fifo_occupancy(grid_team(), count, s, f);
+}
+__global__ void ro_fifo_release_kernel(const DevEvent *events, ReadoutSort s, ReadoutFifo f) {
+  ro_fifo_release(grid_team(), events, s, f);
+}
+__global__ void ro_fifo_commit_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
+                                      const double *now_at) {
+  ro_fifo_commit(events, count, s, f, now_at);
+}
+__global__ void ro_fifo_advance_kernel(ReadoutFifo f) { ro_fifo_advance(f); }
+
+// ---- a small batch in one block --------------------------------------------------------
+// Most batches hold few events, and the phases' kernels then cost their launches:
+// 44 of them, 0.17-0.2 ms a batch.  One block runs the whole submit
+// instead.  Up to kBlockEvents events are sorted in shared memory by a bitonic
+// network on (t, (y, x), arrival) -- the arrival index makes the order the
+// stable one -- and left in the key buffers as the radix passes would leave
+// them; more events (a burst after small batches; the next submit is sized by
+// it) go through the radix passes with this block as the whole team.
+constexpr int kBlockEvents = 4096;
+struct BlockSort {
+  unsigned long long kt[kBlockEvents];
+  unsigned kyx[kBlockEvents], idx[kBlockEvents];
+};
+__device__ __forceinline__ void block_sort(const DevEvent *events, int n, BlockSort &b, const ReadoutSort &s) {
+  const int t = threadIdx.x;
+  int m = 1;
+  while (m < n) m <<= 1;
+  for (int i = t; i < m; i += kSortThreads) {
+    unsigned long long kt = ~0ull;  // above every key of an event: its arrival index is larger too
+    unsigned kyx = kFull;
+    if (i < n) {
+      kt = time_key(events[i].t);
+      kyx = yx_key(events[i]);
+    }
+    b.kt[i] = kt;
+    b.kyx[i] = kyx;
+    b.idx[i] = (unsigned)i;
+  }
+  __syncthreads();
+  for (int size = 2; size <= m; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int q = t; q < m / 2; q += kSortThreads) {
+        const int i = 2 * q - (q & (stride - 1)), j = i + stride;
+        const unsigned long long ki = b.kt[i], kj = b.kt[j];
+        const unsigned yi = b.kyx[i], yj = b.kyx[j], ii = b.idx[i], ij = b.idx[j];
+        const bool after = ki != kj ? ki > kj : yi != yj ? yi > yj : ii > ij;
+        if (after == ((i & size) == 0)) {
+          b.kt[i] = kj;
+          b.kt[j] = ki;
+          b.kyx[i] = yj;
+          b.kyx[j] = yi;
+          b.idx[i] = ij;
+          b.idx[j] = ii;
+        }
+      }
+      __syncthreads();
+    }
+  // nothing varies that a pass would still have to order: the keys stay in buffer 0, unpacked
+  for (int i = t; i < n; i += kSortThreads) {
+    s.kt[0][i] = b.kt[i];
+    s.idx[0][i] = b.idx[i];
+  }
+  __syncthreads();
+}
+__global__ void __launch_bounds__(kSortThreads) ro_block_kernel(const DevEvent *events, const int32_t *count,
+                                                                ReadoutSort s, ReadoutFifo f, const double *now) {
+  extern __shared__ __align__(16) unsigned char ro_shared[];
+  const Team team{0, 1};
+  const int n = *count;
+  const bool small = n <= kBlockEvents;
+  if (threadIdx.x == 0) {
+    // small: the layout of an unpacked key of which no bit varies is read as buffer 0, sorted
+    s.varying[0] = small ? 0x8000000000000000ull : 0ull;
+    s.varying[1] = small ? 1ull : 0ull;
+    s.varying[2] = 0ull;
+    *f.overflow = 0;
+    *f.peak_batch = 0;
+  }
+  __syncthreads();
+  if (small) {
+    block_sort(events, n, *reinterpret_cast<BlockSort *>(ro_shared), s);
+  } else {
+    ro_keys(team, events, count, s);
+    __syncthreads();
+    ro_pack(team, count, s);
+    __syncthreads();
+    for (int pass = 0; pass < kPasses; ++pass) {
+      ro_hist(team, pass, count, s);
+      __syncthreads();
+      if ((key_layout(s).mask >> pass) & 1u) {  // one block: a digit's total is its count, and no block is before it
+        s.digit_total[threadIdx.x] = s.hist[threadIdx.x];
+        s.hist[threadIdx.x] = 0;
+      }
+      __syncthreads();
+      ro_scatter(team, pass, count, s);
+      __syncthreads();
+    }
+  }
+  if (f.step > 0) {
+    ro_fifo_max(team, count, s, f);
+    __syncthreads();
+    ro_fifo_scan(team, count, s, f);
+    __syncthreads();
+    ro_fifo_occupancy(team, count, s, f);
+    __syncthreads();
+  }
+  ro_fifo_commit(events, count, s, f, now);
+  __syncthreads();
+  ro_fifo_release(team, events, s, f);
+  __syncthreads();
+  ro_fifo_advance(f);
 }
 
 // drain (event_readout.cpp:31-34): every pending entry, in order.
@@ -646,11 +787,19 @@ __global__ void ro_drain_commit_kernel(ReadoutFifo f) {
 
 }  // namespace
 
-int readout_submit_launches(bool delayed) { return 2 + kPasses * 3 + (delayed ? 3 : 0) + 3; }
+int readout_submit_launches(bool delayed, int grid) { return grid <= 1 ? 1 : 2 + kPasses * 3 + (delayed ? 3 : 0) + 3; }
+
+cudaError_t prepare_readout() {
+  return cudaFuncSetAttribute(ro_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockSort));
+}
 
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st) {
   if (grid < 1 || grid > kScanThreads) return cudaErrorInvalidValue;
+  if (grid == 1) {
+    ro_block_kernel<<<1, kSortThreads, sizeof(BlockSort), st>>>(events, count, s, f, now);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaMemsetAsync(s.varying, 0, 3 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   ro_keys_kernel<<<grid, 256, 0, st>>>(events, count, s);
