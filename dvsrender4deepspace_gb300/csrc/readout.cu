@@ -44,8 +44,8 @@ constexpr int kPasses = 12;          // 4 bytes of the (y, x) key, then 8 of the
 constexpr int kScanThreads = 1024;   // one thread per sort block in the per-digit scan
 constexpr unsigned kFull = 0xffffffffu;
 
-// The blocks that run a phase together: the grid of its own kernel, or the one
-// block of ro_block_kernel, which runs all phases one after the other.
+// The blocks that run a phase together: the grid of its own kernel, or the
+// cluster (or one block) of ro_cluster_kernel, which runs all phases one after the other.
 struct Team {
   int block, blocks;
 };
@@ -670,14 +670,20 @@ __global__ void ro_fifo_commit_kernel(const DevEvent *events, const int32_t *cou
 }
 __global__ void ro_fifo_advance_kernel(ReadoutFifo f) { ro_fifo_advance(f); }
 
-// ---- a small batch in one block --------------------------------------------------------
+// ---- a batch in one cluster ------------------------------------------------------------
 // Most batches hold few events, and the phases' kernels then cost their launches:
-// 44 of them, 0.17-0.2 ms a batch.  One block runs the whole submit
-// instead.  Up to kBlockEvents events are sorted in shared memory by a bitonic
+// 44 of them, 0.17-0.2 ms a batch.  One launch of one cluster runs the whole
+// submit instead.  Up to kBlockEvents events are sorted by its first block in shared memory, by a bitonic
 // network on (t, (y, x), arrival) -- the arrival index makes the order the
 // stable one -- and left in the key buffers as the radix passes would leave
 // them; more events (a burst after small batches; the next submit is sized by
-// it) go through the radix passes with this block as the whole team.
+// it) go through the radix passes with the cluster's blocks as the team and its hardware barrier between the phases.
+// (One block as the team took 5.3 ms for a burst of 64,500 events.)
+constexpr int kClusterBlocks = 8;  // the portable cluster size
+__device__ __forceinline__ void cluster_barrier() {
+  __threadfence();  // the phases hand over through global memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 constexpr int kBlockEvents = 4096;
 struct BlockSort {
   unsigned long long kt[kBlockEvents];
@@ -724,53 +730,65 @@ __device__ __forceinline__ void block_sort(const DevEvent *events, int n, BlockS
   }
   __syncthreads();
 }
-__global__ void __launch_bounds__(kSortThreads) ro_block_kernel(const DevEvent *events, const int32_t *count,
-                                                                ReadoutSort s, ReadoutFifo f, const double *now) {
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kSortThreads)
+    ro_cluster_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f, const double *now) {
   extern __shared__ __align__(16) unsigned char ro_shared[];
-  const Team team{0, 1};
   const int n = *count;
-  const bool small = n <= kBlockEvents;
-  if (threadIdx.x == 0) {
-    // small: the layout of an unpacked key of which no bit varies is read as buffer 0, sorted
+  const bool small = n <= kBlockEvents;  // the same in every block
+  const bool first = blockIdx.x == 0;
+  if (small && !first) return;
+  const Team team = small ? Team{0, 1} : Team{(int)blockIdx.x, kClusterBlocks};
+  const auto barrier = [small] {
+    if (small) __syncthreads();
+    else cluster_barrier();
+  };
+  if (first && threadIdx.x == 0) {
+    // small: the layout of an unpacked key whose passes leave it in buffer 0
     s.varying[0] = small ? 0x8000000000000000ull : 0ull;
     s.varying[1] = small ? 1ull : 0ull;
     s.varying[2] = 0ull;
     *f.overflow = 0;
     *f.peak_batch = 0;
   }
-  __syncthreads();
+  barrier();
   if (small) {
     block_sort(events, n, *reinterpret_cast<BlockSort *>(ro_shared), s);
   } else {
     ro_keys(team, events, count, s);
-    __syncthreads();
+    barrier();
     ro_pack(team, count, s);
-    __syncthreads();
+    barrier();
     for (int pass = 0; pass < kPasses; ++pass) {
+      if (!((key_layout(s).mask >> pass) & 1u)) continue;  // the digit is every key's
       ro_hist(team, pass, count, s);
-      __syncthreads();
-      if ((key_layout(s).mask >> pass) & 1u) {  // one block: a digit's total is its count, and no block is before it
-        s.digit_total[threadIdx.x] = s.hist[threadIdx.x];
-        s.hist[threadIdx.x] = 0;
+      barrier();
+      if (first) {  // thread d: digit d's counts over the blocks, scanned in place
+        unsigned run = 0;
+        for (int b = 0; b < kClusterBlocks; ++b) {
+          const unsigned c = s.hist[threadIdx.x * kClusterBlocks + b];
+          s.hist[threadIdx.x * kClusterBlocks + b] = run;
+          run += c;
+        }
+        s.digit_total[threadIdx.x] = run;
       }
-      __syncthreads();
+      barrier();
       ro_scatter(team, pass, count, s);
-      __syncthreads();
+      barrier();
     }
   }
   if (f.step > 0) {
     ro_fifo_max(team, count, s, f);
-    __syncthreads();
+    barrier();
     ro_fifo_scan(team, count, s, f);
-    __syncthreads();
+    barrier();
     ro_fifo_occupancy(team, count, s, f);
-    __syncthreads();
+    barrier();
   }
-  ro_fifo_commit(events, count, s, f, now);
-  __syncthreads();
+  if (first) ro_fifo_commit(events, count, s, f, now);
+  barrier();
   ro_fifo_release(team, events, s, f);
-  __syncthreads();
-  ro_fifo_advance(f);
+  barrier();
+  if (first) ro_fifo_advance(f);
 }
 
 // drain (event_readout.cpp:31-34): every pending entry, in order.
@@ -790,14 +808,14 @@ __global__ void ro_drain_commit_kernel(ReadoutFifo f) {
 int readout_submit_launches(bool delayed, int grid) { return grid <= 1 ? 1 : 2 + kPasses * 3 + (delayed ? 3 : 0) + 3; }
 
 cudaError_t prepare_readout() {
-  return cudaFuncSetAttribute(ro_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockSort));
+  return cudaFuncSetAttribute(ro_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockSort));
 }
 
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st) {
   if (grid < 1 || grid > kScanThreads) return cudaErrorInvalidValue;
   if (grid == 1) {
-    ro_block_kernel<<<1, kSortThreads, sizeof(BlockSort), st>>>(events, count, s, f, now);
+    ro_cluster_kernel<<<kClusterBlocks, kSortThreads, sizeof(BlockSort), st>>>(events, count, s, f, now);
     return cudaGetLastError();
   }
   cudaError_t e = cudaMemsetAsync(s.varying, 0, 3 * sizeof(unsigned long long), st);
