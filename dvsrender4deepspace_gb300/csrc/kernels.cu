@@ -83,31 +83,20 @@ __global__ void __launch_bounds__(128, kRays == 4   ? DVS_TRACE_QUAD_MIN_BLOCKS
                                        s_warp[wib], s_beam[kBeam ? wib : 0]);
 }
 
-// Few poses per pixel: one warp per (pixel, pose), lanes carrying the
-// pixel's sub-rays (sample_pixel_subrays).  Item w = (rank, cell) with
-// consecutive warps on the same pixel.
 template <int kMode, int kGeo>
-__global__ void __launch_bounds__(128, DVS_TRACE_PAIR_MIN_BLOCKS)
-    trace_subray_kernel(SceneView S, int n_pix, const int32_t *rank_list, const CellPose *poses, int c0, int nc,
-                        double *radiance, float *depth_out, unsigned long long *counters) {
-  __shared__ int s_code[kWarpsPerBlock][kStackSlots];
-  __shared__ float s_t[kWarpsPerBlock][kStackSlots];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const long long warp = (long long)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= (long long)n_pix * nc) return;  // warp-uniform
-  const int rank = (int)(warp / nc), cell = (int)(warp % nc);
-  const int pixel = __ldg(S.pixel_of_rank + (rank_list ? rank_list[rank] : rank));
+__global__ void __launch_bounds__(128, 4)
+    trace_poses_kernel(const __grid_constant__ SceneView S, int n_pix, const int32_t *rank_list, const CellPose *poses,
+                       int c0, int nc, PoseShape shape, double *radiance, float *depth_out,
+                       unsigned long long *counters) {
+  __shared__ PoseShared s_warp[kWarpsPerBlock];
+  const int wib = threadIdx.x >> 5;
+  const long long item = (long long)blockIdx.x * kWarpsPerBlock + wib;
+  const long long first = item / nc * shape.pixels;
+  if (first >= n_pix) return;  // warp-uniform
+  const int cell = (int)(item % nc);
   const CellPose pose = poses[c0 + cell];
-  const PixelSample s = sample_pixel_subrays<kMode, kGeo>(S, pixel, pose, s_code[wib], s_t[wib]);
-  if (lane == 0) {
-    const size_t o = (size_t)cell * n_pix + rank;
-    store_radiance(S, radiance, o, s.valid ? s.radiance : __longlong_as_double(0x7ff8000000000000ll));
-    if (depth_out) depth_out[o] = s.depth;
-    if (counters) {
-      atomicAdd(counters + kCntPrimary, (unsigned long long)s.primary);
-      atomicAdd(counters + kCntShadow, (unsigned long long)s.shadow);
-    }
-  }
+  trace_pose_item<kMode, kGeo>(S, n_pix, rank_list, pose, cell, shape, radiance, depth_out, counters, (int)first,
+                               s_warp[wib]);
 }
 
 template <class Rng>
@@ -326,18 +315,38 @@ cudaError_t launch_cell_poses(const dvs_optical_interval *ivs, const Cell *cells
 }
 
 namespace {
+constexpr long long kResidentWarps = 2432;  // 152 SMs x 16 warps
+// Few poses: packets of sub-rays.  One sub-ray a pixel fills a packet with a block of 8 x 4 pixels; where so few pixels
+// leave the GPU idle, narrower packets on more warps.
+bool trace_by_pose(const SceneView &scene, int n_pix, int nc) {
+  if (nc >= 8) return false;
+  return scene.samples > 1 || (long long)n_pix * nc < 32 * kResidentWarps;
+}
+PoseShape pose_item_shape(int n_pix, int nc, int ss2, bool scattered) {
+  PoseShape s{1, 0, 0};
+  while ((1 << s.lanes_log2) < ss2 && s.lanes_log2 < 5) ++s.lanes_log2;
+  const int per_packet = 32 >> s.lanes_log2, runs = (ss2 + 31) / 32;
+  // pixels of an item: a packet's, then more for the beam while every SM has items
+  const int most = kPoseTerms / ((1 << s.lanes_log2) + 1);
+  const auto items = [&](int pixels) { return (long long)((n_pix + pixels - 1) / pixels) * nc; };
+  const int limit = scattered ? 1 : most < 32 ? most : 32;
+  while (2 * s.pixels <= limit && items(2 * s.pixels) >= 2 * kResidentWarps && s.pixels * runs < 64 * per_packet)
+    s.pixels *= 2;
+  s.beam = (s.pixels + per_packet - 1) / per_packet * runs >= 8;
+  return s;
+}
 template <int kGeo>
 void trace_list_geo(const SceneView &scene, int n_pix, const int32_t *rank_list, const CellPose *poses, int c0, int nc,
                     int cw_log2, double *radiance, float *depth, unsigned long long *counters, cudaStream_t s) {
-  if (scene.samples * scene.samples >= 32 && nc <= 8) {
-    // few poses per pixel: sub-ray packets (one warp per pixel and pose)
-    const int grid = blocks((long long)n_pix * nc * 32, 128);
+  if (trace_by_pose(scene, n_pix, nc)) {
+    const PoseShape shape = pose_item_shape(n_pix, nc, scene.samples * scene.samples, rank_list != nullptr);
+    const int grid = blocks((long long)((n_pix + shape.pixels - 1) / shape.pixels) * nc * 32, 128);
     if (depth)
-      trace_subray_kernel<kRadianceDepth, kGeo><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, radiance,
-                                                                     depth, counters);
+      trace_poses_kernel<kRadianceDepth, kGeo><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, shape,
+                                                                    radiance, depth, counters);
     else
-      trace_subray_kernel<kRadiance, kGeo><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, radiance,
-                                                                nullptr, counters);
+      trace_poses_kernel<kRadiance, kGeo><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, shape, radiance,
+                                                               nullptr, counters);
     return;
   }
   const int ss2 = scene.samples * scene.samples;
@@ -471,8 +480,8 @@ cudaError_t preload_cells() {
 template <int kGeo>
 cudaError_t preload_camera_geo() {
   cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, trace_subray_kernel<kRadianceDepth, kGeo>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_subray_kernel<kRadiance, kGeo>);
+  cudaError_t e = cudaFuncGetAttributes(&a, trace_poses_kernel<kRadianceDepth, kGeo>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_poses_kernel<kRadiance, kGeo>);
   if (e == cudaSuccess) e = preload_cells<kRadianceDepth, 1, kGeo>();
   if (e == cudaSuccess) e = preload_cells<kRadianceDepth, 2, kGeo>();
   if (e == cudaSuccess) e = preload_cells<kRadiance, 1, kGeo>();

@@ -115,7 +115,7 @@ struct ReadoutFifo {
 // FIFO at time *now (device memory, so a captured graph reads each step's);
 // the released events land in f.out (*f.out_count of them).  grid: blocks
 // of the sort and scan kernels (the sort's hist holds 256 x grid); 1: the whole
-// submit in one kernel of one block.  prepare_readout: once per device before it.
+// submit in one kernel of one cluster.  prepare_readout: once per device before it.
 cudaError_t prepare_readout();
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st);
@@ -207,6 +207,11 @@ cudaError_t launch_trace_jobs(const TraceJobs &jobs, int rays, int geometry, cud
 cudaError_t launch_circuit_jobs(const CircuitJob *jobs, int n_jobs, int total_blocks, bool fp32, bool philox,
                                 cudaStream_t s);
 
+// A warp's item in a trace of few poses: `pixels` Morton-adjacent pixels (at most 32) at one pose, 1 << lanes_log2
+// lanes on a pixel's sub-rays; beam as in ItemShape.
+struct PoseShape {
+  int32_t pixels, lanes_log2, beam;
+};
 cudaError_t launch_trace_cells(const SceneView &scene, int n_pix, const CellPose *poses, int c0, int nc,
                                int cw_log2, double *radiance, float *depth, unsigned long long *counters,
                                cudaStream_t s);

@@ -164,6 +164,91 @@ __device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, 
   }
 }
 
+// Few poses per pixel (camera frames, the initial pose, short exposures, the
+// adaptive probes): a warp's item is several pixels at one pose, its packets 32
+// sub-rays of one pixel, or of as many pixels as they fill, through the item's
+// beam.  After each run of sub-rays the lanes, one per pixel, add its terms in
+// sub-ray order: the FP64 sums of the serial loop, for all the item's
+// pixels at once.  (One lane summing its pixel's 64 terms of a packet through shuffles, and no beam, took
+// 69 ms for a 1280x720 frame with 256 sub-rays, the FP64 pipe busy with one lane's sums.)
+constexpr int kPoseTerms = 288;  // pixels x (sub-rays of a run + 1)
+struct PoseShared {
+  int code[kStackSlots];
+  float t[kStackSlots];
+  Beam beam;
+  double term[kPoseTerms];
+  float hit_t[kPoseTerms];
+};
+template <int kMode, int kGeo>
+__device__ __forceinline__ void trace_pose_item(const SceneView &S, int n_pix, const int32_t *rank_list,
+                                                const CellPose &pose, int cell, PoseShape shape, double *radiance,
+                                                float *depth_out, unsigned long long *counters, int first,
+                                                PoseShared &sh) {
+  const int lane = threadIdx.x & 31, count = min(shape.pixels, n_pix - first);
+  const int run = 1 << shape.lanes_log2, per_packet = 32 >> shape.lanes_log2;
+  const int sub = lane & (run - 1), ss2 = S.samples * S.samples;
+  int pixel = 0;  // of lane i: the item's pixel i
+  if (lane < count) pixel = __ldg(S.pixel_of_rank + (rank_list ? rank_list[first + lane] : first + lane));
+  BeamLists lists{kNoList, kNoList, 0};
+  if (shape.beam) {
+    const float3 o = f3(pose.px, pose.py, pose.pz), l = inverse_direction(f3(pose.lx, pose.ly, pose.lz));
+    float3 dlo = f3(kInf(), kInf(), kInf()), dhi = -dlo;
+    if (lane < count) {
+      const int px_i = pixel % S.width, py_i = pixel / S.width, last = S.samples - 1;
+      for (int k = 0; k < (last ? 4 : 1); ++k) {
+        const float3 d = unit(rotate_ray(pose, f3(subray_x(S, px_i, k & 1 ? last : 0),
+                                                  -subray_y(S, py_i, k & 2 ? last : 0), -1)));
+        dlo = min3(dlo, d);
+        dhi = max3(dhi, d);
+      }
+    }
+    lists = close_beam<kGeo>(S, o, o, dlo, dhi, l, l, 0.0f, sh.beam, sh.code);
+  }
+  double sum = 0, depth = 0;
+  int valid_depth = 0;
+  unsigned primary = 0, shadow = 0;
+  for (int r0 = 0; r0 < ss2; r0 += run) {
+    for (int s0 = 0; s0 < count; s0 += per_packet) {
+      const int p = s0 + (lane >> shape.lanes_log2), r = r0 + sub;
+      const int pix = __shfl_sync(kFull, pixel, min(p, 31));
+      const bool live = p < count && r < ss2;
+      const int rr = live ? r : 0;
+      const RaySample s = sample_ray<kMode, kGeo, false>(S, subray_x(S, pix % S.width, rr % S.samples),
+                                                         subray_y(S, pix / S.width, rr / S.samples), pose, live,
+                                                         sh.code, sh.t, sh.beam, lists);
+      if (live) {
+        const int at = p * (run + 1) + sub;
+        sh.term[at] = s.overflow ? __longlong_as_double(0x7ff8000000000000ll) : s.term;
+        if (kMode != kRadiance) sh.hit_t[at] = s.hit ? s.t : -1.0f;
+      }
+      primary += live ? 1u : 0u;
+      shadow += s.lit ? 1u : 0u;
+    }
+    __syncwarp();
+    if (lane < count) {
+      const int m = min(run, ss2 - r0), at = lane * (run + 1);
+      for (int i = 0; i < m; ++i) {
+        sum += sh.term[at + i];
+        if (kMode != kRadiance && sh.hit_t[at + i] >= 0.0f) {
+          depth += sh.hit_t[at + i];
+          ++valid_depth;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (lane < count) {
+    const size_t o = (size_t)cell * n_pix + first + lane;
+    store_radiance(S, radiance, o, sum / ss2);
+    if (kMode != kRadiance) depth_out[o] = valid_depth ? float(depth / valid_depth) : -1.0f;
+  }
+  const unsigned prim = warp_sum(primary), shad = warp_sum(shadow);
+  if (lane == 0 && counters) {
+    atomicAdd(counters + kCntPrimary, (unsigned long long)prim);
+    atomicAdd(counters + kCntShadow, (unsigned long long)shad);
+  }
+}
+
 // One pixel of a circuit launch (generate_pixels' circuit half,
 // event_sensor.cu:35-50, over one cell chunk): thread r of the launch
 // integrates rank rank_list[r] (or r) from radiance row r.  Called by
