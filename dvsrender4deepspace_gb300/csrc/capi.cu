@@ -531,6 +531,18 @@ int dvs_scene_create(const float *vertices, const float *normals, const uint32_t
       s.a1 = material_albedo(albedos[b], hapke->w);
       s.a2 = material_albedo(albedos[c], hapke->w);
     }
+    float e1[3], e2[3];
+    for (int d = 0; d < 3; ++d) {
+      e1[d] = vertices[3 * (size_t)b + d] - vertices[3 * (size_t)a + d];
+      e2[d] = vertices[3 * (size_t)c + d] - vertices[3 * (size_t)a + d];
+    }
+    const float x = e1[1] * e2[2] - e1[2] * e2[1], y = e1[2] * e2[0] - e1[0] * e2[2], z = e1[0] * e2[1] - e1[1] * e2[0];
+    const float len = std::sqrt(x * x + y * y + z * z);
+    if (len > 0.0f) {
+      s.ng[0] = x / len;
+      s.ng[1] = y / len;
+      s.ng[2] = z / len;
+    }
   }
   const std::vector<int32_t> order = morton_pixel_order(camera->width, camera->height);
 

@@ -717,9 +717,10 @@ __device__ __forceinline__ float next_toward(float x, float to) {
   return to != 0 ? y : x;
 }
 
-// shadow_origin (device_optics.cuh:37-51) from the leaf-order triangle record.
-__device__ float3 shadow_origin(float3 a, float3 e1, float3 e2, float u, float v, float3 light) {
-  float3 point = a + u * e1 + v * e2, normal = unit(cross(e1, e2));
+// shadow_origin (device_optics.cuh:37-51) from the leaf-order triangle and shading records (normal: ShadeRecord::ng).
+__device__ __forceinline__ float3 shadow_origin(float3 a, float3 e1, float3 e2, float3 normal, float u, float v,
+                                                float3 light) {
+  float3 point = a + u * e1 + v * e2;
   if (dot(normal, light) < 0) normal = -normal;
   constexpr float epsilon = 5.960464477539063e-8f, gamma = 8 * epsilon / (1 - 8 * epsilon);
   float3 error = f3(gamma * (fabsf(a.x) + fabsf(u * e1.x) + fabsf(v * e2.x)),
@@ -735,10 +736,12 @@ __device__ float3 shadow_origin(float3 a, float3 e1, float3 e2, float u, float v
 // stored, or v1 - v0, v2 - v0 with the same float subtraction (watertight
 // scenes), so both give the reference's edge bits.
 template <int kGeo>
-__device__ __forceinline__ float3 shadow_origin_rec(float4 a, float4 b, float4 c, float u, float v, float3 light) {
+__device__ __forceinline__ float3 shadow_origin_rec(float4 a, float4 b, float4 c, float4 ng, float u, float v,
+                                                    float3 light) {
+  const float3 n = f3(ng.x, ng.y, ng.z);
   const float3 v0 = f3(a.x, a.y, a.z), p = f3(a.w, b.x, b.y), q = f3(b.z, b.w, c.x);
-  if constexpr (!(kGeo & kGeoWatertight)) return shadow_origin(v0, p, q, u, v, light);
-  else return shadow_origin(v0, p - v0, q - v0, u, v, light);
+  if constexpr (!(kGeo & kGeoWatertight)) return shadow_origin(v0, p, q, n, u, v, light);
+  else return shadow_origin(v0, p - v0, q - v0, n, u, v, light);
 }
 
 struct PixelSample {
@@ -746,6 +749,7 @@ struct PixelSample {
   float depth;
   bool valid;
   unsigned primary, shadow;
+  bool redo;  // a ray left its item's beam: the sample has to be taken without it (warp-uniform)
 };
 
 // What one pixel sample produces.
@@ -777,7 +781,7 @@ __device__ __forceinline__ float subray_y(const SceneView &S, int py_i, int sy) 
 template <int kMode, int kGeo = kGeoReference>
 __device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool active, const CellPose &pose,
                                            int *stack_code, float *stack_t, const SubraySample *subrays) {
-  PixelSample out{0.0, -1.0f, true, 0u, 0u};
+  PixelSample out{0.0, -1.0f, true, 0u, 0u, false};
   double depth = 0;
   int valid_depth = 0;
   const float3 light = f3(pose.lx, pose.ly, pose.lz);
@@ -813,7 +817,7 @@ __device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool a
           if (lit) {
             const float4 *r = tri_record<kGeo>(S, hit.tri, 2);
             const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-            sorigin = shadow_origin_rec<kGeo>(a, b, c, hit.u, hit.v, light);
+            sorigin = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit.u, hit.v, light);
             if (S.has_albedo) {
               albedo = s0.w * w + s1.w * hit.u + s2.w * hit.v;
               r0 = hfunc_r0(albedo);
@@ -1153,8 +1157,8 @@ __device__ void trace_shadow_packet_r(const SceneView &S, const float3 (&o)[R], 
 // that the ray's slab test fails (the beam's interval bounds are extremes of the same
 // rounded operations).  What the beam assumes of a ray -- its direction, or
 // its shadow origin, inside the beam's ranges -- is checked for every ray, and
-// a packet with a ray outside takes the general walk.  An item whose beam has no
-// one-signed direction, or reaches more leaves than a list holds, has no lists
+// a sample with a ray outside is taken again by walks from the root.  An item
+// whose beam reaches more leaves than a list holds has no lists
 // and walks the tree for every packet, two sub-rays per lane.
 constexpr int kBeamLeaves = 32;  // one per lane
 struct Beam {                    // shared memory, one per warp
@@ -1193,17 +1197,61 @@ __device__ __forceinline__ Packet range_packet(float3 olo, float3 ohi, float3 il
   return P;
 }
 // The primary beam's bundle: 1/d of directions of one sign decreases with d, so the ends of the inverse's range are
-// the inverses of the ends, rounded outward by more than rcp_rn's last bit.  A range that holds zero on an axis (or comes so near it that
-// inverse_direction could clamp) has no such bundle.
+// the inverses of the ends, rounded outward by more than rcp_rn's last bit.  On an axis whose range holds zero (or
+// comes so near it that inverse_direction could clamp: the rows and columns of pixels that look along a coordinate
+// plane) the inverse has no range, and leaf boxes are tested there by position: where the rays are on that
+// axis between the entry and the exit that the other axes give.
 __device__ __forceinline__ float rcp_low(float d) { const float y = 1.0f / d; return y - 2.4e-7f * fabsf(y); }
 __device__ __forceinline__ float rcp_high(float d) { const float y = 1.0f / d; return y + 2.4e-7f * fabsf(y); }
 __device__ __forceinline__ bool one_sign(float lo, float hi) { return lo > 1e-18f || hi < -1e-18f; }
-__device__ __forceinline__ Packet primary_packet(const Beam &B) {
+struct PrimaryBundle {
+  Packet P;
+  bool tx, ty, tz;  // axes whose inverse direction keeps one sign
+};
+__device__ __forceinline__ PrimaryBundle primary_bundle(const Beam &B) {
   const float3 dlo = B.dlo, dhi = B.dhi;
-  Packet P = range_packet(B.olo, B.ohi, f3(rcp_low(dhi.x), rcp_low(dhi.y), rcp_low(dhi.z)),
-                          f3(rcp_high(dlo.x), rcp_high(dlo.y), rcp_high(dlo.z)));
-  P.coherent = one_sign(dlo.x, dhi.x) && one_sign(dlo.y, dhi.y) && one_sign(dlo.z, dhi.z);
-  return P;
+  PrimaryBundle b;
+  b.P = range_packet(B.olo, B.ohi, f3(rcp_low(dhi.x), rcp_low(dhi.y), rcp_low(dhi.z)),
+                     f3(rcp_high(dlo.x), rcp_high(dlo.y), rcp_high(dlo.z)));
+  b.tx = one_sign(dlo.x, dhi.x);
+  b.ty = one_sign(dlo.y, dhi.y);
+  b.tz = one_sign(dlo.z, dhi.z);
+  b.P.coherent = b.tx || b.ty || b.tz;
+  return b;
+}
+// Whether rays between entry and exit distance can be inside [lo, hi] on an axis; the margin covers the roundings of a
+// ray's own slab test (three of them on a distance, one on a coordinate).
+__device__ __forceinline__ bool passes(float lo, float hi, float olo, float ohi, float dlo, float dhi, float entry,
+                                       float exit) {
+  const float a = olo + fminf(entry * dlo, exit * dlo), b = ohi + fmaxf(entry * dhi, exit * dhi);
+  const float m = 2e-6f * (fmaxf(fabsf(a), fabsf(b)) + fmaxf(fabsf(olo), fabsf(ohi)) + fmaxf(fabsf(lo), fabsf(hi)));
+  return b + m >= lo && a - m <= hi;
+}
+// The beam's entry and exit distance at a box, and whether one of its rays may enter it.
+__device__ __forceinline__ bool bundle_slab(const ChildRec &c, const PrimaryBundle &b, const Beam &B, float &entry,
+                                            float &exit) {
+  const Packet &P = b.P;
+  float L, U;
+  entry = kRayEps;
+  exit = 1e30f;
+  if (b.tx) {
+    axis_bounds_fixed(c.lo.x, c.hi.x, P.nx, P.o_near.x, P.o_far.x, P.ilo.x, P.ihi.x, L, U);
+    entry = fmaxf(entry, L);
+    exit = fminf(exit, U);
+  }
+  if (b.ty) {
+    axis_bounds_fixed(c.lo.y, c.hi.y, P.ny, P.o_near.y, P.o_far.y, P.ilo.y, P.ihi.y, L, U);
+    entry = fmaxf(entry, L);
+    exit = fminf(exit, U);
+  }
+  if (b.tz) {
+    axis_bounds_fixed(c.lo.z, c.hi.z, P.nz, P.o_near.z, P.o_far.z, P.ilo.z, P.ihi.z, L, U);
+    entry = fmaxf(entry, L);
+    exit = fminf(exit, U);
+  }
+  return exit >= entry && (b.tx || passes(c.lo.x, c.hi.x, P.olo.x, P.ohi.x, B.dlo.x, B.dhi.x, entry, exit)) &&
+         (b.ty || passes(c.lo.y, c.hi.y, P.olo.y, P.ohi.y, B.dlo.y, B.dhi.y, entry, exit)) &&
+         (b.tz || passes(c.lo.z, c.hi.z, P.olo.z, P.ohi.z, B.dlo.z, B.dhi.z, entry, exit));
 }
 __device__ __forceinline__ ChildRec list_leaf(const float4 (*list)[2], int i) {
   const float4 a = list[i][0], b = list[i][1];
@@ -1211,9 +1259,10 @@ __device__ __forceinline__ ChildRec list_leaf(const float4 (*list)[2], int i) {
 }
 
 // The leaves a bundle may reach, in no order: up to four nodes at a time, one
-// child per lane.  Returns their number, kNoList when they are more than the list holds.
-template <int kGeo>
-__device__ __forceinline__ int collect_leaves(const SceneView &S, const Packet &P, int *stack, float4 (*list)[2]) {
+// child per lane (reaches: whether the bundle may enter its box).  Returns their
+// number, kNoList when they are more than the list holds.
+template <int kGeo, class Test>
+__device__ __forceinline__ int collect_leaves(const SceneView &S, const Test &reaches, int *stack, float4 (*list)[2]) {
   const int lane = threadIdx.x & 31, group = lane >> 3, slot = lane & 7;
   const unsigned below = (1u << lane) - 1u;
   int sp = 1, n = 0;
@@ -1226,9 +1275,8 @@ __device__ __forceinline__ int collect_leaves(const SceneView &S, const Packet &
     ChildRec c{};
     bool hit = false;
     if (node >= 0) {
-      float key;
       c = load_child<kGeo>(S, node, slot);
-      hit = c.count >= 0 && packet_slab(c, P, kRayEps, 1e30f, key);
+      hit = c.count >= 0 && reaches(c);
     }
     const unsigned leaves = __ballot_sync(kFull, hit && c.count > 0);
     const unsigned inner = __ballot_sync(kFull, hit && c.count == 0);
@@ -1256,9 +1304,10 @@ __device__ __forceinline__ int collect_leaves(const SceneView &S, const Packet &
 // The primary list: the beam's leaves by entry distance (ties in walk order).
 template <int kGeo>
 __device__ __forceinline__ int build_primary_list(const SceneView &S, Beam &B, int *stack) {
-  const Packet P = primary_packet(B);
-  if (!P.coherent) return kNoList;
-  const int n = collect_leaves<kGeo>(S, P, stack, B.leaf);
+  const PrimaryBundle bundle = primary_bundle(B);
+  if (!bundle.P.coherent) return kNoList;
+  const int n = collect_leaves<kGeo>(
+      S, [&](const ChildRec &c) { float entry, exit; return bundle_slab(c, bundle, B, entry, exit); }, stack, B.leaf);
   if (n > 1) {
     const int lane = threadIdx.x & 31;
     float4 a, b;
@@ -1266,7 +1315,8 @@ __device__ __forceinline__ int build_primary_list(const SceneView &S, Beam &B, i
     if (lane < n) {
       a = B.leaf[lane][0];
       b = B.leaf[lane][1];
-      packet_slab(list_leaf(B.leaf, lane), P, kRayEps, 1e30f, key);
+      float exit;
+      bundle_slab(list_leaf(B.leaf, lane), bundle, B, key, exit);
     }
     int rank = 0;
     for (int j = 0; j < n; ++j) {
@@ -1290,21 +1340,13 @@ __device__ __forceinline__ int build_primary_list(const SceneView &S, Beam &B, i
 template <int kGeo>
 __device__ __forceinline__ int build_shadow_list(const SceneView &S, Beam &B, int n_leaf, int *stack) {
   const int lane = threadIdx.x & 31;
-  const Packet P = primary_packet(B);
+  const PrimaryBundle bundle = primary_bundle(B);
   float3 lo = f3(kInf(), kInf(), kInf()), hi = -lo;
   if (lane < n_leaf) {
     const ChildRec c = list_leaf(B.leaf, lane);
-    float near, t0, t1;
-    packet_slab(c, P, kRayEps, 1e30f, near);
-    float L, U, far = 1e30f;
-    axis_bounds_fixed(c.lo.x, c.hi.x, P.nx, P.o_near.x, P.o_far.x, P.ilo.x, P.ihi.x, L, U);
-    far = fminf(far, U);
-    axis_bounds_fixed(c.lo.y, c.hi.y, P.ny, P.o_near.y, P.o_far.y, P.ilo.y, P.ihi.y, L, U);
-    far = fminf(far, U);
-    axis_bounds_fixed(c.lo.z, c.hi.z, P.nz, P.o_near.z, P.o_far.z, P.ilo.z, P.ihi.z, L, U);
-    far = fminf(far, U);
-    t0 = near;
-    t1 = fmaxf(far, near);
+    float t0, t1;
+    bundle_slab(c, bundle, B, t0, t1);
+    t1 = fmaxf(t0, t1);
     const float3 dlo = B.dlo, dhi = B.dhi;
     lo = max3(c.lo, B.olo + min3(t0 * dlo, t1 * dlo));
     hi = min3(c.hi, B.ohi + max3(t0 * dhi, t1 * dhi));
@@ -1322,7 +1364,8 @@ __device__ __forceinline__ int build_shadow_list(const SceneView &S, Beam &B, in
   __syncwarp();
   const Packet L = range_packet(lo, hi, B.llo, B.lhi);
   if (!L.coherent) return kNoList;
-  return collect_leaves<kGeo>(S, L, stack, B.shadow);
+  return collect_leaves<kGeo>(
+      S, [&](const ChildRec &c) { float key; return packet_slab(c, L, kRayEps, 1e30f, key); }, stack, B.shadow);
 }
 
 // A longer list is first cut to the leaves the packet's own interval bundle may reach, one leaf per lane: the bundle's
@@ -1447,7 +1490,8 @@ __device__ __forceinline__ void nearest_in_list(const SceneView &S, const Beam &
   if (n > kListFilter) {
     float3 ilo, ihi;
     packet_range<R>(idir, live, ilo, ihi);
-    left = list_mask(B.leaf, n, range_packet(B.olo, B.ohi, ilo, ihi));  // one-signed, as the beam
+    const Packet P = range_packet(B.olo, B.ohi, ilo, ihi);
+    if (P.coherent) left = list_mask(B.leaf, n, P);
   }
   for (; left; left &= left - 1u) {
     const ChildRec c = list_leaf(B.leaf, __ffs(left) - 1);
@@ -1549,12 +1593,14 @@ __device__ __forceinline__ unsigned shadow_in_list(const SceneView &S, const Bea
 // sample_pixel_packet with R neighbouring sub-rays per lane (ss^2 a multiple
 // of R).  The per-ray work, the order of the FP64 radiance and depth sums and
 // the ray counts are those of the one-ray loop.
-// kBeam: the item has lists, and the packet's leaves come from them where its rays are inside the beam.
+// kBeam: the item has lists, and the packets' leaves come from them; a ray
+// outside the beam ends the sample (redo).  The loop then holds no call, whose
+// registers would be spilled around it.
 template <int kMode, int R, int kGeo, bool kBeam>
 __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool active,
                                                           const CellPose &pose, int *stack_code, float *stack_t,
                                                           const SubraySample *subrays, Beam &B, BeamLists &lists) {
-  PixelSample out{0.0, -1.0f, true, 0u, 0u};
+  PixelSample out{0.0, -1.0f, true, 0u, 0u, false};
   double depth = 0;
   int valid_depth = 0;
   const float3 light = f3(pose.lx, pose.ly, pose.lz);
@@ -1590,19 +1636,12 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
 #pragma unroll
       for (int r = 0; r < R; ++r) org[r] = origin;
       trace_nearest_packet_r<R, kGeo>(S, org, ray, live, stack_code, stack_t, hit);
-    } else if (__all_sync(kFull, inside)) {
-      nearest_in_list<R, kGeo>(S, B, lists.leaves, origin, ray, live, hit);
     } else {
-      PacketRays<R> in;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        in.o[r] = origin;
-        in.d[r] = ray[r];
-        in.live[r] = live[r];
+      if (!__all_sync(kFull, inside)) {
+        out.redo = true;
+        return out;
       }
-      const PacketHits<R> got = nearest_general<R, kGeo>(S, in, stack_code, stack_t);
-#pragma unroll
-      for (int r = 0; r < R; ++r) hit[r] = got.h[r];
+      nearest_in_list<R, kGeo>(S, B, lists.leaves, origin, ray, live, hit);
     }
     bool lit[R];
     float3 normal[R], sorigin[R];
@@ -1634,7 +1673,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
           if (lit[r]) {
             const float4 *t4 = tri_record<kGeo>(S, hit[r].tri, 2);
             const float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
-            sorigin[r] = shadow_origin_rec<kGeo>(a, b, c, hit[r].u, hit[r].v, light);
+            sorigin[r] = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit[r].u, hit[r].v, light);
             if (S.has_albedo) {
               albedo[r] = s0.w * w + s1.w * hit[r].u + s2.w * hit[r].v;
               r0[r] = hfunc_r0(albedo[r]);
@@ -1659,18 +1698,12 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
           trace_shadow_packet_r<R, kGeo>(S, sorigin, light, sdir, lit, self, stack_code, stack_t, occ);
 #pragma unroll
           for (int r = 0; r < R; ++r) occluded |= occ[r] ? 1u << r : 0u;
-        } else if (__all_sync(kFull, near)) {
-          occluded = shadow_in_list<R, kGeo>(S, B, lists.shadow, sorigin, light, sdir, lit, self, lists.first);
         } else {
-          ShadowRays<R> in;
-          in.light = light;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            in.o[r] = sorigin[r];
-            in.self[r] = self[r];
-            in.live[r] = lit[r];
+          if (!__all_sync(kFull, near)) {
+            out.redo = true;
+            return out;
           }
-          occluded = shadow_general<R, kGeo>(S, in, stack_code, stack_t);
+          occluded = shadow_in_list<R, kGeo>(S, B, lists.shadow, sorigin, light, sdir, lit, self, lists.first);
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -1734,7 +1767,7 @@ __device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, fl
     if (out.lit) {
       const float4 *r = tri_record<kGeo>(S, hit[0].tri, 2);
       const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-      sorigin[0] = shadow_origin_rec<kGeo>(a, b, c, hit[0].u, hit[0].v, light);
+      sorigin[0] = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit[0].u, hit[0].v, light);
       if (S.has_albedo) {
         albedo = s0.w * w + s1.w * hit[0].u + s2.w * hit[0].v;
         r0 = hfunc_r0(albedo);

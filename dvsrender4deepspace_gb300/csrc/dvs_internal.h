@@ -70,12 +70,13 @@ static_assert(sizeof(TriRecord) == 48, "TriRecord layout");
 
 // Shading record in leaf order, 64 bytes: vertex normals and per-vertex
 // material albedo (already passed through the fallback rule of
-// include/dvs/device_optics.cuh:30-33).
+// include/dvs/device_optics.cuh:30-33), and the triangle's own unit normal,
+// cross(e1, e2) normalized, which shadow_origin would form for every lit ray.
 struct alignas(16) ShadeRecord {
   float n0[3], a0;
   float n1[3], a1;
   float n2[3], a2;
-  float pad[4];
+  float ng[3], pad;
 };
 static_assert(sizeof(ShadeRecord) == 64, "ShadeRecord layout");
 

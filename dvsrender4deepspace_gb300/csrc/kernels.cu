@@ -332,7 +332,9 @@ PoseShape pose_item_shape(int n_pix, int nc, int ss2, bool scattered) {
   const int limit = scattered ? 1 : most < 32 ? most : 32;
   while (2 * s.pixels <= limit && items(2 * s.pixels) >= 2 * kResidentWarps && s.pixels * runs < 64 * per_packet)
     s.pixels *= 2;
-  s.beam = (s.pixels + per_packet - 1) / per_packet * runs >= 8;
+  // one walk for the item pays from 8 packets on, or where the item is itself one narrow packet (the walk takes four
+  // nodes at a time and sorts once: 160x120 frames with 4 sub-rays 0.29 -> 0.20 ms); 4 packets over 32 pixels lose 8 %
+  s.beam = s.pixels <= 4 || (s.pixels + per_packet - 1) / per_packet * runs >= 8;
   return s;
 }
 template <int kGeo>

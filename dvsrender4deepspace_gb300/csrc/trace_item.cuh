@@ -38,7 +38,7 @@ __device__ __forceinline__ void store_radiance(const SceneView &S, double *chunk
 #define DVS_TRACE_PAIR_MIN_BLOCKS 4
 #endif
 #ifndef DVS_TRACE_BEAM_MIN_BLOCKS
-#define DVS_TRACE_BEAM_MIN_BLOCKS 4
+#define DVS_TRACE_BEAM_MIN_BLOCKS 5
 #endif
 #ifndef DVS_TRACE_QUAD_MIN_BLOCKS
 #define DVS_TRACE_QUAD_MIN_BLOCKS 3
@@ -81,14 +81,16 @@ __device__ __forceinline__ BeamLists begin_beam(const SceneView &S, int n_pix, c
   return close_beam<kGeo>(S, olo, ohi, dlo, dhi, llo, lhi, 0.0f, B, stack);
 }
 
-// The packets of an item without lists, out of line (few items of a launch with beams): two sub-rays per lane where
-// their count is even, as a launch without beams.
+// A sample of an item without lists (under one in a hundred on the terrains measured), or one whose rays left the
+// beam, out of line: two sub-rays per lane where their count is even, as a launch without beams.
+// (The pose by its address in global memory: a reference to the caller's would hold it in local memory.)
 template <int kMode, int kGeo>
 __device__ __noinline__ PixelSample sample_without_beam(const SceneView &S, int pixel, bool active,
-                                                        const CellPose &pose, TraceShared &sh,
+                                                        const CellPose *pose_at, TraceShared &sh,
                                                         const SubraySample *subrays) {
   BeamLists none{kNoList, kNoList, 0};
   Beam &unused = *reinterpret_cast<Beam *>(&sh);  // not touched without lists
+  const CellPose pose = *pose_at;
   if (S.samples % 2 == 0)
     return sample_pixel_group<kMode, 2, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
   return sample_pixel_group<kMode, 1, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
@@ -141,12 +143,15 @@ __device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, 
     for (int g = g0; g < g1; ++g) {
       const int cell = g * cw + (lane & (cw - 1));
       const bool active = rank < n_pix && cell < nc;
-      const CellPose pose = poses[c0 + (active ? cell : 0)];
+      const CellPose *at = poses + c0 + (active ? cell : 0);
+      const CellPose pose = *at;
       PixelSample s;
-      if (kBeam && lists.shadow < 0)
-        s = sample_without_beam<kMode, kGeo>(S, pixel, active, pose, sh, mine);
-      else
+      bool by_list = !kBeam || lists.shadow >= 0;
+      if (by_list) {
         s = sample_pixel_group<kMode, kRays, kGeo, kBeam>(S, pixel, active, pose, sh.code, sh.t, mine, beam, lists);
+        by_list = !s.redo;
+      }
+      if (kBeam && !by_list) s = sample_without_beam<kMode, kGeo>(S, pixel, active, at, sh, mine);
       if (active) {
         const size_t o = (size_t)cell * n_pix + rank;
         store_radiance(S, radiance, o, s.valid ? s.radiance : __longlong_as_double(0x7ff8000000000000ll));
