@@ -237,7 +237,7 @@ class EventSensor:
         return out[: got.value].copy()
 
     def drain(self):
-        cap = 1 << 20
+        cap = 4096  # a drained queue is mostly short; the buffers that follow a full one are large
         chunks = []
         while True:
             out = np.zeros(cap, EVENT_DTYPE)
@@ -246,6 +246,7 @@ class EventSensor:
             chunks.append(out[: got.value].copy())
             if got.value < cap:
                 break
+            cap = 1 << 20
         return np.concatenate(chunks)
 
     def stats(self):
