@@ -176,9 +176,7 @@ struct DeviceReadout {
     host = host_status;
     *host = HostStatus{};
     unknown_grid = blocks_for(batch / 16);
-    cudaError_t e = prepare_readout();
-    if (e == cudaSuccess) e = cudaMemsetAsync(words, 0, word_bytes, st);  // positions, counters, availability, words
-    return e;
+    return cudaMemsetAsync(words, 0, word_bytes, st);  // positions, counters, availability, words
   }
   size_t place(char *b, size_t ring, size_t max_batch, void **words, size_t *word_bytes) {
     const int max_grid = 608;  // 4 blocks per SM of a GB300

@@ -115,8 +115,7 @@ struct ReadoutFifo {
 // FIFO at time *now (device memory, so a captured graph reads each step's);
 // the released events land in f.out (*f.out_count of them).  grid: blocks
 // of the sort and scan kernels (the sort's hist holds 256 x grid); 1: the whole
-// submit in one kernel of one cluster.  prepare_readout: once per device before it.
-cudaError_t prepare_readout();
+// submit in one kernel of one cluster.
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st);
 cudaError_t launch_readout_drain(ReadoutFifo f, int grid, cudaStream_t st);

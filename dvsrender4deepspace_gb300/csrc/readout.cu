@@ -673,86 +673,107 @@ __global__ void ro_fifo_advance_kernel(ReadoutFifo f) { ro_fifo_advance(f); }
 // ---- a batch in one cluster ------------------------------------------------------------
 // Most batches hold few events, and the phases' kernels then cost their launches:
 // 44 of them, 0.17-0.2 ms a batch.  One launch of one cluster runs the whole
-// submit instead.  Up to kBlockEvents events are sorted by its first block in shared memory, by a bitonic
-// network on (t, (y, x), arrival) -- the arrival index makes the order the
-// stable one -- and left in the key buffers as the radix passes would leave
-// them; more events (a burst after small batches; the next submit is sized by
-// it) go through the radix passes with the cluster's blocks as the team and its hardware barrier between the phases.
-// (One block as the team took 5.3 ms for a burst of 64,500 events.)
+// submit instead, by the number of events:
+//   * up to kBlockEvents: its first block alone, sorting in shared memory by a bitonic
+//     network on (t, (y, x), arrival) -- the arrival index makes the order the stable one;
+//   * up to kClusterBlocks x kBlockEvents: every block sorts its share that way, then
+//     places each of its events by its rank in the other blocks' sorted shares
+//     (3000 events: 119 us in one block's network of 4096);
+//   * more (a burst after small batches; the next submit is sized by it): the radix
+//     passes with the cluster's blocks as the team (64,500 events: 5.3 ms with one block).
+// The first two leave the keys as radix passes would.  The blocks meet at the
+// cluster's hardware barrier and hand over through global memory.
 constexpr int kClusterBlocks = 8;  // the portable cluster size
+constexpr int kBlockEvents = 512;
 __device__ __forceinline__ void cluster_barrier() {
-  __threadfence();  // the phases hand over through global memory
+  __threadfence();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-constexpr int kBlockEvents = 4096;
-struct BlockSort {
-  unsigned long long kt[kBlockEvents];
-  unsigned kyx[kBlockEvents], idx[kBlockEvents];
+struct SortKey {
+  unsigned long long kt;
+  unsigned kyx, idx;
 };
-__device__ __forceinline__ void block_sort(const DevEvent *events, int n, BlockSort &b, const ReadoutSort &s) {
-  const int t = threadIdx.x;
+__device__ __forceinline__ bool before(const SortKey &a, const SortKey &b) {
+  return a.kt != b.kt ? a.kt < b.kt : a.kyx != b.kyx ? a.kyx < b.kyx : a.idx < b.idx;
+}
+// Sorts events [begin, end), at most kBlockEvents, into b.
+__device__ __forceinline__ void block_sort(const DevEvent *events, int begin, int end, SortKey *b) {
+  const int t = threadIdx.x, n = end - begin;
   int m = 1;
   while (m < n) m <<= 1;
   for (int i = t; i < m; i += kSortThreads) {
-    unsigned long long kt = ~0ull;  // above every key of an event: its arrival index is larger too
-    unsigned kyx = kFull;
+    SortKey k{~0ull, kFull, (unsigned)(begin + i)};  // padding: after every event, its arrival index the larger one
     if (i < n) {
-      kt = time_key(events[i].t);
-      kyx = yx_key(events[i]);
+      k.kt = time_key(events[begin + i].t);
+      k.kyx = yx_key(events[begin + i]);
     }
-    b.kt[i] = kt;
-    b.kyx[i] = kyx;
-    b.idx[i] = (unsigned)i;
+    b[i] = k;
   }
   __syncthreads();
   for (int size = 2; size <= m; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
       for (int q = t; q < m / 2; q += kSortThreads) {
         const int i = 2 * q - (q & (stride - 1)), j = i + stride;
-        const unsigned long long ki = b.kt[i], kj = b.kt[j];
-        const unsigned yi = b.kyx[i], yj = b.kyx[j], ii = b.idx[i], ij = b.idx[j];
-        const bool after = ki != kj ? ki > kj : yi != yj ? yi > yj : ii > ij;
-        if (after == ((i & size) == 0)) {
-          b.kt[i] = kj;
-          b.kt[j] = ki;
-          b.kyx[i] = yj;
-          b.kyx[j] = yi;
-          b.idx[i] = ij;
-          b.idx[j] = ii;
+        const SortKey x = b[i], y = b[j];
+        if (before(y, x) == ((i & size) == 0)) {
+          b[i] = y;
+          b[j] = x;
         }
       }
       __syncthreads();
     }
-  // nothing varies that a pass would still have to order: the keys stay in buffer 0, unpacked
-  for (int i = t; i < n; i += kSortThreads) {
-    s.kt[0][i] = b.kt[i];
-    s.idx[0][i] = b.idx[i];
-  }
-  __syncthreads();
 }
 __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kSortThreads)
     ro_cluster_kernel(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f, const double *now) {
-  extern __shared__ __align__(16) unsigned char ro_shared[];
+  __shared__ SortKey sorted[kBlockEvents];
   const int n = *count;
-  const bool small = n <= kBlockEvents;  // the same in every block
+  const bool alone = n <= kBlockEvents, network = n <= kClusterBlocks * kBlockEvents;  // the same in every block
   const bool first = blockIdx.x == 0;
-  if (small && !first) return;
-  const Team team = small ? Team{0, 1} : Team{(int)blockIdx.x, kClusterBlocks};
-  const auto barrier = [small] {
-    if (small) __syncthreads();
+  if (alone && !first) return;
+  const Team team = alone ? Team{0, 1} : Team{(int)blockIdx.x, kClusterBlocks};
+  const auto barrier = [alone] {
+    if (alone) __syncthreads();
     else cluster_barrier();
   };
   if (first && threadIdx.x == 0) {
-    // small: the layout of an unpacked key whose passes leave it in buffer 0
-    s.varying[0] = small ? 0x8000000000000000ull : 0ull;
-    s.varying[1] = small ? 1ull : 0ull;
+    // network: the layout of an unpacked key whose passes leave it in buffer 0
+    s.varying[0] = network ? 0x8000000000000000ull : 0ull;
+    s.varying[1] = network ? 1ull : 0ull;
     s.varying[2] = 0ull;
     *f.overflow = 0;
     *f.peak_batch = 0;
   }
   barrier();
-  if (small) {
-    block_sort(events, n, *reinterpret_cast<BlockSort *>(ro_shared), s);
+  if (network) {
+    int begin, end;
+    tile_of(n, team, begin, end);
+    block_sort(events, begin, end, sorted);
+    if (!alone) {
+      for (int i = threadIdx.x; i < end - begin; i += kSortThreads) {
+        s.kt[1][begin + i] = sorted[i].kt;
+        s.kyx[1][begin + i] = sorted[i].kyx;
+        s.idx[1][begin + i] = sorted[i].idx;
+      }
+      barrier();
+    }
+    for (int i = threadIdx.x; i < end - begin; i += kSortThreads) {
+      const SortKey k = sorted[i];
+      int at = i;
+      for (int o = 0; o < team.blocks; ++o) {
+        if (o == team.block) continue;
+        int lo, hi;
+        tile_of(n, Team{o, team.blocks}, lo, hi);
+        const int base = lo;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (before(SortKey{s.kt[1][mid], s.kyx[1][mid], s.idx[1][mid]}, k)) lo = mid + 1; else hi = mid;
+        }
+        at += lo - base;
+      }
+      s.kt[0][at] = k.kt;
+      s.idx[0][at] = k.idx;
+    }
+    barrier();
   } else {
     ro_keys(team, events, count, s);
     barrier();
@@ -807,15 +828,11 @@ __global__ void ro_drain_commit_kernel(ReadoutFifo f) {
 
 int readout_submit_launches(bool delayed, int grid) { return grid <= 1 ? 1 : 2 + kPasses * 3 + (delayed ? 3 : 0) + 3; }
 
-cudaError_t prepare_readout() {
-  return cudaFuncSetAttribute(ro_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockSort));
-}
-
 cudaError_t launch_readout_submit(const DevEvent *events, const int32_t *count, ReadoutSort s, ReadoutFifo f,
                                   const double *now, int grid, cudaStream_t st) {
   if (grid < 1 || grid > kScanThreads) return cudaErrorInvalidValue;
   if (grid == 1) {
-    ro_cluster_kernel<<<kClusterBlocks, kSortThreads, sizeof(BlockSort), st>>>(events, count, s, f, now);
+    ro_cluster_kernel<<<kClusterBlocks, kSortThreads, 0, st>>>(events, count, s, f, now);
     return cudaGetLastError();
   }
   cudaError_t e = cudaMemsetAsync(s.varying, 0, 3 * sizeof(unsigned long long), st);

@@ -1,5 +1,5 @@
-"""Small batches through the one-block readout against the host FIFO, at the
-sizes where its network, its padding and its capacity of 4096 events end, with
+"""Small batches through the one-cluster readout against the host FIFO, at the
+sizes where one block (512), the cluster's shares (8 x 512) and their padding end, with
 ties in t that (y, x) decide and events equal in all three, whose arrival order
 stays.  Order, fields, drops and peak are exact; delivery times are the same
 FP64 sums grouped as a scan (1 ns, as in test_gpu_readout.py).
@@ -15,7 +15,7 @@ from tests.test_oracle_golden import POSE
 
 pytestmark = pytest.mark.gpu
 
-SIZES = (1, 0, 2, 3, 31, 255, 256, 257, 1000, 2048, 4095, 4096, 4097, 5, 8191, 300)
+SIZES = (1, 0, 2, 3, 31, 255, 256, 257, 511, 512, 513, 514, 1000, 2048, 4095, 4096, 4097, 5, 8191, 300)
 
 
 @pytest.mark.parametrize("bandwidth,latency,capacity", [(0.0, 0.0, 1000), (5e6, 18e-9, 1_000_000), (2e6, 1e-6, 500)])
@@ -37,7 +37,7 @@ def test_block_readout_equals_the_host_fifo(bandwidth, latency, capacity, window
 
 
 def test_a_burst_after_quiet_batches():
-    """The block sized by a quiet batch takes the burst that follows it through the radix passes."""
+    """The cluster sized by a quiet batch takes the burst that follows it through the radix passes."""
     scene, phys = plane_sensor(readout_bandwidth=2e7, readout_latency=1e-6, readout_queue_capacity=500_000,
                                threshold_pos=0.05, threshold_neg=0.05)
     start, end = dict(POSE, intensity_rate=8e6), dict(POSE, intensity_rate=-8e6)
