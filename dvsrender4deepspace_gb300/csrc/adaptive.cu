@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, 4)
     if (!isfinite(initial[j])) bad = true;
   }
   OpticalKnot *out = knots + (size_t)rank * capacity;
-  const double v0 = st.receptor_log[rank];
+  const double v0 = st.receptor_log[rank], x0 = exp(v0);
   const double budget = 1e-3 * fmin(st.threshold_pos[rank], st.threshold_neg[rank]);  // kOpticalVoltageThresholdFraction
   if (lane == 0) out[0] = {0, initial[0]};
   // lane i: pending segment i
@@ -124,11 +124,13 @@ __global__ void __launch_bounds__(128, 4)
     if (lane < pending && verdict == kUndecided) {
       const double actual = middle * photo.electrons_per_radiance + photo.dark_electrons;
       const double estimate = (left + right) * .5 * photo.electrons_per_radiance + photo.dark_electrons;
-      const double residual = fabs(log(fmax(1e-30, actual) / fmax(1e-30, estimate)));
       const double leaf_duration = (b - a) * (end - start);
-      const double voltage_error = fabs(receptor_log_at(v0, actual, leaf_duration, charge) -
-                                        receptor_log_at(v0, estimate, leaf_duration, charge));
-      if (voltage_error <= budget && (residual <= tolerance || fmax(actual, estimate) * leaf_duration < 1.0))
+      const double voltage_error = fabs(receptor_log_from(v0, x0, actual, leaf_duration, charge) -
+                                        receptor_log_from(v0, x0, estimate, leaf_duration, charge));
+      bool smooth = voltage_error <= budget;
+      if (smooth && !(fmax(actual, estimate) * leaf_duration < 1.0))
+        smooth = fabs(log(fmax(1e-30, actual) / fmax(1e-30, estimate))) <= tolerance;
+      if (smooth)
         verdict = kSmooth;
       else if ((b - a) * (end - start) <= photo.integration_step || behind + 2 > kRefineStack)
         verdict = kExact;  // unresolved at the electrical sampling scale: exact tracing
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(128) integrate_knots_kernel(int n, const Cell 
     }
     double light = from + slope * (fraction - left);
     if (exact_index < n_exact && my_exact[exact_index] == c) light = my_exact_rad[exact_index++];
-    double rate = fmax(0.0, light) * photo.electrons_per_radiance + photo.dark_electrons;
+    double rate = (positive(light) ? light : 0.0) * photo.electrons_per_radiance + photo.dark_electrons;
     if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
     const int emitted = circuit_cell(run, p, rate, t0, t1, my_t + count, my_p + count, max_events - count, rng);
     if (emitted == -1) { failed = kErrCapacity; break; }

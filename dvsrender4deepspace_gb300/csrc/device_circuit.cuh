@@ -9,13 +9,16 @@
 namespace dvsgb {
 namespace {
 // ---- pixel circuit (include/dvs/pixel_model.hpp:18-102), FP64 ------------------------
-__device__ __forceinline__ double receptor_log_at(double u, double rate, double dt, double charge) {
+// receptor_log_at given x = exp(u).
+__device__ __forceinline__ double receptor_log_from(double u, double x, double rate, double dt, double charge) {
   if (dt <= 0) return u;
   rate = fmax(0.0, rate);
-  double x = exp(u);
   if (rate == 0) return u - log1p(x * dt / charge);
   double a = exp(-rate * dt / charge), b = -expm1(-rate * dt / charge);
   return -log(a / x + b / rate);
+}
+__device__ __forceinline__ double receptor_log_at(double u, double rate, double dt, double charge) {
+  return dt <= 0 ? u : receptor_log_from(u, exp(u), rate, dt, charge);
 }
 
 struct PixelRegs {
@@ -141,19 +144,27 @@ __device__ __forceinline__ double one_minus_exp_small(double k) {
   s = fma(-k, s, 1.0);
   return k * s;
 }
-// The receptor after dt at a constant rate.
+// Signs and orders of doubles from their bits: in the integer units, not on the FP64 pipe.
+__device__ __forceinline__ bool positive(double v) { return __double_as_longlong(v) > 0; }
+__device__ __forceinline__ bool less_positive(double a, double b) {  // b > 0; a zero or negative a is less
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+// The receptor after dt at a constant rate.  Without photons it discharges, x / (1 + x dt / charge): the lanes of a dim
+// warp draw both, so the two cases share the division.
 __device__ __forceinline__ double receptor_step(double x, double rate, double dt, double inv_charge) {
   const double g = dt * inv_charge, k = rate * g;
-  if (!(k > 0)) return x / fma(x, g, 1.0);  // no photons: the receptor discharges
   double a, b;
-  if (k < 0.35) {
+  if (less_positive(k, 0.35)) {
     b = one_minus_exp_small(k);
     a = 1.0 - b;
   } else {
     a = exp(-k);
     b = 1.0 - a;
   }
-  return x * rate / fma(b, x, a * rate);
+  const bool light = positive(k);
+  const double top = light ? rate : 1.0, rest = light ? a * rate : 1.0, share = light ? b : g;
+  return x * top / fma(share, x, rest);
 }
 
 struct CircuitRun {
@@ -162,17 +173,22 @@ struct CircuitRun {
   double inv_charge;
   bool direct;    // a leaking reference: advance_pixel for every cell
   bool follows;   // the reference is the receptor's log, not yet written down
+  bool settled;   // past the refractory deadline, nothing pending, the receptor between the bounds
 };
+__device__ __forceinline__ bool between(double low, double y, double high) {  // all positive
+  return less_positive(low, y) && less_positive(y, high);
+}
 __device__ __forceinline__ void circuit_bounds(CircuitRun &c) {
   c.high = exp(c.s.reference_log + c.s.threshold_pos);
   c.low = exp(c.s.reference_log - c.s.threshold_neg);
+  c.settled = false;
 }
 __device__ __forceinline__ CircuitRun circuit_begin(const CircuitState &st, int k, const PixelParams &p) {
   CircuitRun c;
   c.s = PixelRegs{st.receptor_log[k], st.reference_log[k], st.refractory_until[k], st.threshold_pos[k],
                   st.threshold_neg[k], st.reset_pending[k] != 0};
   c.direct = p.reference_leak > 0;
-  c.follows = false;
+  c.follows = c.settled = false;
   c.inv_charge = 1.0 / p.charge_scale;
   if (!c.direct) {
     c.x = st.receptor[k];
@@ -206,11 +222,14 @@ __device__ __noinline__ EventCell circuit_event_cell(EventCell e, PixelParams p,
 __device__ __forceinline__ int circuit_cell(CircuitRun &c, const PixelParams &p, double rate, double t0, double t1,
                                             double *out_t, int8_t *out_p, int capacity, curandStateXORWOW_t &rng) {
   if (!c.direct && t0 < t1) {
-    const bool refractory = t1 < c.s.refractory_until;
-    const bool settled = t0 >= c.s.refractory_until && !c.s.reset_pending && c.x < c.high && c.x > c.low;
-    if (refractory || settled) {
+    bool refractory = false;
+    if (!c.settled) {  // a quiet cell leaves the pixel settled: its deadline stays behind it
+      refractory = t1 < c.s.refractory_until;
+      c.settled = t0 >= c.s.refractory_until && !c.s.reset_pending && between(c.low, c.x, c.high);
+    }
+    if (refractory || c.settled) {
       const double y = receptor_step(c.x, rate, t1 - t0, c.inv_charge);
-      if (refractory || (y < c.high && y > c.low)) {
+      if (refractory || between(c.low, y, c.high)) {
         c.x = y;
         c.follows = refractory;
         return 0;
@@ -527,8 +546,9 @@ __device__ __forceinline__ curandStatePhilox4_32_10_t philox_at(unsigned seed, i
 // poisson_electrons (include/dvs/photon_noise.cuh:4-9): cuRAND draws in the
 // reference's order so seeded streams match a reference build on the same toolkit.
 __device__ __forceinline__ double poisson_electrons(curandStateXORWOW_t &rng, double lambda) {
-  if (lambda <= 0) return 0;
-  if (lambda > 1e6) return fmax(0.0, floor(lambda + sqrt(lambda) * curand_normal_double(&rng) + .5));
+  // comparisons of the bits (lambda is finite): integer units, not the FP64 pipe
+  if (__double_as_longlong(lambda) <= 0) return 0;
+  if (__double_as_longlong(lambda) > __double_as_longlong(1e6)) return fmax(0.0, floor(lambda + sqrt(lambda) * curand_normal_double(&rng) + .5));
   return curand_poisson(&rng, lambda);
 }
 

@@ -278,7 +278,7 @@ __device__ __forceinline__ void circuit_rank(int r, int n, const int32_t *rank_l
     for (int c = 0; c < nc; ++c) {
       const Cell cell = cells[c0 + c];
       const double rad = radiance[(size_t)c * n + r];
-      if (!isfinite(rad)) { failed = kErrOptical; break; }
+      if (!finite_bits(rad)) { failed = kErrOptical; break; }
       double rate = rad * photo.electrons_per_radiance + photo.dark_electrons;
       const double t0 = cell.t0, t1 = cell.t1;
       if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
