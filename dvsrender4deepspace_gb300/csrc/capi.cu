@@ -277,7 +277,9 @@ struct dvs_scene {
   double build_seconds = 0;
   double sah_node_visits = 0, sah_triangle_tests = 0;
   HapkeConst hc{};             // the material's constants (form_constants)
-  float coherent_span = 1.0f;  // 0.5 % of the scene's largest extent
+  // 1.5 % of the scene's largest extent (0.5 %: shadow packets of small frames, 8 pixels wide on the ground, were
+  // traced ray by ray: 640x480 frame 0.43 against 0.38 ms, 5-pose exposure 1.06 against 0.92; 5 %: jobs lose 2-5 %)
+  float coherent_span = 1.0f;
   // camera render buffers
   cudaStream_t stream = nullptr;
   double *cam_radiance = nullptr;
@@ -589,7 +591,7 @@ int dvs_scene_create(const float *vertices, const float *normals, const uint32_t
         lo[d] = std::min(lo[d], vertices[3 * i + d]);
         hi[d] = std::max(hi[d], vertices[3 * i + d]);
       }
-    s->coherent_span = 0.005f * std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1.0f});
+    s->coherent_span = 0.015f * std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1.0f});
   }
   cudaGetDevice(&s->device);
   const size_t off_nodes = 0;
