@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, 4)
     if (!isfinite(initial[j])) bad = true;
   }
   OpticalKnot *out = knots + (size_t)rank * capacity;
-  const double v0 = st.receptor_log[rank], x0 = exp(v0);
+  const double x0 = exp(st.receptor_log[rank]), inv_charge = 1.0 / charge;
   const double budget = 1e-3 * fmin(st.threshold_pos[rank], st.threshold_neg[rank]);  // kOpticalVoltageThresholdFraction
   if (lane == 0) out[0] = {0, initial[0]};
   // lane i: pending segment i
@@ -125,8 +125,9 @@ __global__ void __launch_bounds__(128, 4)
       const double actual = middle * photo.electrons_per_radiance + photo.dark_electrons;
       const double estimate = (left + right) * .5 * photo.electrons_per_radiance + photo.dark_electrons;
       const double leaf_duration = (b - a) * (end - start);
-      const double voltage_error = fabs(receptor_log_from(v0, x0, actual, leaf_duration, charge) -
-                                        receptor_log_from(v0, x0, estimate, leaf_duration, charge));
+      // |u(actual) - u(estimate)| from the receptors themselves: one log for both
+      const double voltage_error = fabs(log(receptor_step(x0, fmax(0.0, actual), leaf_duration, inv_charge) /
+                                            receptor_step(x0, fmax(0.0, estimate), leaf_duration, inv_charge)));
       bool smooth = voltage_error <= budget;
       if (smooth && !(fmax(actual, estimate) * leaf_duration < 1.0))
         smooth = fabs(log(fmax(1e-30, actual) / fmax(1e-30, estimate))) <= tolerance;

@@ -9,16 +9,13 @@
 namespace dvsgb {
 namespace {
 // ---- pixel circuit (include/dvs/pixel_model.hpp:18-102), FP64 ------------------------
-// receptor_log_at given x = exp(u).
-__device__ __forceinline__ double receptor_log_from(double u, double x, double rate, double dt, double charge) {
+__device__ __forceinline__ double receptor_log_at(double u, double rate, double dt, double charge) {
   if (dt <= 0) return u;
   rate = fmax(0.0, rate);
+  double x = exp(u);
   if (rate == 0) return u - log1p(x * dt / charge);
   double a = exp(-rate * dt / charge), b = -expm1(-rate * dt / charge);
   return -log(a / x + b / rate);
-}
-__device__ __forceinline__ double receptor_log_at(double u, double rate, double dt, double charge) {
-  return dt <= 0 ? u : receptor_log_from(u, exp(u), rate, dt, charge);
 }
 
 struct PixelRegs {
