@@ -303,7 +303,7 @@ __global__ void identify_exact_kernel(int n, const Cell *cells, int n_cells, dou
 // sample_exact_queries (optical_sampler.cu:132-138): one queued cell per lane,
 // grid-stride over the device-side queue length.
 template <int kGeo>
-__global__ void __launch_bounds__(128) sample_exact_kernel(SceneView S, const CellPose *poses,
+__global__ void __launch_bounds__(128) sample_exact_kernel(const __grid_constant__ SceneView S, const CellPose *poses,
                                                            const int32_t *exact_cells, const int32_t *queue,
                                                            const int32_t *total, int capacity, double *exact_radiance,
                                                            int32_t *error, unsigned long long *counters) {
@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(128) sample_exact_kernel(SceneView S, const Ce
     const int rank = slot / capacity;
     const int pixel = active ? S.pixel_of_rank[rank] : 0;
     const CellPose pose = poses[active ? exact_cells[slot] : 0];
-    const PixelSample s = sample_pixel_packet<kRadiance, kGeo>(S, pixel, active, pose, s_code[wib], s_t[wib], nullptr);
+    const PixelSample s = sample_pixel_group<kRadiance, 1, kGeo, false>(S, pixel, active, pose, s_code[wib], s_t[wib],
+                                                                        nullptr, nullptr, nullptr);
     if (active) {
       if (!s.valid || !isfinite(s.radiance)) atomicOr(error, kErrOptical);
       exact_radiance[slot] = s.radiance;

@@ -95,7 +95,9 @@ template <int kRays>
 cudaError_t trace_jobs_rays(const TraceJobs &jobs, int geometry, cudaStream_t s) {
   bool beam = false;  // one job with beams takes the kernel that has them
   for (int j = 0; j < jobs.n_jobs; ++j) beam = beam || jobs.jobs[j].shape.beam;
-#define DVS_JOBS_GEO(G) (beam ? trace_jobs_geo<kRays, G, true>(jobs, s) : trace_jobs_geo<kRays, G, false>(jobs, s))
+  // (two rays per lane are chosen only where no job has beams)
+#define DVS_JOBS_GEO(G)                                                                                  \
+  (kRays == 1 && beam ? trace_jobs_geo<kRays, G, kRays == 1>(jobs, s) : trace_jobs_geo<kRays, G, false>(jobs, s))
   switch (geometry) {
     case kGeoHalfBounds: return DVS_JOBS_GEO(kGeoHalfBounds);
     case kGeoWatertight: return DVS_JOBS_GEO(kGeoWatertight);

@@ -475,41 +475,6 @@ __device__ __forceinline__ bool packet_slab(const ChildRec &c, const Packet &P, 
   tnear = lb;
   return ub >= lb;
 }
-// Warp minimum and maximum of one value from one order-preserving key;
-// inactive lanes count as +inf for the minimum and -inf for the maximum.
-__device__ __forceinline__ void wminmax(float x, bool active, float &lo, float &hi) {
-  const unsigned k = ford(x);
-  lo = funord(__reduce_min_sync(kFull, active ? k : 0xff800000u));  // ford(+inf)
-  hi = funord(__reduce_max_sync(kFull, active ? k : 0x007fffffu));  // ford(-inf)
-}
-__device__ Packet make_packet(const SceneView &S, float3 o, float3 d, float3 idir, bool active) {
-  Packet P;
-  wminmax(o.x, active, P.olo.x, P.ohi.x);
-  wminmax(o.y, active, P.olo.y, P.ohi.y);
-  wminmax(o.z, active, P.olo.z, P.ohi.z);
-  wminmax(idir.x, active, P.ilo.x, P.ihi.x);
-  wminmax(idir.y, active, P.ilo.y, P.ihi.y);
-  wminmax(idir.z, active, P.ilo.z, P.ihi.z);
-  float dlo, dhi;
-  wminmax(d.x, active, dlo, dhi);
-  const float dx = dhi - dlo;
-  wminmax(d.y, active, dlo, dhi);
-  const float dy = dhi - dlo;
-  wminmax(d.z, active, dlo, dhi);
-  const float dz = dhi - dlo;
-  const float ds = fmaxf(fmaxf(dx, dy), dz);
-  const float os = fmaxf(fmaxf(P.ohi.x - P.olo.x, P.ohi.y - P.olo.y), P.ohi.z - P.olo.z);
-  P.nx = P.ihi.x < 0.0f;
-  P.ny = P.ihi.y < 0.0f;
-  P.nz = P.ihi.z < 0.0f;
-  const bool one_sign = (P.nx || P.ilo.x > 0.0f) && (P.ny || P.ilo.y > 0.0f) && (P.nz || P.ilo.z > 0.0f);
-  // bundles whose footprint stays within a small fraction of the scene
-  P.coherent = one_sign && ds <= kCoherentSpread && os <= S.coherent_span;
-  P.o_near = f3(P.nx ? P.olo.x : P.ohi.x, P.ny ? P.olo.y : P.ohi.y, P.nz ? P.olo.z : P.ohi.z);
-  P.o_far = f3(P.nx ? P.ohi.x : P.olo.x, P.ny ? P.ohi.y : P.olo.y, P.nz ? P.ohi.z : P.olo.z);
-  return P;
-}
-
 // Warp-uniform traversal stack in shared memory: node codes and the packet's
 // entry distance.  Inner node: index >= 0; leaf: -(node * 8 + slot) - 1.
 struct Stack {
@@ -524,190 +489,6 @@ struct HitRecord {
   int tri;
   float t, u, v;
 };
-
-// Expands an inner node: children the packet may hit are ordered near to far;
-// all but the nearest go on the stack.  Returns false when none is hit.
-// Coherent packets test one child per lane (lanes 0..7) with interval bounds;
-// others test every child per ray and take the warp minimum as the key.
-template <bool kSorted, int kGeo>
-__device__ __forceinline__ bool expand_node(const SceneView &S, int node, const Packet &P, float3 o, float3 idir,
-                                            bool lane_live, float t_min, float lane_tmax, float packet_tmax,
-                                            Stack &st, int &next, float &next_t, bool &overflow) {
-  const int lane = threadIdx.x & 31;
-  float key = kInf();
-  bool hit = false;
-  int code = 0;
-  if (P.coherent) {
-    if (lane < kBvhWidth) {
-      const ChildRec c = load_child<kGeo>(S, node, lane);
-      if (c.count >= 0) {
-        hit = packet_slab(c, P, t_min, packet_tmax, key);
-        code = c.count > 0 ? leaf_code(node, lane) : c.child;
-      }
-    }
-  } else {
-    for (int slot = 0; slot < kBvhWidth; ++slot) {
-      const ChildRec c = load_child<kGeo>(S, node, slot);
-      float tn = kInf();
-      const bool h = c.count >= 0 && lane_live && slab(c.lo, c.hi, o, idir, t_min, lane_tmax, tn);
-      const float k = wmin(h ? tn : kInf());
-      if (lane == slot) {
-        hit = k < kInf();
-        key = k;
-        code = c.count > 0 ? leaf_code(node, slot) : c.child;
-      }
-    }
-  }
-  const unsigned mask = __ballot_sync(kFull, hit && lane < kBvhWidth);
-  if (!mask) return false;
-  const int n = __popc(mask);
-  if (n == 1) {  // the common case of a thin packet: nothing to order or push
-    const int only = __ffs(mask) - 1;
-    next = __shfl_sync(kFull, code, only);
-    next_t = __shfl_sync(kFull, key, only);
-    return true;
-  }
-  int rank = 0;
-  if (kSorted) {
-#pragma unroll
-    for (int j = 0; j < kBvhWidth; ++j) {
-      const float kj = __shfl_sync(kFull, key, j);
-      rank += ((mask >> j) & 1) && (kj < key || (kj == key && j < lane)) ? 1 : 0;
-    }
-  } else {
-    rank = __popc(mask & ((1u << lane) - 1u));
-  }
-  if (st.sp + n - 1 > kStackSlots) {
-    overflow = true;
-    return false;
-  }
-  if (hit && lane < kBvhWidth && rank > 0) {
-    const int slot = st.sp + (n - 1 - rank);
-    st.code[slot] = code;
-    st.t[slot] = key;
-  }
-  const int first = __ffs(__ballot_sync(kFull, hit && lane < kBvhWidth && rank == 0)) - 1;
-  next = __shfl_sync(kFull, code, first);
-  next_t = __shfl_sync(kFull, key, first);
-  st.sp += n - 1;
-  __syncwarp();
-  return true;
-}
-
-// Nearest hit for the rays of a warp (trace_nearest, device_ray.hpp:136-158).
-// All 32 lanes call converged; inactive lanes never hit.  Each lane tests a
-// leaf's triangles only when its own slab test reaches the leaf.
-template <int kGeo>
-__device__ HitRecord trace_nearest_packet(const SceneView &S, float3 o, float3 d, bool active, int *stack_code,
-                                          float *stack_t) {
-  const float3 idir = inverse_direction(d);
-  const WtRay wr = wt_ray<kGeo>(d);
-  const float3 op = wt_origin<kGeo>(wr, o);
-  float closest = active ? 1e30f : -1.0f;
-  HitRecord h{0, -1, 0.f, 0.f, 0.f};
-  const Packet P = make_packet(S, o, d, idir, active);
-  float packet_tmax = wmax(active ? closest : -1.0f);
-  Stack st{stack_code, stack_t, 0};
-  int entry = 0;
-  float entry_t = 0.0f;
-  bool overflow = false;
-  while (true) {
-    if (entry_t <= packet_tmax) {
-      if (entry >= 0) {
-        int next;
-        float next_t;
-        if (expand_node<true, kGeo>(S, entry, P, o, idir, active, kRayEps, closest, packet_tmax, st, next, next_t,
-                              overflow)) {
-          entry = next;
-          entry_t = next_t;
-          continue;
-        }
-        if (overflow) break;
-      } else {
-        const int lc = -entry - 1;
-        const ChildRec c = load_child<kGeo>(S, lc / kBvhWidth, lc % kBvhWidth);
-        float tn;
-        const bool need = active && slab(c.lo, c.hi, o, idir, kRayEps, closest, tn);
-        for (int i = 0; i < c.count; ++i) {
-          const float4 *r = tri_record<kGeo>(S, c.child + i, wr.kz);
-          const float4 a = __ldg(r), b = __ldg(r + 1), q = __ldg(r + 2);
-          float t, u, v;
-          if (need && tri_hit<kGeo>(wr, d, o, op, a, b, q, t, u, v) && t < closest) {
-            closest = t;
-            h.hit = 1; h.tri = c.child + i; h.t = t; h.u = u; h.v = v;
-          }
-        }
-        packet_tmax = wmax(active ? closest : -1.0f);
-      }
-    }
-    if (st.sp == 0) break;
-    --st.sp;
-    entry = st.code[st.sp];
-    entry_t = st.t[st.sp];
-  }
-  __syncwarp();
-  if (overflow) h.hit = -1;
-  return h;
-}
-
-// Any hit toward the light (trace_shadow_ray_any_hit, device_ray.hpp:81-135):
-// skips the camera-hit triangle, t in (kRayEps, 1e30); overflow counts as occluded.
-template <int kGeo>
-DVS_SHADE_INLINE __device__ bool trace_shadow_packet(const SceneView &S, float3 o, float3 d, bool active, int self,
-                                                     int *stack_code, float *stack_t) {
-  const float3 idir = inverse_direction(d);
-  const WtRay wr = wt_ray<kGeo>(d);
-  const float3 op = wt_origin<kGeo>(wr, o);
-  bool alive = active;
-  bool occluded = false;
-  const float t_max = 1e30f;
-  const Packet P = make_packet(S, o, d, idir, active);
-  Stack st{stack_code, stack_t, 0};
-  int entry = 0;
-  float entry_t = 0.0f;
-  bool overflow = false;
-  while (__any_sync(kFull, alive)) {
-    if (entry >= 0) {
-      int next;
-      float next_t;
-      if (expand_node<false, kGeo>(S, entry, P, o, idir, alive, kRayEps, alive ? t_max : -1.0f, t_max, st, next, next_t,
-                             overflow)) {
-        entry = next;
-        entry_t = next_t;
-        continue;
-      }
-      if (overflow) {
-        occluded = occluded || alive;  // conservative (device_ray.hpp:119)
-        break;
-      }
-    } else {
-      const int lc = -entry - 1;
-      const ChildRec c = load_child<kGeo>(S, lc / kBvhWidth, lc % kBvhWidth);
-      float tn;
-      const bool need = alive && slab(c.lo, c.hi, o, idir, kRayEps, t_max, tn);
-      for (int i = 0; i < c.count; ++i) {
-        const int id = c.child + i;
-        const float4 *r = tri_record<kGeo>(S, id, wr.kz);
-        const float4 a = __ldg(r), b = __ldg(r + 1), q = __ldg(r + 2);
-        float t, u, v;
-        if (need && alive && id != self &&
-            tri_hit<kGeo>(wr, d, o, op, a, b, q, t, u, v) && t > kRayEps &&
-            t < t_max) {
-          occluded = true;
-          alive = false;
-        }
-      }
-    }
-    if (st.sp == 0) break;
-    --st.sp;
-    entry = st.code[st.sp];
-    entry_t = st.t[st.sp];
-  }
-  (void)entry_t;
-  __syncwarp();
-  return occluded;
-}
-
 
 // The float after a finite x in the direction of the sign of `to` (nextafterf toward +-infinity); x when `to` is zero.
 __device__ __forceinline__ float next_toward(float x, float to) {
@@ -775,82 +556,12 @@ __device__ __forceinline__ float subray_y(const SceneView &S, int py_i, int sy) 
   return (py_i + (sy + .5f) / S.samples - .5f - S.cy) / S.fy;
 }
 
-// sample_pixel (device_optics.cuh:73-94) for one lane of a converged warp.
-// subrays: when every lane of the warp samples the same pixel, its sub-rays'
-// coordinates and cos^4, formed once per warp (shared memory); otherwise nullptr.
-template <int kMode, int kGeo = kGeoReference>
-__device__ PixelSample sample_pixel_packet(const SceneView &S, int pixel, bool active, const CellPose &pose,
-                                           int *stack_code, float *stack_t, const SubraySample *subrays) {
-  PixelSample out{0.0, -1.0f, true, 0u, 0u, false};
-  double depth = 0;
-  int valid_depth = 0;
-  const float3 light = f3(pose.lx, pose.ly, pose.lz);
-  const float3 origin = f3(pose.px, pose.py, pose.pz);
-  const int ss = S.samples;
-  const int px_i = pixel % S.width, py_i = pixel / S.width;
-  const HapkeConst &hc = S.hc;
-  const float3 lnorm = unit(light);  // as in sample_pixel_group
-  for (int sy = 0; sy < ss; ++sy)
-    for (int sx = 0; sx < ss; ++sx) {
-      const float px = subrays ? subrays[sy * ss + sx].px : subray_x(S, px_i, sx);
-      const float py = subrays ? subrays[sy * ss + sx].py : subray_y(S, py_i, sy);
-      const float3 ray = unit(rotate_ray(pose, f3(px, -py, -1)));
-      const HitRecord hit = trace_nearest_packet<kGeo>(S, origin, ray, active && out.valid, stack_code, stack_t);
-      if (active && out.valid) ++out.primary;
-      if (hit.hit < 0) out.valid = false;
-      const bool hitp = active && out.valid && hit.hit == 1;
-      bool lit = false;
-      float3 normal = f3(0, 0, 0), sorigin = f3(0, 0, 0);
-      float albedo = S.hapke.w, r0 = hc.r0_w;
-      if (hitp) {
-        if (kMode != kRadiance) {
-          depth += hit.t;
-          ++valid_depth;
-        }
-        if (kMode != kDepthOnly) {
-          const ShadeRecord *sr = S.shade + hit.tri;
-          const float4 *q = reinterpret_cast<const float4 *>(sr);
-          const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
-          const float w = 1 - hit.u - hit.v;
-          normal = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit.u + f3(s2.x, s2.y, s2.z) * hit.v);
-          lit = !(dot(normal, light) <= 0 || dot(normal, -ray) <= 0);
-          if (lit) {
-            const float4 *r = tri_record<kGeo>(S, hit.tri, 2);
-            const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-            sorigin = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit.u, hit.v, light);
-            if (S.has_albedo) {
-              albedo = s0.w * w + s1.w * hit.u + s2.w * hit.v;
-              r0 = hfunc_r0(albedo);
-            }
-          }
-        }
-      }
-      if (kMode != kDepthOnly) {
-        if (__any_sync(kFull, lit)) {
-          if (lit) ++out.shadow;
-          const bool occ = trace_shadow_packet<kGeo>(S, sorigin, light, lit, hit.tri, stack_code, stack_t);
-          if (lit && !occ) {
-            const double cos4 = subrays ? subrays[sy * ss + sx].cos4 : cos4_of(px, py);
-            // hapke_directional_reflectance (hapke.hpp:153-157)
-            const float3 n = unit(normal), l = lnorm, v = unit(-ray);
-            const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo, r0, S.hapke, hc);
-            out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
-          }
-        }
-      }
-    }
-  out.radiance /= ss * ss;
-  out.depth = valid_depth ? float(depth / valid_depth) : -1.0f;
-  return out;
-}
-
-// ---- two sub-rays per lane ------------------------------------------------------
-// The same traversal with each lane carrying R rays (two neighbouring sub-rays
-// of its pixel-cell): the packet is 32 x R rays, so the interval node tests,
-// the stack traffic and the packet set-up are paid once per 32 x R rays, and
-// a leaf's triangle records are loaded once for the lane's R rays.  Per-ray
-// results are those of the one-ray traversal (every interval bound covers
-// all R rays; leaves are tested per ray).
+// ---- packet walks: R sub-rays per lane ---------------------------------------------
+// A packet is 32 x R rays: each lane carries R neighbouring sub-rays of its
+// pixel-cell, so the interval node tests, the stack traffic and the packet
+// set-up are paid once per 32 x R rays, and a leaf's triangle records are
+// loaded once for the lane's R rays.  Per-ray results do not depend on R
+// (every interval bound covers all R rays; leaves are tested per ray).
 
 // Warp extremes of per-lane [lo, hi] ranges; inactive lanes count as empty.
 __device__ __forceinline__ void wrange(float lo, float hi, bool active, float &wlo, float &whi) {
@@ -900,6 +611,10 @@ __device__ Packet make_packet_r(const SceneView &S, const float3 (&o)[R], const 
   return P;
 }
 
+// Expands an inner node: children the packet may hit are ordered near to far;
+// all but the nearest go on the stack.  Returns false when none is hit.
+// Coherent packets test one child per lane (lanes 0..7) with interval bounds;
+// others test every child per ray and take the warp minimum as the key.
 template <bool kSorted, int R, int kGeo>
 __device__ __forceinline__ bool expand_node_r(const SceneView &S, int node, const Packet &P, const float3 (&o)[R],
                                               const float3 (&idir)[R], const bool (&live)[R], float t_min,
@@ -979,6 +694,9 @@ __device__ __forceinline__ float lane_reach(const bool (&active)[R], const float
   return m;
 }
 
+// Nearest hits of a packet (trace_nearest, device_ray.hpp:136-158).  All 32
+// lanes call converged; inactive rays never hit.  Each ray is tested against a
+// leaf's triangles only when its own slab test reaches the leaf.
 template <int R, int kGeo>
 __device__ void trace_nearest_packet_r(const SceneView &S, const float3 (&o)[R], const float3 (&d)[R],
                                        const bool (&active)[R], int *stack_code, float *stack_t, HitRecord (&h)[R]) {
@@ -1069,6 +787,8 @@ __device__ __forceinline__ ShadowDir shadow_dir(float3 light) {
   return ShadowDir{inverse_direction(light), wt_ray<kGeo>(light)};
 }
 
+// Any hit toward the light (trace_shadow_ray_any_hit, device_ray.hpp:81-135):
+// skips the camera-hit triangle, t in (kRayEps, 1e30); overflow counts as occluded.
 template <int R, int kGeo>
 __device__ void trace_shadow_packet_r(const SceneView &S, const float3 (&o)[R], float3 light, const ShadowDir &sd,
                                       const bool (&active)[R], const int (&self)[R], int *stack_code, float *stack_t,
@@ -1590,16 +1310,18 @@ __device__ __forceinline__ unsigned shadow_in_list(const SceneView &S, const Bea
   return occluded;
 }
 
-// sample_pixel_packet with R neighbouring sub-rays per lane (ss^2 a multiple
-// of R).  The per-ray work, the order of the FP64 radiance and depth sums and
-// the ray counts are those of the one-ray loop.
+// sample_pixel (device_optics.cuh:73-94) for one lane of a converged warp, R
+// neighbouring sub-rays at a time (ss^2 a multiple of R).  The order of the FP64
+// radiance and depth sums and the ray counts do not depend on R.
+// subrays: the sub-rays' coordinates and cos^4, formed once per pixel (shared memory), or nullptr.
 // kBeam: the item has lists, and the packets' leaves come from them; a ray
 // outside the beam ends the sample (redo).  The loop then holds no call, whose
 // registers would be spilled around it.
 template <int kMode, int R, int kGeo, bool kBeam>
 __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, int pixel, bool active,
                                                           const CellPose &pose, int *stack_code, float *stack_t,
-                                                          const SubraySample *subrays, Beam &B, BeamLists &lists) {
+                                                          const SubraySample *subrays, const Beam *beam,
+                                                          BeamLists *lists) {
   PixelSample out{0.0, -1.0f, true, 0u, 0u, false};
   double depth = 0;
   int valid_depth = 0;
@@ -1628,7 +1350,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
       }
       ray[r] = unit(rotate_ray(pose, f3(px[r], -py[r], -1)));
       live[r] = active && out.valid;
-      if constexpr (kBeam) inside = inside && (!live[r] || within(ray[r], B.dlo, B.dhi));
+      if constexpr (kBeam) inside = inside && (!live[r] || within(ray[r], beam->dlo, beam->dhi));
     }
     HitRecord hit[R];
     if constexpr (!kBeam) {
@@ -1641,7 +1363,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
         out.redo = true;
         return out;
       }
-      nearest_in_list<R, kGeo>(S, B, lists.leaves, origin, ray, live, hit);
+      nearest_in_list<R, kGeo>(S, *beam, lists->leaves, origin, ray, live, hit);
     }
     bool lit[R];
     float3 normal[R], sorigin[R];
@@ -1691,7 +1413,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
         bool near = true;
         if constexpr (kBeam) {
 #pragma unroll
-          for (int r = 0; r < R; ++r) near = near && (!lit[r] || within(sorigin[r], B.slo, B.shi));
+          for (int r = 0; r < R; ++r) near = near && (!lit[r] || within(sorigin[r], beam->slo, beam->shi));
         }
         if constexpr (!kBeam) {
           bool occ[R];
@@ -1703,7 +1425,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
             out.redo = true;
             return out;
           }
-          occluded = shadow_in_list<R, kGeo>(S, B, lists.shadow, sorigin, light, sdir, lit, self, lists.first);
+          occluded = shadow_in_list<R, kGeo>(S, *beam, lists->shadow, sorigin, light, sdir, lit, self, lists->first);
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {

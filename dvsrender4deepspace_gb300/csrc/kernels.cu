@@ -2,21 +2,26 @@
 //
 // Built with -fmad=false: every floating-point expression rounds exactly as
 // the reference writes it (and as the oracle computes it on the CPU), so the
-// ray directions, Moller-Trumbore results, shadow origins and the FP64
-// circuit differ from the reference only where CUDA's transcendental
-// functions differ from the host C library.
+// ray directions, Moller-Trumbore results and shadow origins differ from the
+// reference only where CUDA's transcendental functions differ from the host C
+// library (quotients and roots: device_math.cuh), and the FP64 circuit by the
+// last bits of its receptor step (device_circuit.cuh).
 //
 // Work decomposition
-//   * trace_cells: one warp traces a packet of 32 (pixel, cell) samples --
-//     32/CW Morton-adjacent pixels x CW consecutive circuit cells.  All lanes
-//     walk the 8-wide BVH together (warp-uniform control flow); coherent
-//     packets test one child per lane against the packet's ray intervals,
-//     leaves are tested per lane, and each lane keeps its own closest hit.
-//     The traversal stack is warp-uniform and lives in shared memory.
+//   * trace_cells: a warp's item is many packets of 32 (pixel, cell) samples --
+//     32/CW Morton-adjacent pixels x CW consecutive circuit cells -- over the
+//     pixel's sub-rays, several cell groups and pixels.  Items with enough
+//     packets walk the 8-wide BVH once for all of them (the beam,
+//     device_optics.cuh) and test the leaves it reaches; the others walk it per
+//     packet, all lanes together: coherent packets test one child per lane
+//     against the packet's ray intervals, leaves are tested per lane, and each
+//     lane keeps its own closest hit.  The stack and the lists live in shared memory.
+//   * trace_poses: few poses a pixel (frames, initial pose, probes): packets of
+//     one or more pixels' sub-rays, items of several pixels through one beam.
 //   * circuit: one thread per pixel streams the per-cell radiance of a chunk
-//     and integrates the pixel circuit in FP64 (pixel_model.hpp semantics).
+//     and integrates the pixel circuit (pixel_model.hpp semantics).
 //   * emit_events: warp prefix-sum compaction of the per-pixel event slabs.
-//   * event_depth: depth re-trace at each event time (event_sensor.cu:51-59).
+//   * event_depth: depth re-trace at each event time, a warp per event (event_sensor.cu:51-59).
 #include <cstdint>
 #include <type_traits>
 #include <cuda_runtime.h>

@@ -88,12 +88,10 @@ template <int kMode, int kGeo>
 __device__ __noinline__ PixelSample sample_without_beam(const SceneView &S, int pixel, bool active,
                                                         const CellPose *pose_at, TraceShared &sh,
                                                         const SubraySample *subrays) {
-  BeamLists none{kNoList, kNoList, 0};
-  Beam &unused = *reinterpret_cast<Beam *>(&sh);  // not touched without lists
   const CellPose pose = *pose_at;
   if (S.samples % 2 == 0)
-    return sample_pixel_group<kMode, 2, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
-  return sample_pixel_group<kMode, 1, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, unused, none);
+    return sample_pixel_group<kMode, 2, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, nullptr, nullptr);
+  return sample_pixel_group<kMode, 1, kGeo, false>(S, pixel, active, pose, sh.code, sh.t, subrays, nullptr, nullptr);
 }
 
 // One warp's item of a trace launch: shape.sets pixel sets (32/CW
@@ -148,7 +146,7 @@ __device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, 
       PixelSample s;
       bool by_list = !kBeam || lists.shadow >= 0;
       if (by_list) {
-        s = sample_pixel_group<kMode, kRays, kGeo, kBeam>(S, pixel, active, pose, sh.code, sh.t, mine, beam, lists);
+        s = sample_pixel_group<kMode, kRays, kGeo, kBeam>(S, pixel, active, pose, sh.code, sh.t, mine, &beam, &lists);
         by_list = !s.redo;
       }
       if (kBeam && !by_list) s = sample_without_beam<kMode, kGeo>(S, pixel, active, at, sh, mine);
