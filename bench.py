@@ -82,12 +82,12 @@ METRIC = "DVS events/s and Mrays/s at 1280x720 on 1 GB300; serving p99 latency v
 # (dram__bytes_read.sum + dram__bytes_write.sum) per pixel-cell.  Radiance
 # writes still held in L2 when the kernel ends are not in the DRAM count.
 TRACE_WARP_INSTRUCTIONS_PER_RAY = {
-    ("precision", "half+watertight", "sah", 32, 2): 1466157173123 / 29471262019,
-    ("orbit", "reference", "sah", 32, 2): 79970172908 / 1768685229,
+    ("precision", "half+watertight", "sah", 32, 1): 731631334830 / 29471262019,
+    ("orbit", "reference", "sah", 32, 1): 50147058636 / 1768685229,
 }
 TRACE_DRAM_BYTES_PER_PIXEL_CELL = {
-    ("precision", "half+watertight", "sah", 32, 2): (66908416 + 219526144) / (921600 * 64),
-    ("orbit", "reference", "sah", 32, 2): (14630400 + 178991360) / (89960 * 640),
+    ("precision", "half+watertight", "sah", 32, 1): (71990016 + 284999168) / (921600 * 64),
+    ("orbit", "reference", "sah", 32, 1): (17014784 + 235764224) / (89960 * 640),
 }
 # ncu DRAM counters (dram__bytes_read.sum + dram__bytes_write.sum) of the 44
 # launches of one device-readout batch of 4,194,304 events (the readout
@@ -525,7 +525,7 @@ def run_gb300(args):
     # per ray that ncu counted for this kernel and format, at the sampled clock
     rays_per_launch = rays / max(1, st["optics_launches"])
     issue = None
-    shape = ((tuning["cells_per_warp"], tuning["rays_per_lane"]) if tuning else (args.cw or 32, args.rays or 2))
+    shape = ((tuning["cells_per_warp"], tuning["rays_per_lane"]) if tuning else (args.cw or 32, args.rays or 1))
     counted = (args.workload, args.geometry, args.builder) + shape
     ipr = TRACE_WARP_INSTRUCTIONS_PER_RAY.get(counted)
     sm_mhz = clocks.summary()["sm_mhz"]

@@ -1180,7 +1180,7 @@ static int enqueue(dvs_sensor *s, const dvs_optical_interval *ivs, size_t count)
     CUDA_TRY(launch_circuit(n, s->cells, (int)c0, nc, s->radiance, s->p, s->photo, s->max_events, s->st, s->ev_count,
                             s->slab_t, s->slab_p, s->error_word, s->counters, s->stream),
              "integrate circuits");
-    s->stats.launches += 2;
+    s->stats.launches += circuit_draws_ahead(n, s->p, s->photo) ? 3 : 2;
     s->stats.optics_launches += 1;
     s->stats.circuit_launches += 1;
   }

@@ -540,6 +540,12 @@ __device__ __forceinline__ curandStatePhilox4_32_10_t philox_at(unsigned seed, i
   return st;
 }
 
+// A cell's photon count as a rate, from its own place in the pixel's stream.
+__device__ __forceinline__ float philox_rate(const PhotoParams &photo, float rate, int pixel, const Cell &cell) {
+  curandStatePhilox4_32_10_t ph = philox_at(photo.seed, pixel, cell.t0);
+  return poisson_electrons_philox(ph, rate * cell.dt) / cell.dt;
+}
+
 // poisson_electrons (include/dvs/photon_noise.cuh:4-9): cuRAND draws in the
 // reference's order so seeded streams match a reference build on the same toolkit.
 __device__ __forceinline__ double poisson_electrons(curandStateXORWOW_t &rng, double lambda) {

@@ -132,6 +132,21 @@ __global__ void init_pixels_kernel(int n, const int32_t *pixel_of_rank, const do
   if constexpr (std::is_same<Rng, curandStateXORWOW_t>::value) st.rng[k] = rng;
 }
 
+// The photon counts of a float radiance chunk, in place, as rates: the draw of circuit_rank's Philox cells, a thread per
+// pixel-cell.
+__global__ void __launch_bounds__(128) philox_draws_kernel(int n, const Cell *cells, int c0, int nc,
+                                                           const int32_t *pixel_of_rank, PhotoParams photo,
+                                                           float *chunk) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (long long)n * nc) return;
+  const int c = (int)(i / n), r = (int)(i - (long long)c * n);
+  const float rad = chunk[i];
+  if (!isfinite(rad)) return;  // the circuit reports it
+  const Cell cell = cells[c0 + c];
+  chunk[i] = philox_rate(photo, rad * (float)photo.electrons_per_radiance + (float)photo.dark_electrons,
+                         pixel_of_rank[r], cell);
+}
+
 template <bool kF32, bool kPhilox>
 __global__ void __launch_bounds__(128) circuit_kernel(int n, const int32_t *rank_list, const Cell *cells, int c0,
                                                       int nc, const double *radiance, PixelParams p,
@@ -278,6 +293,7 @@ __global__ void poisson_draws_kernel(int generator, double lambda, unsigned seed
   }
 }
 
+constexpr long long kResidentWarps = 2432;  // 152 SMs x 16 warps
 inline int blocks(long long threads, int per_block) { return (int)((threads + per_block - 1) / per_block); }
 
 }  // namespace
@@ -320,7 +336,6 @@ cudaError_t launch_cell_poses(const dvs_optical_interval *ivs, const Cell *cells
 }
 
 namespace {
-constexpr long long kResidentWarps = 2432;  // 152 SMs x 16 warps
 // Few poses: packets of sub-rays.  One sub-ray a pixel fills a packet with a block of 8 x 4 pixels; where so few pixels
 // leave the GPU idle, narrower packets on more warps.
 bool trace_by_pose(const SceneView &scene, int n_pix, int nc) {
@@ -440,9 +455,24 @@ cudaError_t launch_circuit_list(int n, const int32_t *rank_list, const Cell *cel
   return cudaGetLastError();
 }
 
-cudaError_t launch_circuit(int n, const Cell *cells, int c0, int nc, const double *radiance, PixelParams p,
+// A Philox draw depends on its pixel and cell alone.  With few pixels the
+// circuit's threads, one a pixel, cannot hide a cell's chain of draw and receptor
+// step, so the draws of all cells go ahead on a thread each: 64 cells of 64x48
+// pixels 93 -> 68 us, of 128x96 95 -> 76, of 256x192 102 -> 98; of 320x240 110 ->
+// 118, so the line lies at two warps a scheduler.  (Reset noise continues a
+// cell's stream after its draw and keeps the draw in the circuit.)
+bool circuit_draws_ahead(int n, const PixelParams &p, const PhotoParams &photo) {
+  return photo.philox && photo.chunk_f32 && photo.shot_noise && p.reset_noise_std == 0 && n < kResidentWarps * 16;
+}
+
+cudaError_t launch_circuit(int n, const Cell *cells, int c0, int nc, double *radiance, PixelParams p,
                            PhotoParams photo, int max_events, CircuitState st, int32_t *ev_count, double *slab_t,
                            int8_t *slab_p, int32_t *error, unsigned long long *counters, cudaStream_t s) {
+  if (circuit_draws_ahead(n, p, photo)) {
+    philox_draws_kernel<<<blocks((long long)n * nc, 128), 128, 0, s>>>(n, cells, c0, nc, st.pixel, photo,
+                                                                       reinterpret_cast<float *>(radiance));
+    photo.drawn = 1;
+  }
   return launch_circuit_list(n, nullptr, cells, c0, nc, radiance, p, photo, max_events, st, ev_count, slab_t, slab_p,
                              error, counters, s);
 }

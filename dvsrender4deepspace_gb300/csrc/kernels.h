@@ -59,6 +59,7 @@ struct PhotoParams {
   int32_t fp32_circuit;  // receptor/contrast arithmetic in FP32 (times and crossing solves stay FP64)
   int32_t philox;        // counter-based Philox noise keyed by (seed, pixel, cell index) instead of XORWOW
   uint32_t seed;
+  int32_t drawn;         // the chunk holds rates: the cells' photon counts are drawn already (launch_circuit)
   int32_t chunk_f32;     // the circuit reads a float radiance chunk (FP32 circuits: the values it uses are floats)
 };
 
@@ -217,7 +218,9 @@ cudaError_t launch_trace_cells(const SceneView &scene, int n_pix, const CellPose
 cudaError_t launch_init_pixels(int n_pix, const int32_t *pixel_of_rank, const double *radiance, PixelParams p,
                                PhotoParams photo, double threshold_std, double threshold_min, unsigned seed,
                                CircuitState st, int32_t *error, cudaStream_t s);
-cudaError_t launch_circuit(int n_pix, const Cell *cells, int c0, int nc, const double *radiance, PixelParams p,
+// Whether a circuit launch draws its cells' photon counts ahead in a kernel of its own (in place of the chunk's radiance).
+bool circuit_draws_ahead(int n_pix, const PixelParams &p, const PhotoParams &photo);
+cudaError_t launch_circuit(int n_pix, const Cell *cells, int c0, int nc, double *radiance, PixelParams p,
                            PhotoParams photo, int max_events, CircuitState st, int32_t *ev_count, double *slab_t,
                            int8_t *slab_p, int32_t *error, unsigned long long *counters, cudaStream_t s);
 cudaError_t launch_emit_events(int n_pix, const int32_t *pixel_of_rank, int width, int max_events,

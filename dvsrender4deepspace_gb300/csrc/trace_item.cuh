@@ -299,12 +299,15 @@ __device__ __forceinline__ void circuit_rank(int r, int n, const int32_t *rank_l
       const size_t o = (size_t)c * n + r;
       const float rad = chunk_f ? chunk_f[o] : (float)radiance[o];
       if (!isfinite(rad)) { failed = kErrOptical; break; }
-      float rate = rad * e_rad + dark;
+      float rate = photo.drawn ? rad : rad * e_rad + dark;
       const float dt = cell.dt;
       int emitted;
       if (kPhilox) {
-        curandStatePhilox4_32_10_t ph = philox_at(photo.seed, pixel, cell.t0);
-        if (photo.shot_noise) rate = poisson_electrons_philox(ph, rate * dt) / dt;
+        curandStatePhilox4_32_10_t ph{};
+        if (!photo.drawn) {  // drawn: nothing more is taken from the stream
+          ph = philox_at(photo.seed, pixel, cell.t0);
+          if (photo.shot_noise) rate = poisson_electrons_philox(ph, rate * dt) / dt;
+        }
         emitted = advance_pixel_f32(s, p, pf, rate, cell.t0, dt, my_t + cnt, my_p + cnt, max_events - cnt, ph);
       } else {
         if (photo.shot_noise) rate = (float)poisson_electrons(rng, (double)(rate * dt)) / dt;
