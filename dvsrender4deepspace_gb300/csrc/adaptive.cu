@@ -60,7 +60,9 @@ __global__ void probe_poses_kernel(const dvs_optical_interval *ivs, int n_ivs, d
 // kAhead pending segments: two probes each, their poses one per lane, their
 // sub-rays 32 to a packet through the pixel's beam.  Knots, fallbacks and
 // counters are the depth-first walk's: an overflow of the knot capacity takes
-// back the count of the splits that walk would not have reached.
+// back the splits that walk would not have reached, their rays and their
+// errors.  Those are the splits of segments that lie behind the overflow, so
+// each split's tally goes with the leftmost of its pending descendants.
 //
 // Bound by the latency of the probes' packets and the FP64 pipe of the
 // verdicts.  One pixel per lane instead (32 pixels in lock-step, each lane
@@ -76,8 +78,13 @@ struct RefineShared {
   CellPose pose[32];
   double term[32][kProbeRays + 1];  // [probe][sub-ray], rows apart in the banks
   double seg[5][32];
+  unsigned long long tally[32];
   int behind[32], verdict[32];
+  unsigned char traced[32][kProbeRays + 4];  // rays of term's sub-ray (1, or 2 with its shadow ray), kProbeBad
 };
+constexpr int kProbeBad = 4;
+// a tally counts rays, and above them probes that overflowed or are not finite
+constexpr int kTallyBadShift = 40;
 enum : int { kUndecided = 0, kSmooth = 1, kExact = 2, kSplit = 3 };
 
 template <int kGeo>
@@ -95,7 +102,7 @@ __global__ void __launch_bounds__(128, 4)
   const int pixel = S.pixel_of_rank[rank];
   const int px_i = pixel % S.width, py_i = pixel / S.width, ss2 = S.samples * S.samples;
   bool bad = false;
-  unsigned rays = 0;
+  unsigned long long traced = 0, tally = 0;  // of this lane's probes; of the splits that go with segment `lane`
   double initial[5];
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
@@ -162,6 +169,7 @@ __global__ void __launch_bounds__(128, 4)
       if (overs) {
         fallback = true;
         not_reached = pending - 1 - emit - __shfl_sync(kFull, behind, emit);
+        if (lane > emit && lane < pending) traced -= tally;  // modulo 2^64; the warp's sum is not negative
         break;
       }
       pending -= done;
@@ -173,6 +181,7 @@ __global__ void __launch_bounds__(128, 4)
       right = __shfl_sync(kFull, right, from);
       behind = __shfl_sync(kFull, behind, from);
       verdict = __shfl_sync(kFull, verdict, from);
+      tally = __shfl_sync(kFull, tally, from);
     }
     if (pending == 0) break;
     // the first pending segment splits; others while the list stays within kAhead
@@ -203,6 +212,8 @@ __global__ void __launch_bounds__(128, 4)
     }
     __syncwarp();
     double sum = 0;
+    unsigned long long probe = 0;
+    bool probe_bad = false;
     for (int r0 = 0; r0 < ss2; r0 += kProbeRays) {
       const int m = min(kProbeRays, ss2 - r0), total = probes * m;
       for (int q0 = 0; q0 < total; q0 += 32) {
@@ -212,19 +223,27 @@ __global__ void __launch_bounds__(128, 4)
         const RaySample s = sample_ray<kRadiance, kGeo, true>(S, subray_x(S, px_i, r % S.samples),
                                                               subray_y(S, py_i, r / S.samples), pose, live, sh.code,
                                                               sh.t, sh.beam, lists);
-        if (live) sh.term[k][q - k * m] = s.term;
-        if (s.overflow) bad = true;
-        rays += (live ? 1u : 0u) + (s.lit ? 1u : 0u);
+        if (live) {
+          sh.term[k][q - k * m] = s.term;
+          sh.traced[k][q - k * m] = (unsigned char)((s.lit ? 2 : 1) | (s.overflow ? kProbeBad : 0));
+        }
       }
       __syncwarp();
       if (lane < probes)
-        for (int i = 0; i < m; ++i) sum += sh.term[lane][i];  // in sub-ray order, as the pixel sample's sum
+        for (int i = 0; i < m; ++i) {
+          sum += sh.term[lane][i];  // in sub-ray order, as the pixel sample's sum
+          const unsigned t = sh.traced[lane][i];
+          probe += t & 3u;
+          probe_bad |= (t & kProbeBad) != 0;
+        }
       __syncwarp();
     }
     sum /= ss2;
-    if (lane < probes && !isfinite(sum)) bad = true;
+    if (lane < probes && (probe_bad || !isfinite(sum))) probe += 1ull << kTallyBadShift;
+    traced += probe;
     // the list with each chosen segment replaced by its halves
     const double left_mid = __shfl_sync(kFull, sum, (2 * slot) & 31), right_mid = __shfl_sync(kFull, sum, (2 * slot + 1) & 31);
+    const unsigned long long spent = __shfl_sync(kFull, probe, (2 * slot) & 31) + __shfl_sync(kFull, probe, (2 * slot + 1) & 31);
     const int to = lane + slot;
     if (lane < pending) {
       const double mid = (a + b) * .5;
@@ -235,6 +254,7 @@ __global__ void __launch_bounds__(128, 4)
       sh.seg[4][to] = mine ? middle : right;
       sh.behind[to] = mine ? behind + 1 : behind;
       sh.verdict[to] = mine ? kUndecided : verdict;
+      sh.tally[to] = mine ? tally + spent : tally;
       if (mine) {
         sh.seg[0][to + 1] = mid;
         sh.seg[1][to + 1] = b;
@@ -243,6 +263,7 @@ __global__ void __launch_bounds__(128, 4)
         sh.seg[4][to + 1] = right;
         sh.behind[to + 1] = behind;
         sh.verdict[to + 1] = kUndecided;
+        sh.tally[to + 1] = 0;
       }
     }
     __syncwarp();
@@ -255,9 +276,12 @@ __global__ void __launch_bounds__(128, 4)
     right = sh.seg[4][lane];
     behind = sh.behind[lane];
     verdict = sh.verdict[lane];
+    tally = sh.tally[lane];
     __syncwarp();
   }
-  if (bad) atomicOr(error, kErrOptical);
+#pragma unroll
+  for (int k = 16; k; k >>= 1) traced += __shfl_xor_sync(kFull, traced, k);
+  if (bad || traced >> kTallyBadShift) atomicOr(error, kErrOptical);
   if (lane == 0) {
     counts[rank] = fallback ? -1 : written;
     atomicAdd(ref_stats + kRefTraced, 5ull + 2ull * (unsigned)(splits - not_reached));
@@ -265,8 +289,7 @@ __global__ void __launch_bounds__(128, 4)
     else atomicMax(ref_stats + kRefMaxKnots, (unsigned long long)written);
     if (exact_segments) atomicAdd(ref_stats + kRefExactSegments, (unsigned long long)exact_segments);
   }
-  const unsigned wr = __reduce_add_sync(kFull, rays);
-  if (lane == 0 && counters) atomicAdd(counters + kCntPrimary, (unsigned long long)wr);
+  if (lane == 0 && counters) atomicAdd(counters + kCntPrimary, traced & ((1ull << kTallyBadShift) - 1));
 }
 
 // identify_exact_cells (optical_sampler.cu:114-131): cells whose midpoint falls

@@ -48,3 +48,35 @@ def test_bands_refine_as_the_whole_sensor(ss, geometry, horizons, pulse, toleran
     assert max(b[1]["maximum_knots"] for b in bands) == stats["maximum_knots"]
     if tolerance == 1e-11:
         assert stats["fallback_pixels"] > 0
+
+
+@pytest.mark.parametrize("capacity_reached", [True, False])
+def test_rays_are_the_probes_rays(capacity_reached):
+    """Over gentle ground under a high sun every ray through a pixel's centre hits and casts a shadow ray (the native
+    run shows it; with many sub-rays a few slip through Moeller-Trumbore's edges), so the rays of a window are twice
+    its counted probes, exact cells and fallback pixels' native cells: probes that the depth-first walk does not
+    reach before a pixel's knots overflow are in neither count."""
+    ss = 1
+    x = 10.0 * np.arange(64)
+    height = 2.0 * np.sin(x[None, :] / 50.0) + 2.0 * np.cos(x[:, None] / 60.0)
+    V, N, I = terrain.mesh_from_heightfield(height.astype(np.float32), 10.0)
+    cam = dict(width=31, height=9, fx=30.0, fy=30.0, cx=15.5, cy=4.5)
+    scene = DeviceScene(V, N, I, cam, ss, HAPKE, geometry=0)
+    traj = trajectory.StraightPass((5.0, -8.0, 350.0), (80.0, 10.0, 0.0), trajectory.sun_direction(60, 40), 1000.0, 0.4)
+    ivs = trajectory.horizons(traj, 0.0, 1e-5, 190 if capacity_reached else 20)
+    phys = physic(photon_shot_noise=0)
+    rays = []
+    tolerance = 1e-11 if capacity_reached else 1e-4
+    for process in (lambda s: s.process_many(ivs), lambda s: s.process_adaptive(ivs, tolerance)):
+        s = EventSensor(scene, phys)
+        s.initialize(traj.state(0.0), 0.0)
+        before = s.stats()
+        assert process(s) is not None
+        after = s.stats()
+        rays.append(sum(after[k] - before[k] for k in ("primary_rays", "shadow_rays")))
+    pixels, stats = 31 * 9, s.refinement_statistics()
+    assert rays[0] % (pixels * 2 * ss * ss) == 0
+    cells = rays[0] // (pixels * 2 * ss * ss)
+    samples = stats["traced_pixel_samples"] + stats["native_cell_queries"] + stats["fallback_pixels"] * cells
+    assert (stats["fallback_pixels"] > 0) == capacity_reached
+    assert rays[1] == 2 * ss * ss * samples
