@@ -121,7 +121,7 @@ __device__ int advance_pixel(PixelRegs &s, const PixelParams &p, double rate, do
 // u near 10 has a last bit of 2e-15, so one log and exp a cell move x by
 // that relative amount, the step above by a few 1e-16.  x is kept between runs
 // (CircuitState::receptor), so how cells are batched changes no bit.  A
-// leaking reference moves the bounds in every cell and takes advance_pixel.
+// reference that leaks, in either direction, moves the bounds in every cell and takes advance_pixel.
 
 // 1 - e^-k for 0 <= k < 0.35 by the Taylor series of (1 - e^-k) / k, whose first term left out is k^14 / 15! < 3e-19.
 __device__ __forceinline__ double one_minus_exp_small(double k) {
@@ -168,7 +168,7 @@ struct CircuitRun {
   PixelRegs s;
   double x, high, low;  // receptor and the comparator's bounds on it
   double inv_charge;
-  bool direct;    // a leaking reference: advance_pixel for every cell
+  bool direct;    // a reference that leaks, up or down: advance_pixel for every cell
   bool follows;   // the reference is the receptor's log, not yet written down
   bool settled;   // past the refractory deadline, nothing pending, the receptor between the bounds
 };
@@ -184,7 +184,7 @@ __device__ __forceinline__ CircuitRun circuit_begin(const CircuitState &st, int 
   CircuitRun c;
   c.s = PixelRegs{st.receptor_log[k], st.reference_log[k], st.refractory_until[k], st.threshold_pos[k],
                   st.threshold_neg[k], st.reset_pending[k] != 0};
-  c.direct = p.reference_leak > 0;
+  c.direct = !(p.reference_leak == 0);
   c.follows = c.settled = false;
   c.inv_charge = 1.0 / p.charge_scale;
   if (!c.direct) {
