@@ -123,7 +123,7 @@ __device__ int advance_pixel(PixelRegs &s, const PixelParams &p, double rate, do
 // (CircuitState::receptor), so how cells are batched changes no bit.  A
 // reference that leaks, in either direction, moves the bounds in every cell and takes advance_pixel.
 
-// 1 - e^-k for 0 <= k < 0.35 by the Taylor series of (1 - e^-k) / k, whose first term left out is k^14 / 15! < 3e-19.
+// 1 - e^-k for |k| < 0.35 by the Taylor series of (1 - e^-k) / k, whose first term left out is k^14 / 15! < 4e-19.
 __device__ __forceinline__ double one_minus_exp_small(double k) {
   double s = 1.0 / 87178291200.0;  // 1 / 14!
   s = fma(-k, s, 1.0 / 6227020800.0);
@@ -148,18 +148,18 @@ __device__ __forceinline__ bool less_positive(double a, double b) {  // b > 0; a
 }
 __device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 // The receptor after dt at a constant rate.  Without photons it discharges, x / (1 + x dt / charge): the lanes of a dim
-// warp draw both, so the two cases share the division.
+// warp draw both, so the two cases share the division.  The charge, and k with it, may have either sign.
 __device__ __forceinline__ double receptor_step(double x, double rate, double dt, double inv_charge) {
   const double g = dt * inv_charge, k = rate * g;
   double a, b;
-  if (less_positive(k, 0.35)) {
+  if (less_positive(fabs(k), 0.35)) {
     b = one_minus_exp_small(k);
     a = 1.0 - b;
   } else {
     a = exp(-k);
     b = 1.0 - a;
   }
-  const bool light = positive(k);
+  const bool light = positive(rate);
   const double top = light ? rate : 1.0, rest = light ? a * rate : 1.0, share = light ? b : g;
   return x * top / fma(share, x, rest);
 }
