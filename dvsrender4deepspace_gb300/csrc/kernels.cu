@@ -141,8 +141,10 @@ __global__ void __launch_bounds__(128) philox_draws_kernel(int n, const Cell *ce
   if (i >= (long long)n * nc) return;
   const int c = (int)(i / n), r = (int)(i - (long long)c * n);
   const float rad = chunk[i];
-  if (!isfinite(rad)) return;  // the circuit reports it
   const Cell cell = cells[c0 + c];
+  // a radiance that is not finite stays for the circuit to report; a cell of no length draws nothing (its rate would be
+  // 0 / 0, which the circuit would report too), and the circuit passes over it
+  if (!isfinite(rad) || !(cell.dt > 0.0f)) return;
   chunk[i] = philox_rate(photo, rad * (float)photo.electrons_per_radiance + (float)photo.dark_electrons,
                          pixel_of_rank[r], cell);
 }
