@@ -73,6 +73,16 @@ void derive(const dvs_physic &c, bool effects, PixelParams &p, PhotoParams &phot
   }
 }
 
+// The power of two that a mesh's normals are stored with.  Only the direction of an interpolated normal counts, and a
+// power of two changes none of its bits; with the longest component near 2^59 neither short normals nor the products
+// of the interpolation leave the range of the kernels' roots (a squared length that is normal).  Normals whose
+// squares are zero or infinite in floats have no direction, as normalize has it.
+double normal_scaling(const float *normals, size_t n_vertices) {
+  float largest = 0;
+  for (size_t i = 0; i < 3 * n_vertices; ++i) largest = std::max(largest, std::fabs(normals[i]));
+  return largest * largest > 0 ? std::ldexp(1.0, std::max(0, 59 - std::ilogb(largest))) : 1.0;
+}
+
 float material_albedo(float value, float fallback) {  // device_optics.cuh:30-33
   return std::isfinite(value) && value >= 0 && value <= 1 ? value : fallback;
 }
@@ -520,6 +530,7 @@ int dvs_scene_create(const float *vertices, const float *normals, const uint32_t
   const size_t copies = watertight ? 3 : 1;
   std::vector<TriRecord> tris(n_triangles * copies);
   std::vector<ShadeRecord> shade(n_triangles);
+  const double normal_scale = normal_scaling(normals, n_vertices);
   const long long nt = (long long)n_triangles;
 #pragma omp parallel for schedule(static)
   for (long long i = 0; i < nt; ++i) {
@@ -545,9 +556,9 @@ int dvs_scene_create(const float *vertices, const float *normals, const uint32_t
     ShadeRecord &s = shade[i];
     std::memset(&s, 0, sizeof(s));
     for (int d = 0; d < 3; ++d) {
-      s.n0[d] = normals[3 * (size_t)a + d];
-      s.n1[d] = normals[3 * (size_t)b + d];
-      s.n2[d] = normals[3 * (size_t)c + d];
+      s.n0[d] = (float)(normals[3 * (size_t)a + d] * normal_scale);
+      s.n1[d] = (float)(normals[3 * (size_t)b + d] * normal_scale);
+      s.n2[d] = (float)(normals[3 * (size_t)c + d] * normal_scale);
     }
     if (albedos) {
       s.a0 = material_albedo(albedos[a], hapke->w);

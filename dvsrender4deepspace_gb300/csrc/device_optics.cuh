@@ -34,7 +34,8 @@ __device__ __forceinline__ float3 normalize(float3 v) {
   if (len > 0.0f) return v / len;
   return f3(0.0f, 0.0f, 0.0f);
 }
-// normalize in the forms of device_math.cuh (a zero vector stays zero).
+// normalize in the forms of device_math.cuh (a zero vector stays zero).  Not for vectors shorter than 2^-63, whose
+// squares are denormal: rays and lights are near 1, a scene's normals are stored long enough (normal_scaling).
 __device__ __forceinline__ float3 unit(float3 v) {
   const float len = sqrt_rn(dot(v, v));
   if (!(len > 0.0f)) return f3(0.0f, 0.0f, 0.0f);

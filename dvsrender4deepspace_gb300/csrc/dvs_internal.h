@@ -68,9 +68,9 @@ struct alignas(16) TriRecord {
 };
 static_assert(sizeof(TriRecord) == 48, "TriRecord layout");
 
-// Shading record in leaf order, 64 bytes: vertex normals and per-vertex
-// material albedo (already passed through the fallback rule of
-// include/dvs/device_optics.cuh:30-33), and the triangle's own unit normal,
+// Shading record in leaf order, 64 bytes: vertex normals (all of a scene's
+// times one power of two, normal_scaling), per-vertex material albedo (already
+// passed through the fallback rule of include/dvs/device_optics.cuh:30-33), and the triangle's own unit normal,
 // cross(e1, e2) normalized, which shadow_origin would form for every lit ray.
 struct alignas(16) ShadeRecord {
   float n0[3], a0;
