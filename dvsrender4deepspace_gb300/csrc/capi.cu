@@ -321,7 +321,6 @@ struct dvs_scene {
     v.cx = camera.cx;
     v.cy = camera.cy;
     v.coherent_span = coherent_span;
-    v.hapke = hapke;
     v.hc = hc;
     v.rays = 0;  // automatic
     return v;

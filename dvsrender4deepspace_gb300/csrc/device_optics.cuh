@@ -63,10 +63,12 @@ __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fm
 // tan(pi_f / 2) < 0, whose exp overflows and makes the sample NaN (dropped by
 // the caller's fmaxf) -- here tan(psi/2) = -inf there.
 __device__ __forceinline__ float pow15(float y) { return y * sqrt_rn(y); }
-__device__ __forceinline__ float hg_double_lobe(float cosg, float b, const HapkeConst &h) {
-  const float term1 = div_rn(h.lobe_pos, pow15(1.0f - 2.0f * b * cosg + b * b));
-  const float term2 = div_rn(h.lobe_neg, pow15(1.0f + 2.0f * b * cosg + b * b));
-  return term1 + term2;
+__device__ __forceinline__ float hg_double_lobe(float cosg, const HapkeConst &h) {
+  const float den1 = pow15(1.0f - 2.0f * h.b * cosg + h.b * h.b);
+  const float den2 = pow15(1.0f + 2.0f * h.b * cosg + h.b * h.b);
+  const float lobes = div_rn(h.lobe_pos, den1) + div_rn(h.lobe_neg, den2);
+  // a lobe so narrow that its denominator rounds to 0: the quotient by 0 that div_rn does not give
+  return fminf(den1, den2) == 0.0f ? h.lobe_zero : lobes;
 }
 __device__ __forceinline__ float b_s(float tg, float h, float inv_h) {
   if (h <= 0.0f) return tg <= 0.0f ? 1.0f : 0.0f;
@@ -93,25 +95,36 @@ __device__ __forceinline__ float porosity_k(float phi) {
   return -logf(1.0f - p) / p;
 }
 
-// The parts of hapke.hpp that depend on the material only, each the value
-// hapke.hpp recomputes inside every call (same operations, same rounding):
-// evaluated on the device once per scene (hapke_const_kernel) and read from the
-// view as constants.  Evaluated per pixel sample loop, two tanf, a powf and a
+// A material as the kernels read it.  The parts of hapke.hpp that depend on the
+// material only are each the value hapke.hpp recomputes inside every call (same
+// operations, same rounding; divisors brought into div_by's range): evaluated on
+// the device once per scene (hapke_const_kernel) and read from the view as constants.  Evaluated per pixel sample loop, two tanf, a powf and a
 // logf were a sixth of a one-ray loop.
 __device__ __forceinline__ HapkeConst hapke_const(const dvs_hapke &p) {
   HapkeConst h;
+  h.w = p.w;
+  h.hC = p.hC;
+  h.B_S0 = p.B_S0;
+  h.B_C0 = p.B_C0;
   h.K = porosity_k(p.phi);
-  h.inv_K = 1.0f / h.K;
+  h.K_div = isinf(h.K) ? 1e30f : h.K;  // the H-functions' argument is as good as 0 either way
+  h.inv_K = 1.0f / h.K_div;
   h.rough = !(p.thetap <= 1e-8f);
   h.tan_t = tanf(p.thetap);
   h.cot_t = 1.0f / h.tan_t;
   h.chi = 1.0f / sqrtf(1.0f + kPi * h.tan_t * h.tan_t);
   h.r0_w = hfunc_r0(p.w);
   h.tg_max = tanf(kPi / 2.0f - 1e-6f);
+  // beyond |b| = 1e12, where the denominators leave the float range, the lobes are as good as 0
+  const bool lobes = !(fabsf(p.b) > 1e12f);
+  h.b = lobes ? p.b : 0.0f;
   const float one_minus_bb = 1.0f - p.b * p.b;
-  h.lobe_pos = ((1.0f + p.c) * 0.5f) * one_minus_bb;
-  h.lobe_neg = ((1.0f - p.c) * 0.5f) * one_minus_bb;
-  h.inv_hS = 1.0f / p.hS;
+  h.lobe_pos = lobes ? ((1.0f + p.c) * 0.5f) * one_minus_bb : 0.0f;
+  h.lobe_neg = lobes ? ((1.0f - p.c) * 0.5f) * one_minus_bb : 0.0f;
+  h.lobe_zero = (p.b > 0.0f ? h.lobe_pos : h.lobe_neg) * kInf();
+  // narrower than 1e-30 the surge is below 1e-26 off the exact opposition and 1 at it, as here
+  h.hS = p.hS > 0.0f && p.hS < 1e-30f ? 1e-30f : p.hS;
+  h.inv_hS = 1.0f / h.hS;
   return h;
 }
 // The quotient q = cot(thetap) cos(y) / max(sin(y), 1e-6) shared by e1 and e2.
@@ -128,10 +141,13 @@ __device__ __forceinline__ float e_quot(float cot_t, float cosy, float siny) {
 // hapke_reflectance (hapke.hpp:131-152) in the identity form above; r0 is
 // hfunc's r0 for this albedo.  Quotients with a divisor in common share its
 // reciprocal, and constant divisors have theirs beforehand.  The divisors are
-// positive (2 - e1 >= 1, the shadowing denominators at least 1e-6) or end in a
-// NaN or infinite sample as with /, which the caller's fmaxf drops.
+// normal: 2 - e1 >= 1, the shadowing denominators and sines at least 1e-6, the
+// material's own brought into range (hapke_const), the lobes' checked
+// (hg_double_lobe); 1 + cos g and 1 + cos psi are 0 or at least 6e-8, with the
+// 0 noted at its use.  A NaN sample (the azimuth's above) is dropped by the
+// caller's fmaxf; an infinite one is not, and makes the call report it.
 DVS_SHADE_INLINE __device__ float hapke_reflectance(float cosi, float cose, float cosg, float albedo, float r0,
-                                                    const dvs_hapke &p, const HapkeConst &h) {
+                                                    const HapkeConst &h) {
   if (cosi <= 0 || cose <= 0) return 0;
   cosi = clampf(cosi, 0, 1);
   cose = clampf(cose, 0, 1);
@@ -140,11 +156,11 @@ DVS_SHADE_INLINE __device__ float hapke_reflectance(float cosi, float cose, floa
   const float tg = fminf(sqrt_rn(div_rn(1.0f - cosg, 1.0f + cosg)), h.tg_max);  // cos g = -1: NaN, and fminf takes tg_max
   const float cpsi = clampf(div_rn(cosg - cosi * cose, sini * sine + 1e-6f), -1.0f, 1.0f);
   const float psi = acosf(cpsi);
-  const float p_g = hg_double_lobe(cosg, p.b, h);
-  const float BS = b_s(tg, p.hS, h.inv_hS);
+  const float p_g = hg_double_lobe(cosg, h);
+  const float BS = b_s(tg, h.hS, h.inv_hS);
   // b_c is finite, so with B_C0 == 0 the factor (1 + BC * B_C0) is exactly 1
   // whatever BC is: skip its evaluation.
-  const float BC = p.B_C0 != 0.0f ? b_c(tg, p.hC) : 0.0f;
+  const float BC = h.B_C0 != 0.0f ? b_c(tg, h.hC) : 0.0f;
   const float K = h.K;
   float mu0, mue, S;
   if (!h.rough) {
@@ -178,10 +194,10 @@ DVS_SHADE_INLINE __device__ float hapke_reflectance(float cosi, float cose, floa
     const float shadowed = low ? div_by(cosi, eta_i, yi) : div_rn(cose, eta_e);
     S = div_rn(f, 1.0f - fp + fp * ch * shadowed);
   }
-  const float M = hfunc(div_by(mu0, K, h.inv_K), albedo, r0) * hfunc(div_by(mue, K, h.inv_K), albedo, r0) - 1.0f;
+  const float M = hfunc(div_by(mu0, h.K_div, h.inv_K), albedo, r0) * hfunc(div_by(mue, h.K_div, h.inv_K), albedo, r0) - 1.0f;
   const float LS = div_rn(mu0, mu0 + mue + 1e-6f);
-  return div_by(albedo, 4.0f * kPi, 1.0f / (4.0f * kPi)) * LS * K * (p_g * (1.0f + BS * p.B_S0) + M) *
-         (1.0f + BC * p.B_C0) * S;
+  return div_by(albedo, 4.0f * kPi, 1.0f / (4.0f * kPi)) * LS * K * (p_g * (1.0f + BS * h.B_S0) + M) *
+         (1.0f + BC * h.B_C0) * S;
 }
 
 // ---- pose interpolation (include/dvs/device_optics.cuh:6-29) ---------------------
@@ -1378,7 +1394,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
       lit[r] = false;
       normal[r] = f3(0, 0, 0);
       sorigin[r] = f3(0, 0, 0);
-      albedo[r] = S.hapke.w;
+      albedo[r] = S.hc.w;
       r0[r] = hc.r0_w;
       self[r] = hit[r].tri;
       if (hitp) {
@@ -1434,7 +1450,7 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
           if (lit[r] && !((occluded >> r) & 1u)) {
             const double cos4 = subrays ? subrays[j + r].cos4 : cos4_of(px[r], py[r]);
             const float3 n = unit(normal[r]), l = lnorm, v = unit(-ray[r]);
-            const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], S.hapke, hc);
+            const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], hc);
             out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
           }
         }
@@ -1480,7 +1496,7 @@ __device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, fl
   out.t = hit[0].t;
   if (kMode == kDepthOnly) return out;
   float3 normal = f3(0, 0, 0), sorigin[1] = {f3(0, 0, 0)};
-  float albedo = S.hapke.w, r0 = S.hc.r0_w;
+  float albedo = S.hc.w, r0 = S.hc.r0_w;
   if (out.hit) {
     const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[0].tri);
     const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
@@ -1507,7 +1523,7 @@ __device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, fl
     occluded = shadow_general<1, kGeo>(S, ShadowRays<1>{{sorigin[0]}, light, {self[0]}, {out.lit}}, stack_code, stack_t);
   if (out.lit && !occluded) {
     const float3 n = unit(normal), l = unit(light), v = unit(-ray[0]);
-    const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo, r0, S.hapke, S.hc);
+    const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo, r0, S.hc);
     out.term = fmaxf(0, n_h * pose.intensity) * cos4_of(px, py);
   }
   return out;

@@ -8,14 +8,17 @@
 
 namespace dvsgb {
 
-// Material constants of the Hapke model, formed on the device once per scene (launch_hapke_const).
+// A material as the kernels read it, formed on the device once per scene (launch_hapke_const).
 struct HapkeConst {
-  float K, inv_K;            // porosity factor and its reciprocal
+  float w, hC, B_S0, B_C0;   // as dvs_hapke
+  float K, K_div, inv_K;     // porosity factor, itself as a divisor (finite) and that one's reciprocal
   float tan_t, cot_t, chi;   // mean slope thetap: tan, cot and chi(thetap)
   float r0_w;                // the H-function's r0 at the scene's single-scattering albedo
   float tg_max;              // cap of tan(phase / 2)
-  float lobe_pos, lobe_neg;  // numerators of the two Henyey-Greenstein lobes
-  float inv_hS;              // 1 / hS
+  float b;                   // asymmetry of the two Henyey-Greenstein lobes
+  float lobe_pos, lobe_neg;  // their numerators
+  float lobe_zero;           // their sum where a denominator rounds to 0
+  float hS, inv_hS;          // width of the opposition surge as a divisor (0 or at least 1e-30) and its reciprocal
   int32_t rough;             // thetap > 1e-8
 };
 struct SceneView {
@@ -28,7 +31,6 @@ struct SceneView {
   int32_t width, height, samples, has_albedo;
   float fx, fy, cx, cy;
   float coherent_span;  // largest origin spread a warp packet traverses as one interval bundle
-  dvs_hapke hapke;
   HapkeConst hc;
   int32_t rays;         // sub-rays a lane may carry: 1, 2 or 4 (used when samples^2 is a multiple), 0 = automatic
   int32_t radiance_f32; // 1: the radiance chunk is written as float (read by an FP32 circuit), 0: as double
@@ -170,7 +172,7 @@ struct TraceJob {
   ItemShape shape;
 };
 // A trace launch's whole job table, passed as the kernel's parameter block
-// (24.6 KB at 128 jobs, within the 32 KB parameter limit).
+// (29.0 KB at 128 jobs, within the 32 KB parameter limit).
 struct TraceJobs {
   TraceJob jobs[kMaxBatchJobs];
   long long total_items;

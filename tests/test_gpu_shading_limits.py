@@ -39,3 +39,51 @@ def test_short_normals_keep_their_direction(ground, ss):
         g, w = g(), w()
         assert (w > 0).mean() > 0.5
         np.testing.assert_allclose(g, w, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("width", [1e-33, 1e-36, 1e-39, 1e-44])
+def test_opposition_surge_of_no_width(ground, width):
+    """The surge 1 / (1 + tan(g/2) / hS) is below 1e-15 for every ray of this view at hS = 1e-20 and below."""
+    V, N, I = ground
+    base = DeviceScene(V, N, I, CAM, 2, dict(HAPKE, hS=1e-20))
+    for g, w in zip(renders(base.view(CAM, 2, dict(HAPKE, hS=width))), renders(base)):
+        w = w()
+        assert (w > 0).mean() > 0.5
+        np.testing.assert_array_equal(g(), w)
+
+
+def test_infinite_porosity_factor_is_reported(ground):
+    """K = -log(1 - p) / p is infinite where p = 1.209 phi^(2/3) rounds to 1:
+    lit samples are then infinite, and the call reports them as before."""
+    V, N, I = ground
+    base = DeviceScene(V, N, I, CAM, 1, HAPKE)
+    phi, reported = np.float32((1.0 / 1.209) ** 1.5), 0
+    for _ in range(8):
+        phi = np.nextafter(phi, np.float32(0))
+    for _ in range(17):
+        errors = 0
+        for render in renders(base.view(CAM, 1, dict(HAPKE, phi=float(phi)))):
+            try:
+                render()
+            except OpticalError:
+                errors += 1
+        assert errors in (0, 2)
+        reported += errors == 2
+        phi = np.nextafter(phi, np.float32(1))
+    assert reported > 0
+
+
+def test_lobe_without_width_is_reported():
+    """b = 1 - 2^-13: at opposition (sun behind the camera, nadir pixel)
+    1 - 2 b + b^2 rounds to 0 in floats, and the forward lobe is infinite."""
+    V = np.array([[-100, -100, 0], [100, -100, 0], [100, 100, 0], [-100, 100, 0]], np.float32)
+    N = np.tile(np.float32([0, 0, 1]), (4, 1))
+    I = np.array([[0, 1, 2], [0, 2, 3]], np.uint32)
+    cam = dict(width=3, height=3, fx=10.0, fy=10.0, cx=1.0, cy=1.0)  # one ray a pixel: the middle one looks along -z
+    pose = dict(position=(1.0, 2.0, 10.0), rotation=(0, 0, 0, 1), light=(0, 0, 1), intensity=1000)
+    b = np.float32(1.0 - 2.0 ** -13)
+    assert np.float32(np.float32(1) - np.float32(2) * b) + b * b == 0
+    scene = DeviceScene(V, N, I, cam, 1, dict(HAPKE, b=float(b), c=0.5, thetap=0.0))
+    for render in renders(scene, pose):
+        with pytest.raises(OpticalError):
+            render()
