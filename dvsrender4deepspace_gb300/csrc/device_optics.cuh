@@ -339,7 +339,7 @@ __device__ __forceinline__ bool intersect_wt(const WtRay &w, float3 o, float3 v0
   const float det = U + V + W;
   if (det == 0.0f) return false;
   const float T = U * (w.sz * az) + V * (w.sz * bz) + W * (w.sz * cz);
-  const float rcp = rcp_rn(det);  // beyond the float range: NaN, a miss
+  const float rcp = rcp_small(det);  // the smallest triangles' is denormal; beyond the float range: a miss
   t = T * rcp;
   if (!(t > kRayEps)) return false;
   u = V * rcp;
