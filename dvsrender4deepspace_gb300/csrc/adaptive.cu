@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(128, 4)
       const double estimate = (left + right) * .5 * photo.electrons_per_radiance + photo.dark_electrons;
       const double leaf_duration = (b - a) * (end - start);
       // |u(actual) - u(estimate)| from the receptors themselves: one log for both
-      const double voltage_error = fabs(log(receptor_step(x0, fmax(0.0, actual), leaf_duration, inv_charge) /
-                                            receptor_step(x0, fmax(0.0, estimate), leaf_duration, inv_charge)));
+      const double voltage_error = fabs(log(receptor_step(x0, fmax(0.0, actual), leaf_duration * inv_charge) /
+                                            receptor_step(x0, fmax(0.0, estimate), leaf_duration * inv_charge)));
       bool smooth = voltage_error <= budget;
       if (smooth && !(fmax(actual, estimate) * leaf_duration < 1.0))
         smooth = fabs(log(fmax(1e-30, actual) / fmax(1e-30, estimate))) <= tolerance;
@@ -354,7 +354,10 @@ __global__ void __launch_bounds__(128) sample_exact_kernel(const __grid_constant
 }
 
 // integrate_optical_knots (event_sensor.cu:88-114): every native cell from the
-// knots (or its exactly traced radiance); events carry no depth.
+// knots (or its exactly traced radiance); events carry no depth.  Bound by the
+// FP64 pipe: the cells' window fractions, the same for every pixel, are
+// formed 32 at a time, shared out over the lanes (in every thread, with its quotient by the
+// window, they made 120 x 90 pixels x 200 horizons of 10 us 67.1 ms instead of 62.5).
 __global__ void __launch_bounds__(128) integrate_knots_kernel(int n, const Cell *cells, int n_cells, double start,
                                                               double end, const OpticalKnot *knots,
                                                               const int32_t *knot_counts, int capacity,
@@ -363,8 +366,13 @@ __global__ void __launch_bounds__(128) integrate_knots_kernel(int n, const Cell 
                                                               PhotoParams photo, int max_events, CircuitState st,
                                                               int32_t *ev_count, double *slab_t, int8_t *slab_p,
                                                               int32_t *error) {
-  const int rank = blockIdx.x * blockDim.x + threadIdx.x;
-  if (rank >= n || knot_counts[rank] < 0) return;
+  __shared__ double s_fraction[4][32];
+  double *fractions = s_fraction[threadIdx.x >> 5];
+  const int rank = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const bool mine = rank < n && knot_counts[rank] >= 0;
+  const unsigned team = __ballot_sync(kFull, mine);  // the lanes with a pixel
+  if (!mine) return;
+  const int member = __popc(team & ((1u << lane) - 1u)), members = __popc(team);
   const OpticalKnot *values = knots + (size_t)rank * capacity;
   const int size = knot_counts[rank];
   const int n_exact = exact_counts ? exact_counts[rank] : 0;
@@ -375,31 +383,39 @@ __global__ void __launch_bounds__(128) integrate_knots_kernel(int n, const Cell 
   double *my_t = slab_t + (size_t)rank * max_events;
   int8_t *my_p = slab_p + (size_t)rank * max_events;
   int a = 0, exact_index = 0, count = 0, failed = 0;
-  // the segment [a, a + 1] of the knots: its left end and light, and the light's slope over the window fraction
+  // the segment [a, a + 1] of the knots: its left end and light, its length and the light's change over it
   double left = segment_fraction(values, 0), right = segment_fraction(values, 1);
-  double from = values[0].radiance, slope = (values[1].radiance - from) / (right - left);
-  const double inv_window = 1.0 / (end - start);
-  for (int c = 0; c < n_cells; ++c) {
-    const Cell cell = cells[c];
-    const double t0 = cell.t0, t1 = cell.t1;
-    const double fraction = ((t0 + t1) * .5 - start) * inv_window;
-    if (a + 2 < size && fraction > right) {
-      do {
-        ++a;
-        right = segment_fraction(values, a + 1);
-      } while (a + 2 < size && fraction > right);
-      left = segment_fraction(values, a);
-      from = values[a].radiance;
-      slope = (values[a + 1].radiance - from) / (right - left);
+  double from = values[0].radiance, change = values[1].radiance - from;
+  double length = right - left, inv_length = 1.0 / length;
+  for (int c0 = 0; c0 < n_cells; c0 += 32) {
+    const int tile = min(32, n_cells - c0);
+    for (int i = member; i < tile; i += members)
+      fractions[i] = ((cells[c0 + i].t0 + cells[c0 + i].t1) * .5 - start) / (end - start);
+    __syncwarp(team);
+    for (int c = c0; !failed && c < c0 + tile; ++c) {
+      const Cell cell = cells[c];
+      const double fraction = fractions[c - c0];
+      if (a + 2 < size && fraction > right) {
+        do {
+          ++a;
+          right = segment_fraction(values, a + 1);
+        } while (a + 2 < size && fraction > right);
+        left = segment_fraction(values, a);
+        from = values[a].radiance;
+        change = values[a + 1].radiance - from;
+        length = right - left;
+        inv_length = 1.0 / length;
+      }
+      double light = from + change * quotient(fraction - left, length, inv_length);
+      if (exact_index < n_exact && my_exact[exact_index] == c) light = my_exact_rad[exact_index++];
+      double rate = (positive(light) ? light : 0.0) * photo.electrons_per_radiance + photo.dark_electrons;
+      if (photo.shot_noise) rate = quotient(poisson_electrons(rng, rate * cell.len), cell.len, cell.inv_len);
+      const int emitted = circuit_cell(run, p, rate, cell, my_t + count, my_p + count, max_events - count, rng);
+      if (emitted == -1) failed = kErrCapacity;
+      else if (emitted == -2) failed = kErrStalled;
+      else count += emitted;
     }
-    double light = from + slope * (fraction - left);
-    if (exact_index < n_exact && my_exact[exact_index] == c) light = my_exact_rad[exact_index++];
-    double rate = (positive(light) ? light : 0.0) * photo.electrons_per_radiance + photo.dark_electrons;
-    if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
-    const int emitted = circuit_cell(run, p, rate, t0, t1, my_t + count, my_p + count, max_events - count, rng);
-    if (emitted == -1) { failed = kErrCapacity; break; }
-    if (emitted == -2) { failed = kErrStalled; break; }
-    count += emitted;
+    __syncwarp(team);
   }
   circuit_end(run, st, rank);
   st.rng[rank] = rng;

@@ -1103,6 +1103,7 @@ static int stage_batch(dvs_sensor *s, const dvs_optical_interval *ivs, size_t co
   for (size_t i = 0; i < count; ++i) n_cells += (size_t)std::ceil((ivs[i].t1 - ivs[i].t0) / s->photo.integration_step);
   CUDA_TRY(grow_pinned(s->h_cells, s->h_cells_cap, n_cells, &s->pinned), "cell staging");
   CUDA_TRY(grow_pinned(s->h_ivs, s->h_ivs_cap, count, &s->pinned), "interval staging");
+  const double inv_charge = 1.0 / s->p.charge_scale;
   size_t c = 0;
   for (size_t i = 0; i < count; ++i) {
     const dvs_optical_interval &iv = ivs[i];
@@ -1113,8 +1114,10 @@ static int stage_batch(dvs_sensor *s, const dvs_optical_interval *ivs, size_t co
       cell.t0 = iv.t0 + step * dt;
       cell.t1 = step + 1 == steps ? iv.t1 : iv.t0 + (step + 1) * dt;
       cell.interval = (int32_t)i;
-      cell.dt = (float)(cell.t1 - cell.t0);
-      cell.inv_len = 1.0 / (cell.t1 - cell.t0);
+      cell.len = cell.t1 - cell.t0;
+      cell.inv_len = 1.0 / cell.len;
+      cell.g = cell.len * inv_charge;
+      cell.dt = (float)cell.len;
     }
   }
   std::memcpy(s->h_ivs, ivs, sizeof(dvs_optical_interval) * count);

@@ -149,8 +149,9 @@ __device__ __forceinline__ bool less_positive(double a, double b) {  // b > 0; a
 __device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 // The receptor after dt at a constant rate.  Without photons it discharges, x / (1 + x dt / charge): the lanes of a dim
 // warp draw both, so the two cases share the division.  The charge, and k with it, may have either sign.
-__device__ __forceinline__ double receptor_step(double x, double rate, double dt, double inv_charge) {
-  const double g = dt * inv_charge, k = rate * g;
+// g: dt / charge.
+__device__ __forceinline__ double receptor_step(double x, double rate, double g) {
+  const double k = rate * g;
   double a, b;
   if (less_positive(fabs(k), 0.35)) {
     b = one_minus_exp_small(k);
@@ -167,7 +168,6 @@ __device__ __forceinline__ double receptor_step(double x, double rate, double dt
 struct CircuitRun {
   PixelRegs s;
   double x, high, low;  // receptor and the comparator's bounds on it
-  double inv_charge;
   bool direct;    // a reference that leaks, up or down: advance_pixel for every cell
   bool follows;   // the reference is the receptor's log, not yet written down
   bool settled;   // past the refractory deadline, nothing pending, the receptor between the bounds
@@ -186,7 +186,6 @@ __device__ __forceinline__ CircuitRun circuit_begin(const CircuitState &st, int 
                   st.threshold_neg[k], st.reset_pending[k] != 0};
   c.direct = !(p.reference_leak == 0);
   c.follows = c.settled = false;
-  c.inv_charge = 1.0 / p.charge_scale;
   if (!c.direct) {
     c.x = st.receptor[k];
     if (!(log(c.x) == c.s.receptor_log)) c.x = exp(c.s.receptor_log);  // written by another circuit
@@ -216,16 +215,17 @@ __device__ __noinline__ EventCell circuit_event_cell(EventCell e, PixelParams p,
   }
   return e;
 }
-__device__ __forceinline__ int circuit_cell(CircuitRun &c, const PixelParams &p, double rate, double t0, double t1,
+__device__ __forceinline__ int circuit_cell(CircuitRun &c, const PixelParams &p, double rate, const Cell &cell,
                                             double *out_t, int8_t *out_p, int capacity, curandStateXORWOW_t &rng) {
-  if (!c.direct && t0 < t1) {
+  const double t0 = cell.t0, t1 = cell.t1;
+  if (!c.direct && positive(cell.len)) {
     bool refractory = false;
     if (!c.settled) {  // a quiet cell leaves the pixel settled: its deadline stays behind it
       refractory = t1 < c.s.refractory_until;
       c.settled = t0 >= c.s.refractory_until && !c.s.reset_pending && between(c.low, c.x, c.high);
     }
     if (refractory || c.settled) {
-      const double y = receptor_step(c.x, rate, t1 - t0, c.inv_charge);
+      const double y = receptor_step(c.x, rate, cell.g);
       if (refractory || between(c.low, y, c.high)) {
         c.x = y;
         c.follows = refractory;

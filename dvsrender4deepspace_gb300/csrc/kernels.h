@@ -47,7 +47,8 @@ struct alignas(16) CellPose {
 // One circuit integration cell (event_sensor.cu:37-40): [t0, t1) of interval.
 struct alignas(16) Cell {
   double t0, t1;
-  double inv_len;  // 1 / (t1 - t0), formed once on the host: a photon count's rate without a division per pixel
+  // t1 - t0, its reciprocal and its quotient by the charge scale, formed once on the host: nothing of them per pixel
+  double len, inv_len, g;
   int32_t interval;
   float dt;  // (float)(t1 - t0), rounded once on the host: the FP32 circuit's cell length
 };

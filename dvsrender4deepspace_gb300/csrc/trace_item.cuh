@@ -278,9 +278,8 @@ __device__ __forceinline__ void circuit_rank(int r, int n, const int32_t *rank_l
       const double rad = radiance[(size_t)c * n + r];
       if (!finite_bits(rad)) { failed = kErrOptical; break; }
       double rate = rad * photo.electrons_per_radiance + photo.dark_electrons;
-      const double t0 = cell.t0, t1 = cell.t1;
-      if (photo.shot_noise) rate = poisson_electrons(rng, rate * (t1 - t0)) * cell.inv_len;
-      const int emitted = circuit_cell(run, p, rate, t0, t1, my_t + cnt, my_p + cnt, max_events - cnt, rng);
+      if (photo.shot_noise) rate = quotient(poisson_electrons(rng, rate * cell.len), cell.len, cell.inv_len);
+      const int emitted = circuit_cell(run, p, rate, cell, my_t + cnt, my_p + cnt, max_events - cnt, rng);
       if (emitted == -1) { failed = kErrCapacity; break; }
       if (emitted == -2) { failed = kErrStalled; break; }
       cnt += emitted;

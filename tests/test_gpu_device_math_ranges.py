@@ -1,7 +1,9 @@
 """Reciprocals of the trace kernels (csrc/device_math.cuh) over the ranges they
 are used in: rcp_rn for every normal float up to 2^126, rcp_small for every one
 from 2^-128 to 2^124.  As test_gpu_device_math.py states, a result is the correctly
-rounded one or, rarely, its neighbour.  And the triangle that needs the latter:
+rounded one or, rarely, its neighbour.  The FP64 quotients by a divisor known
+beforehand: their own error before the last rounding is 2^-52 ulp, so none of
+2^26 pairs differs from the operator.  And the triangle that needs the latter:
 one so small that the watertight test's determinant is denormal is hit.
 """
 import os
@@ -28,6 +30,7 @@ def test_reciprocals_over_their_ranges(tmp_path):
         differ, worst = rows[f]
         assert worst <= 1 and differ <= n >> 19, (f, differ, worst)
     assert rows["beyond_finite"] == [0]
+    assert rows["quotient"] == [0] and rows["product"][0] > 1 << 20
 
 
 @pytest.mark.parametrize("size", [1e-3, 1e-12, 3e-20])
