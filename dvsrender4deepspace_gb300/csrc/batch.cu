@@ -127,23 +127,21 @@ ItemShape trace_item_shape(int n_pix, int nc, int cw_log2, int sub_rays, int ray
            (n_sets + 2 * s.sets - 1) / (2 * s.sets) * ((n_groups + s.groups - 1) / s.groups) >= kMinItems)
       s.sets *= 2;
   // fewer packets do not pay for the beam's own walks, and packets over more than four pixels (fewer than 8 cells) are
-  // themselves as wide as the beam
-  s.beam = cw_log2 >= 3 && s.sets * s.groups * packets >= kBeamPackets;
+  // themselves as wide as the beam; several rays per lane walk (trace_rays)
+  s.beam = rays == 1 && cw_log2 >= 3 && s.sets * s.groups * packets >= kBeamPackets;
   return s;
 }
 
-// Measured with beams: one ray per lane 93.6 ms against two 131 ms for an orbit batch (346x260, 16 sub-rays, 640
-// cells), 305 against 397 ms at 1280x720 (64 sub-rays, 64 cells): the beam leaves no node tests to share between a
-// lane's rays, and the second ray's code does not fit the instruction cache.  Without beams two per lane share them.
+// One ray per lane wherever items hold beams: 93.6 ms against two rays' 131 ms with beams and 117 ms without for an
+// orbit batch (346x260, 16 sub-rays, 640 cells), 305 against 397 ms at 1280x720 (64 sub-rays, 64 cells): the beam
+// leaves no node tests to share between a lane's rays, and the second ray's code does not fit the instruction cache.
+// Without beams two per lane share them, or what the sensor's tuning asks for.
 int trace_rays(const SceneView &view, int n_pix, int nc, int cw_log2, bool scattered) {
-  const int ss2 = view.samples * view.samples;
-  if (view.rays == 0) {
-    if (trace_item_shape(n_pix, nc, cw_log2, ss2, 1, scattered).beam) return 1;
-    return ss2 % 2 == 0 ? 2 : 1;
-  }
+  const int ss2 = view.samples * view.samples, most = view.rays ? view.rays : 2;
+  if (trace_item_shape(n_pix, nc, cw_log2, ss2, 1, scattered).beam) return 1;
   // four rays per lane only in the reference format (the others keep two)
-  if (view.geometry == kGeoReference && view.rays >= 4 && ss2 % 4 == 0) return 4;
-  return view.rays >= 2 && ss2 % 2 == 0 ? 2 : 1;
+  if (view.geometry == kGeoReference && most >= 4 && ss2 % 4 == 0) return 4;
+  return most >= 2 && ss2 % 2 == 0 ? 2 : 1;
 }
 
 long long trace_job_items(int n_pix, int nc, const ItemShape &s) {

@@ -377,26 +377,20 @@ void trace_list_geo(const SceneView &scene, int n_pix, const int32_t *rank_list,
   const int rays = trace_rays(scene, n_pix, nc, cw_log2, rank_list != nullptr);
   const ItemShape shape = trace_item_shape(n_pix, nc, cw_log2, ss2, rays, rank_list != nullptr);
   const int grid = blocks(trace_job_items(n_pix, nc, shape) * 32, 128);
-#define DVS_TRACE_LAUNCH(MODE, RAYS, DEPTH)                                                                         \
-  do {                                                                                                              \
-    if (shape.beam)                                                                                                 \
-      trace_cells_kernel<MODE, RAYS, kGeo, true><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc,       \
-                                                                      shape, radiance, DEPTH, counters);            \
-    else                                                                                                            \
-      trace_cells_kernel<MODE, RAYS, kGeo, false><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc,      \
-                                                                       shape, radiance, DEPTH, counters);           \
+#define DVS_TRACE_LAUNCH(MODE, RAYS, BEAM)                                                                        \
+  trace_cells_kernel<MODE, RAYS, kGeo, BEAM><<<grid, 128, 0, s>>>(scene, n_pix, rank_list, poses, c0, nc, shape, \
+                                                                  radiance, depth, counters)
+#define DVS_TRACE_MODE(MODE)                            \
+  do {                                                  \
+    if constexpr (kGeo == kGeoReference)                \
+      if (rays == 4) { DVS_TRACE_LAUNCH(MODE, 4, false); return; } \
+    if (rays == 2) DVS_TRACE_LAUNCH(MODE, 2, false);    \
+    else if (shape.beam) DVS_TRACE_LAUNCH(MODE, 1, true); \
+    else DVS_TRACE_LAUNCH(MODE, 1, false);              \
   } while (0)
-  if (depth) {
-    if constexpr (kGeo == kGeoReference)
-      if (rays == 4) { DVS_TRACE_LAUNCH(kRadianceDepth, 4, depth); return; }
-    if (rays == 2) DVS_TRACE_LAUNCH(kRadianceDepth, 2, depth);
-    else DVS_TRACE_LAUNCH(kRadianceDepth, 1, depth);
-  } else {
-    if constexpr (kGeo == kGeoReference)
-      if (rays == 4) { DVS_TRACE_LAUNCH(kRadiance, 4, nullptr); return; }
-    if (rays == 2) DVS_TRACE_LAUNCH(kRadiance, 2, nullptr);
-    else DVS_TRACE_LAUNCH(kRadiance, 1, nullptr);
-  }
+  if (depth) DVS_TRACE_MODE(kRadianceDepth);
+  else DVS_TRACE_MODE(kRadiance);
+#undef DVS_TRACE_MODE
 #undef DVS_TRACE_LAUNCH
 }
 }  // namespace
@@ -513,8 +507,10 @@ namespace {
 template <int kMode, int kRays, int kGeo>
 cudaError_t preload_cells() {
   cudaFuncAttributes a;
-  const cudaError_t e = cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, true>);
-  return e == cudaSuccess ? cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, false>) : e;
+  cudaError_t e = cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, false>);
+  if constexpr (kRays == 1)
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, trace_cells_kernel<kMode, kRays, kGeo, true>);
+  return e;
 }
 template <int kGeo>
 cudaError_t preload_camera_geo() {

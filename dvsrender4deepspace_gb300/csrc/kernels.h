@@ -32,7 +32,7 @@ struct SceneView {
   float fx, fy, cx, cy;
   float coherent_span;  // largest origin spread a warp packet traverses as one interval bundle
   HapkeConst hc;
-  int32_t rays;         // sub-rays a lane may carry: 1, 2 or 4 (used when samples^2 is a multiple), 0 = automatic
+  int32_t rays;         // sub-rays a lane carries at most: 1, 2 or 4 (trace_rays), 0 = automatic
   int32_t radiance_f32; // 1: the radiance chunk is written as float (read by an FP32 circuit), 0: as double
 };
 
@@ -195,8 +195,8 @@ struct CircuitJob {
   unsigned long long *counters;
   int32_t n, c0, nc, max_events, first_block, pad;
 };
-// The sub-rays per lane a trace of this view runs with: the view's, or automatically one where its items hold beams
-// and two (when the sub-ray count is even) where they do not.
+// The sub-rays per lane a trace of this view runs with: one where its items hold beams, else the view's (automatically
+// two) where the sub-ray count is a multiple.
 int trace_rays(const SceneView &view, int n_pix, int nc, int cw_log2, bool scattered);
 // The item shape of a trace of n_pix pixels (neighbours in rank order, or scattered ones) x nc cells, and its items.
 ItemShape trace_item_shape(int n_pix, int nc, int cw_log2, int sub_rays, int rays, bool scattered);

@@ -356,10 +356,12 @@ int dvs_device_readout_counters(const dvs_device_readout *readout, uint64_t *dro
 int dvs_device_readout_last_ms(const dvs_device_readout *readout, double *ms);
 
 /* Traversal packet shape: cells_per_warp 1..32 (power of two; 0 = automatic)
- * and rays_per_lane 1, 2 or 4 neighbouring sub-rays per lane, used when the
- * pixel's sub-ray count is a multiple of it.  Until this or the autotuner
- * sets one, each trace chooses: one where its warps' items are large enough to
- * share one walk of the tree, two otherwise.  Results do not depend on it. */
+ * and rays_per_lane, the most neighbouring sub-rays a lane carries: 1, 2 or 4,
+ * used when the pixel's sub-ray count is a multiple of it.  Traces whose warps'
+ * items are large enough to share one walk of the tree carry one.  Until this
+ * or the autotuner sets it, the others carry two.  Results do not depend on it,
+ * but for which of two triangles that a ray hits at the same distance (a common
+ * edge, a triangle that lies twice in the mesh) it takes. */
 int dvs_sensor_set_tuning(dvs_sensor *sensor, int32_t cells_per_warp, int32_t rays_per_lane);
 typedef struct {
   int32_t cells_per_warp, rays_per_lane;  /* the shape chosen and now set */
