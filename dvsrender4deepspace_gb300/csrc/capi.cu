@@ -1751,6 +1751,8 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
   // -- cells per warp 4..32, one or two sub-rays per lane -- and keeps the
   // fastest, then the circuit-step chunk (autotune_chunk).  No circuit
   // state, RNG or time changes, so the same batch is then processed as usual.
+  // A batch of so few cells that its trace is laid out by poses has no packet
+  // shape to time, and leaves the sensor's as it is.
   if (!out) return fail(DVS_ERR_INVALID, "null argument");
   if (s && s->pending) return fail(DVS_ERR_INVALID, "collect the enqueued batch before autotuning");
   size_t n_cells = 0;
@@ -1787,12 +1789,14 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
   float best = -1, def_ms = -1;
   const int default_rays = trace_rays(view, n_sub, nc, default_log2, true);
   int best_log2 = default_log2, best_rays = default_rays, tried = 0;
+  const bool by_pose = trace_by_pose(view, n, nc) || trace_by_pose(view, n_sub, nc);
   cudaError_t err = cudaSuccess;
-  for (int rays = 1; rays <= 4 && err == cudaSuccess; rays *= 2) {
+  for (int rays = 1; !by_pose && rays <= 4 && err == cudaSuccess; rays *= 2) {
     if (ss2 % rays) break;
     view.rays = rays;
     for (int lg = 2; lg <= 5 && err == cudaSuccess; ++lg) {
       if ((1 << lg) > nc && lg > 2) break;
+      if (trace_rays(view, n_sub, nc, lg, true) != rays) continue;  // runs as a candidate with fewer rays
       float ms = -1;
       for (int rep = 0; rep < 4 && err == cudaSuccess; ++rep) {  // the first launch warms caches
         float t = 0;
@@ -1824,8 +1828,11 @@ int dvs_sensor_autotune(dvs_sensor *s, const dvs_optical_interval *ivs, size_t c
     best_log2 = default_log2;
     best_rays = default_rays;
   }
-  s->opt.cells_per_warp = 1 << best_log2;
-  s->rays_per_lane = best_rays;
+  if (!by_pose) {
+    s->opt.cells_per_warp = 1 << best_log2;
+    // where the shape shares walks, one ray is what every tuning takes: nothing to hold other traces to
+    if (!trace_item_shape(n_sub, nc, best_log2, ss2, 1, true).beam) s->rays_per_lane = best_rays;
+  }
   out->cells_per_warp = 1 << best_log2;
   out->rays_per_lane = best_rays;
   out->candidates = tried;

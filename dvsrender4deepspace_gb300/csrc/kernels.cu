@@ -22,6 +22,7 @@
 //     and integrates the pixel circuit (pixel_model.hpp semantics).
 //   * emit_events: warp prefix-sum compaction of the per-pixel event slabs.
 //   * event_depth: depth re-trace at each event time, a warp per event (event_sensor.cu:51-59).
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 #include <cuda_runtime.h>
@@ -337,7 +338,6 @@ cudaError_t launch_cell_poses(const dvs_optical_interval *ivs, const Cell *cells
   return cudaGetLastError();
 }
 
-namespace {
 // Few poses: packets of sub-rays.  One sub-ray a pixel fills a packet with a block of 8 x 4 pixels; where so few pixels
 // leave the GPU idle, narrower packets on more warps.
 bool trace_by_pose(const SceneView &scene, int n_pix, int nc) {
@@ -348,17 +348,19 @@ PoseShape pose_item_shape(int n_pix, int nc, int ss2, bool scattered) {
   PoseShape s{1, 0, 0};
   while ((1 << s.lanes_log2) < ss2 && s.lanes_log2 < 5) ++s.lanes_log2;
   const int per_packet = 32 >> s.lanes_log2, runs = (ss2 + 31) / 32;
-  // pixels of an item: a packet's, then more for the beam while every SM has items
-  const int most = kPoseTerms / ((1 << s.lanes_log2) + 1);
+  // pixels of an item: a packet's, then more for the beam while every SM has items (scattered pixels share no beam)
+  const int most = std::min(32, kPoseTerms / ((1 << s.lanes_log2) + 1));
   const auto items = [&](int pixels) { return (long long)((n_pix + pixels - 1) / pixels) * nc; };
-  const int limit = scattered ? 1 : most < 32 ? most : 32;
+  const int limit = scattered ? per_packet : most;
   while (2 * s.pixels <= limit && items(2 * s.pixels) >= 2 * kResidentWarps && s.pixels * runs < 64 * per_packet)
     s.pixels *= 2;
   // one walk for the item pays from 8 packets on, or where the item is itself one narrow packet (the walk takes four
   // nodes at a time and sorts once: 160x120 frames with 4 sub-rays 0.29 -> 0.20 ms); 4 packets over 32 pixels lose 8 %
-  s.beam = s.pixels <= 4 || (s.pixels + per_packet - 1) / per_packet * runs >= 8;
+  s.beam = scattered ? s.pixels == 1 : s.pixels <= 4 || (s.pixels + per_packet - 1) / per_packet * runs >= 8;
   return s;
 }
+
+namespace {
 template <int kGeo>
 void trace_list_geo(const SceneView &scene, int n_pix, const int32_t *rank_list, const CellPose *poses, int c0, int nc,
                     int cw_log2, double *radiance, float *depth, unsigned long long *counters, cudaStream_t s) {

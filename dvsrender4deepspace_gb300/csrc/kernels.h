@@ -215,6 +215,10 @@ cudaError_t launch_circuit_jobs(const CircuitJob *jobs, int n_jobs, int total_bl
 struct PoseShape {
   int32_t pixels, lanes_log2, beam;
 };
+// Whether a trace of n_pix pixels x nc poses is laid out that way, whatever the cells per warp and rays per lane, and
+// its item shape.
+bool trace_by_pose(const SceneView &scene, int n_pix, int nc);
+PoseShape pose_item_shape(int n_pix, int nc, int ss2, bool scattered);
 cudaError_t launch_trace_cells(const SceneView &scene, int n_pix, const CellPose *poses, int c0, int nc,
                                int cw_log2, double *radiance, float *depth, unsigned long long *counters,
                                cudaStream_t s);

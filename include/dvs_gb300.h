@@ -375,7 +375,9 @@ typedef struct {
  * dvs_sensor_process/enqueue will be given next):
  *  1. packet shape: the trace of up to 64 circuit cells over a patch of up
  *     to 32768 pixels from the middle of the image, for each shape (cells per
- *     warp 4..32 x 1, 2 or 4 sub-rays per lane);
+ *     warp 4..32 x 1, 2 or 4 sub-rays per lane, where they differ).  Batches
+ *     of fewer than 8 cells are mostly traced without packets of cells: no
+ *     candidates then, times of -1, and the sensor's shape stays as it is;
  *  2. circuit-step chunking: the whole optics -> circuit pipeline of every
  *     pixel with the chosen shape over as many cells as the batch's default
  *     chunk (at least 64, at most the batch), for chunks of 1, 1/2, 1/4 and

@@ -36,6 +36,25 @@ int main() {
                             walk[4] != (ss2 % 4 == 0 && geometry == 0 ? 4 : walk[2])))
                 ++broken;
             }
+  // items of a trace by poses fill their packets where there are items enough for the GPU; scattered pixels, whose beam
+  // would be too wide, hold just one packet and share none
+  long poses = 0;
+  for (int samples : {1, 2, 3, 4, 5, 6, 8, 16})
+    for (int n_pix : {1, 31, 1024, 89960, 921600})
+      for (int nc = 1; nc < 8; ++nc)
+        for (bool scattered : {false, true}) {
+          SceneView v{};
+          v.samples = samples;
+          if (!trace_by_pose(v, n_pix, nc)) continue;
+          ++poses;
+          const PoseShape s = pose_item_shape(n_pix, nc, samples * samples, scattered);
+          const int per_packet = 32 >> s.lanes_log2;
+          const bool many = (long long)n_pix * nc >= 32 * 4864;
+          if (s.pixels < 1 || s.pixels > 32 || (many && s.pixels < per_packet) ||
+              (scattered && (s.pixels > per_packet || (s.beam && s.pixels > 1))))
+            ++broken;
+        }
+  if (!poses) ++broken;
   std::printf("traces %ld\nbeams %ld\nbroken %ld\n", traces, beams, broken);
   return 0;
 }
