@@ -687,6 +687,7 @@ constexpr int kClusterBlocks = 8;  // the portable cluster size
 constexpr int kBlockEvents = 512;
 __device__ __forceinline__ void cluster_barrier() {
   __threadfence();
+  __syncwarp();  // the aligned forms want the whole warp, and phases leave lanes behind that did the serial part
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 struct SortKey {
