@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(128, 4)
         const int q = min(q0 + lane, total - 1), k = q / m, r = r0 + q - k * m;
         const bool live = q0 + lane < total;
         const CellPose pose = sh.pose[k];
-        const RaySample s = sample_ray<kRadiance, kGeo, true>(S, subray_x(S, px_i, r % S.samples),
-                                                              subray_y(S, py_i, r / S.samples), pose, live, sh.code,
-                                                              sh.t, sh.beam, lists);
+        const RaySample s = sample_ray<kGeo, true>(S, subray_x(S, px_i, r % S.samples),
+                                                   subray_y(S, py_i, r / S.samples), pose, live, sh.code,
+                                                   sh.t, sh.beam, lists);
         if (live) {
           sh.term[k][q - k * m] = s.term;
           sh.traced[k][q - k * m] = (unsigned char)((s.lit ? 2 : 1) | (s.overflow ? kProbeBad : 0));

@@ -551,7 +551,7 @@ struct PixelSample {
 };
 
 // What one pixel sample produces.
-enum SampleMode : int { kRadiance = 0, kRadianceDepth = 1, kDepthOnly = 2 };
+enum SampleMode : int { kRadiance = 0, kRadianceDepth = 1 };
 
 // cos^4 field falloff (device_optics.cuh:90) in FP64, as the reference.
 __device__ __forceinline__ double cos4_of(float px, float py) {
@@ -586,6 +586,18 @@ __device__ __forceinline__ void wrange(float lo, float hi, bool active, float &w
   whi = funord(__reduce_max_sync(kFull, active ? ford(hi) : 0x007fffffu));
 }
 
+// The interval bundle of given ranges; coherent means each axis' inverse direction keeps one sign.
+__device__ __forceinline__ Packet range_packet(float3 olo, float3 ohi, float3 ilo, float3 ihi) {
+  Packet P;
+  P.olo = olo; P.ohi = ohi; P.ilo = ilo; P.ihi = ihi;
+  P.nx = ihi.x < 0.0f;
+  P.ny = ihi.y < 0.0f;
+  P.nz = ihi.z < 0.0f;
+  P.coherent = (P.nx || ilo.x > 0.0f) && (P.ny || ilo.y > 0.0f) && (P.nz || ilo.z > 0.0f);
+  P.o_near = f3(P.nx ? olo.x : ohi.x, P.ny ? olo.y : ohi.y, P.nz ? olo.z : ohi.z);
+  P.o_far = f3(P.nx ? ohi.x : olo.x, P.ny ? ohi.y : olo.y, P.nz ? ohi.z : olo.z);
+  return P;
+}
 template <int R>
 __device__ Packet make_packet_r(const SceneView &S, const float3 (&o)[R], const float3 (&d)[R],
                                 const float3 (&idir)[R], const bool (&active)[R]) {
@@ -602,13 +614,12 @@ __device__ Packet make_packet_r(const SceneView &S, const float3 (&o)[R], const 
       dlo = f3(fminf(dlo.x, d[r].x), fminf(dlo.y, d[r].y), fminf(dlo.z, d[r].z));
       dhi = f3(fmaxf(dhi.x, d[r].x), fmaxf(dhi.y, d[r].y), fmaxf(dhi.z, d[r].z));
     }
-  Packet P;
-  wrange(olo.x, ohi.x, any, P.olo.x, P.ohi.x);
-  wrange(olo.y, ohi.y, any, P.olo.y, P.ohi.y);
-  wrange(olo.z, ohi.z, any, P.olo.z, P.ohi.z);
-  wrange(ilo.x, ihi.x, any, P.ilo.x, P.ihi.x);
-  wrange(ilo.y, ihi.y, any, P.ilo.y, P.ihi.y);
-  wrange(ilo.z, ihi.z, any, P.ilo.z, P.ihi.z);
+  wrange(olo.x, ohi.x, any, olo.x, ohi.x);
+  wrange(olo.y, ohi.y, any, olo.y, ohi.y);
+  wrange(olo.z, ohi.z, any, olo.z, ohi.z);
+  wrange(ilo.x, ihi.x, any, ilo.x, ihi.x);
+  wrange(ilo.y, ihi.y, any, ilo.y, ihi.y);
+  wrange(ilo.z, ihi.z, any, ilo.z, ihi.z);
   float wl, wh;
   wrange(dlo.x, dhi.x, any, wl, wh);
   const float dx = wh - wl;
@@ -617,14 +628,9 @@ __device__ Packet make_packet_r(const SceneView &S, const float3 (&o)[R], const 
   wrange(dlo.z, dhi.z, any, wl, wh);
   const float dz = wh - wl;
   const float ds = fmaxf(fmaxf(dx, dy), dz);
-  const float os = fmaxf(fmaxf(P.ohi.x - P.olo.x, P.ohi.y - P.olo.y), P.ohi.z - P.olo.z);
-  P.nx = P.ihi.x < 0.0f;
-  P.ny = P.ihi.y < 0.0f;
-  P.nz = P.ihi.z < 0.0f;
-  const bool one_sign = (P.nx || P.ilo.x > 0.0f) && (P.ny || P.ilo.y > 0.0f) && (P.nz || P.ilo.z > 0.0f);
-  P.coherent = one_sign && ds <= kCoherentSpread && os <= S.coherent_span;
-  P.o_near = f3(P.nx ? P.olo.x : P.ohi.x, P.ny ? P.olo.y : P.ohi.y, P.nz ? P.olo.z : P.ohi.z);
-  P.o_far = f3(P.nx ? P.ohi.x : P.olo.x, P.ny ? P.ohi.y : P.olo.y, P.nz ? P.ohi.z : P.olo.z);
+  const float os = fmaxf(fmaxf(ohi.x - olo.x, ohi.y - olo.y), ohi.z - olo.z);
+  Packet P = range_packet(olo, ohi, ilo, ihi);
+  P.coherent = P.coherent && ds <= kCoherentSpread && os <= S.coherent_span;
   return P;
 }
 
@@ -889,14 +895,16 @@ __device__ void trace_shadow_packet_r(const SceneView &S, const float3 (&o)[R], 
 // shared memory; each packet then tests only these.  A second list holds the
 // leaves between the beam's hit points and the light.
 //
-// The lists never change a result: a leaf's triangles are tested after the
-// ray's own slab test as before, and a leaf that is not in the list is one
-// that the ray's slab test fails (the beam's interval bounds are extremes of the same
-// rounded operations).  What the beam assumes of a ray -- its direction, or
-// its shadow origin, inside the beam's ranges -- is checked for every ray, and
-// a sample with a ray outside is taken again by walks from the root.  An item
-// whose beam reaches more leaves than a list holds has no lists
-// and walks the tree for every packet, two sub-rays per lane.
+// The lists change which leaves are looked at, not what a ray hits: a leaf's
+// triangles are tested after the ray's own slab test as before, and a leaf that is
+// not in the list is one that the ray's slab test fails (the beam's interval bounds
+// are extremes of the same rounded operations).  Only where two triangles are hit
+// at exactly the same distance (a common edge, a triangle that lies twice in the
+// mesh) may the list's order find the other one first.  What the beam assumes of
+// a ray -- its direction, or its shadow origin, inside the beam's ranges -- is
+// checked for every ray, and a sample with a ray outside is taken again by walks
+// from the root.  An item whose beam reaches more leaves than a list holds has no
+// lists and walks the tree for every packet, two sub-rays per lane.
 constexpr int kBeamLeaves = 32;  // one per lane
 struct Beam {                    // shared memory, one per warp
   float4 leaf[kBeamLeaves][2];   // {lo, hi.x}, {hi.y, hi.z, first triangle, count}, nearest entry first
@@ -916,23 +924,9 @@ __device__ __forceinline__ float3 max3(float3 a, float3 b) { return f3(fmaxf(a.x
 __device__ __forceinline__ bool within(float3 v, float3 lo, float3 hi) {
   return v.x >= lo.x && v.x <= hi.x && v.y >= lo.y && v.y <= hi.y && v.z >= lo.z && v.z <= hi.z;
 }
-__device__ __forceinline__ float wlow(float x) { return funord(__reduce_min_sync(kFull, ford(x))); }
-__device__ __forceinline__ float whigh(float x) { return funord(__reduce_max_sync(kFull, ford(x))); }
-__device__ __forceinline__ float3 wlow3(float3 v) { return f3(wlow(v.x), wlow(v.y), wlow(v.z)); }
-__device__ __forceinline__ float3 whigh3(float3 v) { return f3(whigh(v.x), whigh(v.y), whigh(v.z)); }
+__device__ __forceinline__ float3 wmin3(float3 v) { return f3(wmin(v.x), wmin(v.y), wmin(v.z)); }
+__device__ __forceinline__ float3 wmax3(float3 v) { return f3(wmax(v.x), wmax(v.y), wmax(v.z)); }
 
-// The interval bundle of given ranges; coherent means each axis' inverse direction keeps one sign.
-__device__ __forceinline__ Packet range_packet(float3 olo, float3 ohi, float3 ilo, float3 ihi) {
-  Packet P;
-  P.olo = olo; P.ohi = ohi; P.ilo = ilo; P.ihi = ihi;
-  P.nx = ihi.x < 0.0f;
-  P.ny = ihi.y < 0.0f;
-  P.nz = ihi.z < 0.0f;
-  P.coherent = (P.nx || ilo.x > 0.0f) && (P.ny || ilo.y > 0.0f) && (P.nz || ilo.z > 0.0f);
-  P.o_near = f3(P.nx ? olo.x : ohi.x, P.ny ? olo.y : ohi.y, P.nz ? olo.z : ohi.z);
-  P.o_far = f3(P.nx ? ohi.x : olo.x, P.ny ? ohi.y : olo.y, P.nz ? ohi.z : olo.z);
-  return P;
-}
 // The primary beam's bundle: 1/d of directions of one sign decreases with d, so the ends of the inverse's range are
 // the inverses of the ends, rounded outward by more than rcp_rn's last bit.  On an axis whose range holds zero (or
 // comes so near it that inverse_direction could clamp: the rows and columns of pixels that look along a coordinate
@@ -1092,8 +1086,8 @@ __device__ __forceinline__ int build_shadow_list(const SceneView &S, Beam &B, in
     lo = lo - f3(m, m, m);
     hi = hi + f3(m, m, m);
   }
-  lo = wlow3(lo);
-  hi = whigh3(hi);
+  lo = wmin3(lo);
+  hi = wmax3(hi);
   if (lane == 0) {
     B.slo = lo;
     B.shi = hi;
@@ -1129,8 +1123,8 @@ __device__ __forceinline__ void packet_range(const float3 (&v)[R], const bool (&
       lo = min3(lo, v[r]);
       hi = max3(hi, v[r]);
     }
-  lo = wlow3(lo);
-  hi = whigh3(hi);
+  lo = wmin3(lo);
+  hi = wmax3(hi);
 }
 
 // A wider bundle of directions (the sum of its extents per axis) takes no beam.
@@ -1141,12 +1135,12 @@ constexpr float kBeamSpread = 0.1f;
 template <int kGeo>
 __device__ __forceinline__ BeamLists close_beam(const SceneView &S, float3 olo, float3 ohi, float3 dlo, float3 dhi,
                                                 float3 llo, float3 lhi, float reach, Beam &B, int *stack) {
-  olo = wlow3(olo);
-  ohi = whigh3(ohi);
-  dlo = wlow3(dlo);
-  dhi = whigh3(dhi);
-  llo = wlow3(llo);
-  lhi = whigh3(lhi);
+  olo = wmin3(olo);
+  ohi = wmax3(ohi);
+  dlo = wmin3(dlo);
+  dhi = wmax3(dhi);
+  llo = wmin3(llo);
+  lhi = wmax3(lhi);
   const float ext = (dhi.x - dlo.x) + (dhi.y - dlo.y) + (dhi.z - dlo.z);
   BeamLists lists{kNoList, kNoList, 0};
   if (!(ext <= kBeamSpread)) return lists;  // a wide bundle reaches too many leaves (or a ray has no direction)
@@ -1402,57 +1396,53 @@ __device__ __forceinline__ PixelSample sample_pixel_group(const SceneView &S, in
           depth += hit[r].t;
           ++valid_depth;
         }
-        if (kMode != kDepthOnly) {
-          const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[r].tri);
-          const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
-          const float w = 1 - hit[r].u - hit[r].v;
-          normal[r] = unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u +
-                                f3(s2.x, s2.y, s2.z) * hit[r].v);
-          lit[r] = !(dot(normal[r], light) <= 0 || dot(normal[r], -ray[r]) <= 0);
-          if (lit[r]) {
-            const float4 *t4 = tri_record<kGeo>(S, hit[r].tri, 2);
-            const float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
-            sorigin[r] = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit[r].u, hit[r].v, light);
-            if (S.has_albedo) {
-              albedo[r] = s0.w * w + s1.w * hit[r].u + s2.w * hit[r].v;
-              r0[r] = hfunc_r0(albedo[r]);
-            }
+        const float4 *q = reinterpret_cast<const float4 *>(S.shade + hit[r].tri);
+        const float4 s0 = __ldg(q), s1 = __ldg(q + 1), s2 = __ldg(q + 2);
+        const float w = 1 - hit[r].u - hit[r].v;
+        normal[r] =
+            unit(f3(s0.x, s0.y, s0.z) * w + f3(s1.x, s1.y, s1.z) * hit[r].u + f3(s2.x, s2.y, s2.z) * hit[r].v);
+        lit[r] = !(dot(normal[r], light) <= 0 || dot(normal[r], -ray[r]) <= 0);
+        if (lit[r]) {
+          const float4 *t4 = tri_record<kGeo>(S, hit[r].tri, 2);
+          const float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
+          sorigin[r] = shadow_origin_rec<kGeo>(a, b, c, __ldg(q + 3), hit[r].u, hit[r].v, light);
+          if (S.has_albedo) {
+            albedo[r] = s0.w * w + s1.w * hit[r].u + s2.w * hit[r].v;
+            r0[r] = hfunc_r0(albedo[r]);
           }
         }
       }
     }
-    if (kMode != kDepthOnly) {
-      bool any_lit = false;
+    bool any_lit = false;
 #pragma unroll
-      for (int r = 0; r < R; ++r) any_lit = any_lit || lit[r];
-      if (__any_sync(kFull, any_lit)) {
-        unsigned occluded = 0;
-        bool near = true;
-        if constexpr (kBeam) {
+    for (int r = 0; r < R; ++r) any_lit = any_lit || lit[r];
+    if (__any_sync(kFull, any_lit)) {
+      unsigned occluded = 0;
+      bool near = true;
+      if constexpr (kBeam) {
 #pragma unroll
-          for (int r = 0; r < R; ++r) near = near && (!lit[r] || within(sorigin[r], beam->slo, beam->shi));
+        for (int r = 0; r < R; ++r) near = near && (!lit[r] || within(sorigin[r], beam->slo, beam->shi));
+      }
+      if constexpr (!kBeam) {
+        bool occ[R];
+        trace_shadow_packet_r<R, kGeo>(S, sorigin, light, sdir, lit, self, stack_code, stack_t, occ);
+#pragma unroll
+        for (int r = 0; r < R; ++r) occluded |= occ[r] ? 1u << r : 0u;
+      } else {
+        if (!__all_sync(kFull, near)) {
+          out.redo = true;
+          return out;
         }
-        if constexpr (!kBeam) {
-          bool occ[R];
-          trace_shadow_packet_r<R, kGeo>(S, sorigin, light, sdir, lit, self, stack_code, stack_t, occ);
+        occluded = shadow_in_list<R, kGeo>(S, *beam, lists->shadow, sorigin, light, sdir, lit, self, lists->first);
+      }
 #pragma unroll
-          for (int r = 0; r < R; ++r) occluded |= occ[r] ? 1u << r : 0u;
-        } else {
-          if (!__all_sync(kFull, near)) {
-            out.redo = true;
-            return out;
-          }
-          occluded = shadow_in_list<R, kGeo>(S, *beam, lists->shadow, sorigin, light, sdir, lit, self, lists->first);
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (lit[r]) ++out.shadow;
-          if (lit[r] && !((occluded >> r) & 1u)) {
-            const double cos4 = subrays ? subrays[j + r].cos4 : cos4_of(px[r], py[r]);
-            const float3 n = unit(normal[r]), l = lnorm, v = unit(-ray[r]);
-            const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], hc);
-            out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
-          }
+      for (int r = 0; r < R; ++r) {
+        if (lit[r]) ++out.shadow;
+        if (lit[r] && !((occluded >> r) & 1u)) {
+          const double cos4 = subrays ? subrays[j + r].cos4 : cos4_of(px[r], py[r]);
+          const float3 n = unit(normal[r]), l = lnorm, v = unit(-ray[r]);
+          const float n_h = hapke_reflectance(dot(n, l), dot(n, v), dot(l, v), albedo[r], r0[r], hc);
+          out.radiance += fmaxf(0, n_h * pose.intensity) * cos4;
         }
       }
     }
@@ -1472,7 +1462,7 @@ struct RaySample {
   float t;  // hit distance
   bool hit, lit, overflow;
 };
-template <int kMode, int kGeo, bool kChecked>
+template <int kGeo, bool kChecked>
 __device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, float py, const CellPose &pose, bool live,
                                                 int *stack_code, float *stack_t, Beam &B, BeamLists &lists) {
   RaySample out{0.0, 0.0f, false, false, false};
@@ -1494,7 +1484,6 @@ __device__ __forceinline__ RaySample sample_ray(const SceneView &S, float px, fl
   out.overflow = live && hit[0].hit < 0;
   out.hit = live && hit[0].hit == 1;
   out.t = hit[0].t;
-  if (kMode == kDepthOnly) return out;
   float3 normal = f3(0, 0, 0), sorigin[1] = {f3(0, 0, 0)};
   float albedo = S.hc.w, r0 = S.hc.r0_w;
   if (out.hit) {

@@ -124,7 +124,7 @@ __device__ __forceinline__ void trace_cells_item(const SceneView &S, int n_pix, 
     // the set's ppw pixels: their sub-rays' coordinates and FP64 cos^4 once per
     // set (entry p * ss2 + j: sub-ray j of the pixel in lanes p * cw ...)
     const int table = ppw * ss2;
-    const bool shared_subrays = kMode != kDepthOnly && table <= kSubrayTable;
+    const bool shared_subrays = table <= kSubrayTable;
     if (shared_subrays) {
       for (int q0 = 0; q0 < table; q0 += 32) {  // warp-uniform: every lane takes part in the shuffle
         const int q = q0 + lane, p = min(q / ss2, ppw - 1);
@@ -216,9 +216,9 @@ __device__ __forceinline__ void trace_pose_item(const SceneView &S, int n_pix, c
       const int pix = __shfl_sync(kFull, pixel, min(p, 31));
       const bool live = p < count && r < ss2;
       const int rr = live ? r : 0;
-      const RaySample s = sample_ray<kMode, kGeo, false>(S, subray_x(S, pix % S.width, rr % S.samples),
-                                                         subray_y(S, pix / S.width, rr / S.samples), pose, live,
-                                                         sh.code, sh.t, sh.beam, lists);
+      const RaySample s = sample_ray<kGeo, false>(S, subray_x(S, pix % S.width, rr % S.samples),
+                                                  subray_y(S, pix / S.width, rr / S.samples), pose, live, sh.code,
+                                                  sh.t, sh.beam, lists);
       if (live) {
         const int at = p * (run + 1) + sub;
         sh.term[at] = s.overflow ? __longlong_as_double(0x7ff8000000000000ll) : s.term;
