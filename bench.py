@@ -82,12 +82,12 @@ METRIC = "DVS events/s and Mrays/s at 1280x720 on 1 GB300; serving p99 latency v
 # (dram__bytes_read.sum + dram__bytes_write.sum) per pixel-cell.  Radiance
 # writes still held in L2 when the kernel ends are not in the DRAM count.
 TRACE_WARP_INSTRUCTIONS_PER_RAY = {
-    ("precision", "half+watertight", "sah", 32, 1): 731631334830 / 29471262019,
-    ("orbit", "reference", "sah", 32, 1): 50147058636 / 1768685229,
+    ("precision", "half+watertight", "sah", 32, 1): 733444959002 / 29471262019,
+    ("orbit", "reference", "sah", 32, 1): 50196567867 / 1768685229,
 }
 TRACE_DRAM_BYTES_PER_PIXEL_CELL = {
-    ("precision", "half+watertight", "sah", 32, 1): (71990016 + 284999168) / (921600 * 64),
-    ("orbit", "reference", "sah", 32, 1): (17014784 + 235764224) / (89960 * 640),
+    ("precision", "half+watertight", "sah", 32, 1): (68543232 + 281074688) / (921600 * 64),
+    ("orbit", "reference", "sah", 32, 1): (13885184 + 235275264) / (89960 * 640),
 }
 # ncu DRAM counters (dram__bytes_read.sum + dram__bytes_write.sum) of the 44
 # launches of one device-readout batch of 4,194,304 events (the readout

@@ -456,9 +456,10 @@ cudaError_t launch_circuit_list(int n, const int32_t *rank_list, const Cell *cel
 // A Philox draw depends on its pixel and cell alone.  With few pixels the
 // circuit's threads, one a pixel, cannot hide a cell's chain of draw and receptor
 // step, so the draws of all cells go ahead on a thread each: 64 cells of 64x48
-// pixels 93 -> 68 us, of 128x96 95 -> 76, of 256x192 102 -> 98; of 320x240 110 ->
-// 118, so the line lies at two warps a scheduler.  (Reset noise continues a
-// cell's stream after its draw and keeps the draw in the circuit.)
+// pixels 93 -> 68 us, of 128x96 95 -> 76.  The gain shrinks to 4 us at 256x192 and
+// is a loss of 8 at 320x240 (110 -> 118), so the line lies below both, at 38,912
+// pixels: two warps a scheduler.  (Reset noise continues a cell's stream after its
+// draw and keeps the draw in the circuit.)
 bool circuit_draws_ahead(int n, const PixelParams &p, const PhotoParams &photo) {
   return photo.philox && photo.chunk_f32 && photo.shot_noise && p.reset_noise_std == 0 && n < kResidentWarps * 16;
 }

@@ -104,10 +104,8 @@ def build():
     """Compile the two oracle libraries (and the reference harness when the
     reference checkout is present)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    # the reference checkout: DVS_REFERENCE_DIR, else the development
-    # container's read-only checkout (absent on the GPU machines)
-    ref = os.environ.get("DVS_REFERENCE_DIR") or "/root/reference"
-    if os.path.isdir(os.path.join(ref, "include", "dvs")):
+    ref = os.environ.get("DVS_REFERENCE_DIR")  # the reference checkout, where there is one
+    if ref and os.path.isdir(os.path.join(ref, "include", "dvs")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + ref], check=True)
 
 
